@@ -50,6 +50,7 @@ struct cujpegxl_encoder {
     unsigned long long* result_pinned{nullptr};
     std::size_t arena_bytes{0};
     bool pending{false};
+    bool frontend_planes{false};  // the quantised planes are the frontend's own, not a caller's
     // Learned decisions: the attached network (not owned), its margin and
     // flags, and the per-frame decision buffers in the arena.
     const cujpegxl_b200_acsnet* net{nullptr};
@@ -199,6 +200,7 @@ void release(cujpegxl_encoder* e) {
     e->arena = nullptr;
     e->nv12_pinned = nullptr;
     e->geo_w = e->geo_h = 0;
+    e->frontend_planes = false;
 }
 
 // Allocates every per-geometry buffer (nothing is allocated per frame).
@@ -228,6 +230,7 @@ bool allocate(cujpegxl_encoder* e) {
     const std::size_t o_sec{a.take(plan.sections.size() * sizeof(jxb::Section))};
     const std::size_t o_str{a.take(plan.stripes.size() * sizeof(jxb::Stripe))};
     const std::size_t o_ord{a.take(plan.order.size() * 2)};
+    const std::size_t o_rank{a.take(plan.rank.size() * 2)};
     const std::size_t o_pre{a.take(plan.pre_const.size())};
     const std::size_t o_mid{a.take(plan.mid_const.size())};
     const std::size_t o_acp{a.take(plan.ac_prefix.size())};
@@ -251,8 +254,9 @@ bool allocate(cujpegxl_encoder* e) {
     const std::size_t o_to{a.take(static_cast<std::size_t>(tiles + 1) * 8)};
     const std::size_t o_sp{a.take(plan.sections.size() * 8)};
     const std::size_t o_res{a.take(4 * 8)};
-    const std::uint32_t tok_cap{static_cast<std::uint32_t>(std::min<std::size_t>(nb * jxb::kTokensPerBlock, 0xfffffff0u))};
-    const std::size_t o_tok{a.take(static_cast<std::size_t>(tok_cap) * 4)};
+    const std::size_t tok_words{nb * jxb::kTokensPerBlock};
+    const std::uint32_t tok_cap{static_cast<std::uint32_t>(std::min<std::size_t>(tok_words, 0xfffffff0u))};
+    const std::size_t o_tok{a.take(tok_words * 4)};
     const std::size_t o_tokn{a.take(4)};
     const std::size_t o_stok{a.take(plan.stripes.size() * 8)};
     const std::size_t o_out{a.take(out_cap)};
@@ -317,6 +321,8 @@ bool allocate(cujpegxl_encoder* e) {
     ed.nzn = fo.nzn;
     ed.nzc = fo.nzc;
     ed.order = reinterpret_cast<const std::uint16_t*>(b + o_ord);
+    ed.rank = reinterpret_cast<const std::uint16_t*>(b + o_rank);
+    ed.direct = true;
     ed.pre_const = b + o_pre;
     ed.pre_const_bits = plan.pre_const_bits;
     ed.mid_const = b + o_mid;
@@ -360,6 +366,8 @@ bool allocate(cujpegxl_encoder* e) {
             cudaMemcpy(b + o_str, plan.stripes.data(), plan.stripes.size() * sizeof(jxb::Stripe),
                        cudaMemcpyHostToDevice) == cudaSuccess &&
             cudaMemcpy(b + o_ord, plan.order.data(), plan.order.size() * 2, cudaMemcpyHostToDevice) ==
+                cudaSuccess &&
+            cudaMemcpy(b + o_rank, plan.rank.data(), plan.rank.size() * 2, cudaMemcpyHostToDevice) ==
                 cudaSuccess &&
             cudaMemcpy(b + o_pre, plan.pre_const.data(), plan.pre_const.size(), cudaMemcpyHostToDevice) ==
                 cudaSuccess &&
@@ -418,8 +426,16 @@ bool enqueue_frame(cujpegxl_encoder* e, const std::uint8_t* luma, std::size_t lp
         in.net_qf = dec.qf;
         in.tile_order = dec.tile_order;
     }
-    if ((stages & 1u) && !jxb::frontend_launch(in, e->fs, ft, e->fo, st)) return false;
-    return (stages & 2u) == 0 || jxb::entropy_launch(e->ed, st);
+    if (stages & 1u) {
+        if (!jxb::frontend_launch(in, e->fs, ft, e->fo, st)) return false;
+        e->frontend_planes = true;
+    }
+    if ((stages & 2u) == 0) return true;
+    if (e->frontend_planes) return jxb::entropy_launch(e->ed, st);
+    // The entropy stage alone over planes that no frontend wrote.
+    jxb::EntropyDev ed{e->ed};
+    ed.direct = false;
+    return jxb::entropy_launch(ed, st);
 }
 
 cujpegxl_status finish(cujpegxl_encoder* e, cujpegxl_output* output);
@@ -835,13 +851,14 @@ cujpegxl_status cujpegxl_b200_encode_planes(cujpegxl_encoder* encoder, const cuj
     if (!ok) return CUJPEGXL_INTERNAL_ERROR;
     // The DcGlobal blob now belongs to these planes; force a refresh on the next encode.
     encoder->geo_distance = -1.0f;
-    const std::uint32_t saved_bits{encoder->ed.dc_global_bits};
-    encoder->ed.dc_global_bits = nbits;
+    encoder->frontend_planes = false;
+    jxb::EntropyDev ed{encoder->ed};
+    ed.dc_global_bits = nbits;
+    ed.direct = false;
     nz_kernel<<<static_cast<unsigned>((nb + 255) / 256), 256, 0, st>>>(
         encoder->fo.ac, encoder->fo.acs, static_cast<int>(W / 8), static_cast<int>(H / 8), encoder->fo.nzn,
         encoder->fo.nzc);
-    ok = cudaGetLastError() == cudaSuccess && jxb::entropy_launch(encoder->ed, st);
-    encoder->ed.dc_global_bits = saved_bits;
+    ok = cudaGetLastError() == cudaSuccess && jxb::entropy_launch(ed, st);
     if (!ok) return CUJPEGXL_INTERNAL_ERROR;
     return finish(encoder, output);
 }

@@ -398,6 +398,47 @@ __device__ __forceinline__ std::uint32_t token_table_index(std::uint32_t t) {
 __device__ __forceinline__ std::uint32_t token_extra_count(std::uint32_t t) { return (t >> 11) & 15u; }
 __device__ __forceinline__ std::uint32_t token_extra_bits(std::uint32_t t) { return t >> 15; }
 
+// Where a stripe's tokens are: tokens below `split` at near[t], the others at
+// far[t]; near is null when they did not fit the pool. Direct stripes have
+// kTokensPerBlock places a block of their own, and what exceeds those runs of
+// the output buffer's end (dense_tokens). Otherwise the stripe's run of the
+// pool holds all of them. `split` is a multiple of 32.
+struct StripeTokens {
+    const std::uint32_t* near;
+    const std::uint32_t* far;
+    std::uint32_t split;
+    __device__ __forceinline__ const std::uint32_t* at(std::uint32_t t) const { return (t < split ? near : far) + t; }
+};
+
+__device__ __forceinline__ std::uint32_t stripe_blocks(const EntropyDev& e, const Stripe& st) {
+    return (st.item0 - e.ac_first) / 3;  // blocks of the stripes before it
+}
+
+// Place of a direct stripe's tokens from `split` on, given its offset (in
+// tokens, counted back from the end of the output buffer) there.
+//
+// The file cannot reach them. A token is at most 13 extra bits and a code; a
+// cluster's code is optimal for its counts raised to a floor that adds less
+// than 15% to their sum (a depth above 15 needs a total of a thousand times
+// the floor), so no worse than 6 bits a token on that sum, the length of a
+// fixed code for 64 symbols. With at most 192 tokens a block that is 2.5 x 192
+// bytes of tokens and, for the other items, less than 48, against the
+// buffer's 1200 bytes a block (worst_case_output) and 4 x (192 - 32) of
+// tokens kept here. The layout checks it all the same.
+__device__ __forceinline__ std::uint32_t* dense_tokens(const EntropyDev& e, std::uint32_t back) {
+    return reinterpret_cast<std::uint32_t*>(e.out + e.out_capacity) - back;
+}
+
+__device__ __forceinline__ StripeTokens stripe_tokens(const EntropyDev& e, const Stripe& st, unsigned blk, int cells) {
+    const std::uint32_t place{e.stripe_tok[2 * blk]};
+    if (!e.direct) {
+        return {place != kNoTokens ? e.tok_pool + place : nullptr, nullptr, 0xffffffe0u};
+    }
+    const std::uint32_t split{static_cast<std::uint32_t>(cells) * kTokensPerBlock};
+    return {e.tok_pool + static_cast<std::size_t>(stripe_blocks(e, st)) * kTokensPerBlock,
+            dense_tokens(e, place) - split, split};
+}
+
 // Number of coefficient tokens of an item: the scan positions from `covered`
 // through its last non-zero coefficient, exactly those on which
 // coeff_tokens reports `has` (all positions to the end of the transform when
@@ -465,7 +506,7 @@ __device__ std::uint32_t cta_exclusive_scan(std::uint32_t v, std::uint32_t* warp
 // tokens counted into the 32-cluster histogram and written, in stream order,
 // to a run of the token pool that the stripe reserves once it knows their
 // number (count tokens first sized, then the coefficient extents).
-__device__ __forceinline__ void ac_tok_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+__device__ __forceinline__ void ac_tok_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char ac_smem[];
     StripeStage& s{*reinterpret_cast<StripeStage*>(ac_smem)};
     std::uint32_t* hist{reinterpret_cast<std::uint32_t*>(ac_smem + sizeof(StripeStage))};  // [32][64]
@@ -548,6 +589,347 @@ __device__ __forceinline__ void ac_tok_body(const EntropyDev& e, const unsigned 
     __syncthreads();
     for (int i{tid}; i < kNumClusters * kAcSymbols; i += kAcThreads) {
         if (hist[i]) atomicAdd(&e.ac_hist[(i / kAcSymbols) * 256 + i % kAcSymbols], hist[i]);
+    }
+}
+
+// ---- pass 1 for the frontend's own planes: one lane per token -------------------------
+
+constexpr int kStripeRegions = kAcGroupBlocks / 4;  // 32x32-pixel regions of a stripe
+
+// What the direct token pass keeps in shared memory (the coefficients
+// themselves stay in global memory).
+struct DirectStage {
+    std::uint32_t hist[kNumClusters * kAcSymbols];
+    // Non-zero coefficients in scan order, two words per block. The 16 blocks
+    // of a region lie in Z order, in which the blocks of an aligned DCT16 or
+    // DCT32 are adjacent, so an item's words are contiguous.
+    std::uint32_t bitmap[3][kStripeRegions][32];
+    std::uint16_t before[3][kStripeRegions][32];     // the item's non-zeros in its earlier words
+    std::uint16_t count[kStripeItems];               // tokens of each item
+    std::uint32_t info[kStripeItems];                // what a token needs to know of each item (pack_direct_item)
+    std::uint32_t item_off[kStripeItems + 33];       // first token of each item that has any, then a sentinel
+    std::uint32_t item_info[kStripeItems];           // and its info
+    alignas(16) std::uint16_t order[64 + 256 + 1024];  // raw index of each scan position
+    std::uint16_t rank[64 + 256 + 1024];               // scan position of each raw index
+    alignas(16) std::uint8_t nz_ctx[64];               // copy of g_coeff_ctx, as in StripeStage
+    std::uint8_t freq_ctx[64];
+    std::uint8_t zd_cluster[2][kZdRow];
+    std::uint8_t nzn[3][kStripeRows + 1][kAcGroupBlocks];  // row 0: the block row above the stripe
+    // Of each block: its transform's log2 side in blocks (bits 9-10), the
+    // block's ordinal in it (bits 5-8) and its first bitmap word (bits 0-4).
+    std::uint16_t owner[kStripeRows][kAcGroupBlocks];
+    std::uint32_t scan[kAcWarps + 1];
+    std::uint32_t far;  // offset of the tokens past the stripe's own places (dense_tokens)
+};
+static_assert(offsetof(DirectStage, zd_cluster) + 2 * kZdRow == offsetof(DirectStage, nz_ctx) + kCoeffCtxBytes &&
+                  offsetof(DirectStage, nz_ctx) % 16 == 0 && offsetof(DirectStage, order) % 16 == 0 &&
+                  offsetof(DirectStage, rank) % 16 == 0,
+              "context and order tables: aligned contiguous copies");
+constexpr unsigned kNoOwner = 0xffffu;
+
+// First entry of a transform of 2^lside blocks a side in the concatenated orders.
+__device__ __forceinline__ int order_base(int lside) { return lside == 0 ? 0 : (lside == 1 ? 64 : 320); }
+
+// First bitmap word of stripe block (r, x) in its region: twice its Z-order index.
+__device__ __forceinline__ int bitmap_word(int r, int x) {
+    return 2 * ((x & 1) | ((r & 1) << 1) | ((x & 2) << 1) | ((r & 2) << 2));
+}
+
+// Non-zeros (11 bits), log2 side (2), block column (5) and row (2), plane (2).
+__device__ __forceinline__ std::uint32_t pack_direct_item(std::uint32_t nz, int lside, int x, int r, int c) {
+    return nz | (static_cast<std::uint32_t>(lside) << 11) | (static_cast<std::uint32_t>(x) << 13) |
+           (static_cast<std::uint32_t>(r) << 18) | (static_cast<std::uint32_t>(c) << 20);
+}
+
+// One CTA per stripe of planes the frontend wrote (every block covered by
+// exactly one transform, transforms at multiples of their size, non-zero
+// counts exact; anything else would give other tokens but stays inside the
+// stripe's arrays and pool run). A first pass reads the coefficients in
+// storage order, eight per load, and sets one bit per non-zero at its scan
+// position; an item's token count, and for every position the non-zeros left
+// and the previous coefficient, then follow from population counts, so the
+// tokens are independent of each other and are written one per lane, whatever
+// the mix of item sizes. The stripe's tokens have a fixed place in the pool;
+// only a stripe of more than kTokensPerBlock a block reserves room for the
+// rest, so everything is stored and stored once.
+__device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const unsigned blk) {
+    extern __shared__ __align__(16) unsigned char ac_smem[];
+    DirectStage& s{*reinterpret_cast<DirectStage*>(ac_smem)};
+    const int tid{static_cast<int>(threadIdx.x)};
+    const int lane{tid & 31};
+    const int warp{tid >> 5};
+    const Stripe st{e.stripes[blk]};
+    const GroupGeom gg{ac_group_geom(e, st.group)};
+    const std::size_t blk0{static_cast<std::size_t>(gg.by0 + st.r0) * e.bw + gg.bx0};
+    const int cells{st.rows * gg.gw};
+
+    // The stripe's coefficients, 16 bytes (eight of one block) per load, all
+    // loads issued before anything waits.
+    static_assert(kAcGroupBlocks * (kCoeffsPerBlock / 8) <= kAcThreads, "one vector of each block row per thread");
+    const bool loads{tid < gg.gw * (kCoeffsPerBlock / 8)};
+    uint4 v[3][kStripeRows];
+#pragma unroll
+    for (int c{0}; c < 3; ++c) {
+        const uint4* src{reinterpret_cast<const uint4*>(
+                             e.ac + (static_cast<std::size_t>(c) * e.nblocks + blk0) * kCoeffsPerBlock) + tid};
+#pragma unroll
+        for (int r{0}; r < kStripeRows; ++r) {
+            v[c][r] = loads && r < st.rows ? __ldg(src + static_cast<std::size_t>(r) * e.bw * (kCoeffsPerBlock / 8))
+                                           : make_uint4(0, 0, 0, 0);
+        }
+    }
+    // Tables, strategies and count predictions; cleared bitmap and histogram.
+    constexpr int kOrderVecs{(64 + 256 + 1024) * 2 / 16};
+    for (int i{tid}; i < kOrderVecs; i += kAcThreads) {
+        cp_async16(reinterpret_cast<uint4*>(s.order) + i, reinterpret_cast<const uint4*>(e.order) + i);
+        cp_async16(reinterpret_cast<uint4*>(s.rank) + i, reinterpret_cast<const uint4*>(e.rank) + i);
+    }
+    for (int i{tid}; i < kCoeffCtxBytes / 16; i += kAcThreads) {
+        cp_async16(reinterpret_cast<uint4*>(s.nz_ctx) + i, reinterpret_cast<const uint4*>(g_coeff_ctx) + i);
+    }
+    // One block per thread, so a block's default owner is written by the
+    // thread that may then claim it for its own transform.
+    static_assert(kStripeRows * kAcGroupBlocks <= kAcThreads, "one block per thread");
+    const int cr{tid / gg.gw};
+    const int cx{tid - cr * gg.gw};
+    int side{0};
+    if (tid < cells) {
+        const std::size_t b{blk0 + static_cast<std::size_t>(cr) * e.bw + cx};
+        const int n{e.acs[b]};
+        std::uint8_t pn[3], pt[3];
+#pragma unroll
+        for (int c{0}; c < 3; ++c) {
+            const std::size_t cb{static_cast<std::size_t>(c) * e.nblocks + b};
+            pn[c] = e.nzn[cb];
+            pt[c] = cr == 0 && st.r0 > 0 ? e.nzn[cb - e.bw] : 0;
+        }
+        s.owner[cr][cx] = kNoOwner;
+        side = n == 8 ? 1 : (n == 16 ? 2 : (n == 32 ? 4 : 0));
+        if (cr + side > st.rows || cx + side > gg.gw || ((cr | cx) & (side - 1)) != 0) side = 0;
+#pragma unroll
+        for (int c{0}; c < 3; ++c) {
+            s.nzn[c][cr + 1][cx] = pn[c];
+            if (cr == 0) s.nzn[c][0][cx] = pt[c];
+        }
+    }
+    for (int i{tid}; i < kNumClusters * kAcSymbols; i += kAcThreads) s.hist[i] = 0;
+    for (int i{tid}; i < 3 * kStripeRegions * 32; i += kAcThreads) (&s.bitmap[0][0][0])[i] = 0;
+    __syncthreads();
+    if (side != 0) {
+        const int lside{side >> 1};
+        const int own{(lside << 9) | bitmap_word(cr, cx)};
+        for (int q{0}; q < side * side; ++q) {
+            s.owner[cr + (q >> lside)][cx + (q & (side - 1))] = static_cast<std::uint16_t>(own | (q << 5));
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+
+    if (loads) {
+        const int x{tid >> 3};
+#pragma unroll
+        for (int r{0}; r < kStripeRows; ++r) {
+            if (r >= st.rows) continue;
+            const unsigned own{s.owner[r][x]};
+            if (own == kNoOwner) continue;
+            const int lside{static_cast<int>(own >> 9)};
+            const int covered{1 << (2 * lside)};
+            const std::uint16_t* rank{s.rank + order_base(lside) + ((own >> 5) & 15u) * kCoeffsPerBlock +
+                                      (tid & 7) * 8};
+#pragma unroll
+            for (int c{0}; c < 3; ++c) {
+                const std::uint32_t word[4]{v[c][r].x, v[c][r].y, v[c][r].z, v[c][r].w};
+                if ((word[0] | word[1] | word[2] | word[3]) == 0) continue;
+                std::uint32_t* bits{&s.bitmap[c][x >> 2][own & 31u]};
+                // Bit i: coefficient i of the vector is not zero.
+                std::uint32_t set{0};
+#pragma unroll
+                for (int i{0}; i < 8; ++i) {
+                    set |= ((word[i >> 1] >> (16 * (i & 1))) & 0xffffu) != 0 ? 1u << i : 0u;
+                }
+                while (set != 0) {
+                    const int k{rank[__ffs(set) - 1]};
+                    set &= set - 1;
+                    // Positions below `covered` are the low frequencies, never coded here.
+                    if (k >= covered) atomicOr(&bits[k >> 5], 1u << (k & 31));
+                }
+            }
+        }
+    }
+    __syncthreads();
+
+    // Tokens of each item: its count token, then every scan position through
+    // its last non-zero. A warp per region and plane, a lane per bitmap word;
+    // sums over an item's words are segmented warp scans.
+    for (int u{warp}; u < 3 * kStripeRegions; u += kAcWarps) {
+        const int c{u / kStripeRegions};
+        const int region{u - c * kStripeRegions};
+        const int z{lane >> 1};
+        const int r{((z >> 1) & 1) | ((z >> 2) & 2)};
+        const int x{4 * region + ((z & 1) | ((z >> 1) & 2))};
+        const unsigned own{r < st.rows && x < gg.gw ? s.owner[r][x] : kNoOwner};
+        const int lside{own != kNoOwner ? static_cast<int>(own >> 9) : 0};
+        const int words{2 << (2 * lside)};
+        const int seg{lane & ~(words - 1)};
+        const std::uint32_t m{s.bitmap[c][region][lane]};
+        const std::uint32_t pc{static_cast<std::uint32_t>(__popc(m))};
+        std::uint32_t sum{pc};
+#pragma unroll
+        for (int off{1}; off < 32; off <<= 1) {
+            const std::uint32_t t{__shfl_up_sync(kFull, sum, off)};
+            if (lane - seg >= off) sum += t;
+        }
+        s.before[c][region][lane] = static_cast<std::uint16_t>(sum - pc);
+        const std::uint32_t nz{__shfl_sync(kFull, sum, seg + words - 1)};
+        const unsigned filled{__ballot_sync(kFull, m != 0) & (kFull >> (32 - words) << seg)};
+        const int last{filled != 0 ? 31 - __clz(static_cast<int>(filled)) : seg};
+        const std::uint32_t lm{__shfl_sync(kFull, m, last)};
+        const std::uint32_t covered{1u << (2 * lside)};
+        const std::uint32_t end{max(covered, 32u * static_cast<std::uint32_t>(last - seg + 1) -
+                                                 static_cast<std::uint32_t>(__clz(static_cast<int>(lm))))};
+        if ((lane & 1) == 0 && r < st.rows && x < gg.gw) {
+            const int j{3 * (r * gg.gw + x) + (c == 1 ? 0 : (c == 0 ? 1 : 2))};
+            const bool first{own != kNoOwner && lane == seg};
+            s.count[j] = first ? static_cast<std::uint16_t>(1 + end - covered) : static_cast<std::uint16_t>(0);
+            s.info[j] = pack_direct_item(nz, lside, x, r, c);
+        }
+    }
+    __syncthreads();
+    // Offsets: tokens in the low half of the scanned word, items with tokens
+    // in the high half. Each thread takes two adjacent items.
+    const int nitems{3 * cells};
+    std::uint32_t count[2];
+#pragma unroll
+    for (int h{0}; h < 2; ++h) count[h] = 2 * tid + h < nitems ? s.count[2 * tid + h] : 0u;
+    const std::uint32_t mine{count[0] + count[1] + ((count[0] != 0 ? 0x10000u : 0u) + (count[1] != 0 ? 0x10000u : 0u))};
+    std::uint32_t both{0};
+    std::uint32_t off{cta_exclusive_scan(mine, s.scan, both)};
+#pragma unroll
+    for (int h{0}; h < 2; ++h) {
+        if (count[h] == 0) continue;
+        s.item_off[off >> 16] = off & 0xffffu;
+        s.item_info[off >> 16] = s.info[2 * tid + h];
+        off += 0x10000u + count[h];
+    }
+    const int nactive{static_cast<int>(both >> 16)};
+    if (tid < 33) s.item_off[nactive + tid] = 0xffffffffu;
+    const std::uint32_t total{min(both & 0xffffu, static_cast<std::uint32_t>(cells) * kMaxTokensPerBlock)};
+    const std::uint32_t own{static_cast<std::uint32_t>(cells) * kTokensPerBlock};
+    if (tid == 0) {
+        std::uint32_t far{0};
+        if (total > own) {
+            const std::uint32_t more{(total - own + 31u) & ~31u};
+            far = atomicAdd(e.tok_count, more) + more;
+        }
+        s.far = far;
+        e.stripe_tok[2 * blk] = far;
+        e.stripe_tok[2 * blk + 1] = total;
+    }
+    __syncthreads();
+
+    // Each warp takes a contiguous run of tokens, 32 at a time: the items that
+    // start among them come from one load and one reduction, so a lane knows
+    // its item without a search. kAhead groups are prepared together, so that
+    // their coefficient loads overlap.
+    constexpr int kAhead{4};
+    std::uint32_t* near{e.tok_pool + static_cast<std::size_t>(stripe_blocks(e, st)) * kTokensPerBlock};
+    std::uint32_t* far{dense_tokens(e, s.far) - own};
+    const std::uint32_t groups{(total + 31) / 32};
+    const std::uint32_t per_warp{(groups + kAcWarps - 1) / kAcWarps};
+    const std::uint32_t t_first{32 * per_warp * static_cast<std::uint32_t>(warp)};
+    const std::uint32_t t_end{min(total, t_first + 32 * per_warp)};
+    int base{0};  // the item of token t0
+    if (t_first < t_end) {
+        int hi{nactive - 1};
+        while (base < hi) {
+            const int mid{(base + hi + 1) >> 1};
+            if (s.item_off[mid] <= t_first) {
+                base = mid;
+            } else {
+                hi = mid - 1;
+            }
+        }
+    }
+    for (std::uint32_t t0{t_first}; t0 < t_end; t0 += 32 * kAhead) {
+        std::uint32_t info[kAhead];
+        std::uint32_t at[kAhead];      // token index inside its item
+        std::uint32_t state[kAhead];   // non-zeros left << 1 | previous coefficient non-zero
+        std::int32_t val[kAhead];
+#pragma unroll
+        for (int g{0}; g < kAhead; ++g) {
+            const std::uint32_t tg{t0 + 32 * g};
+            const std::uint32_t rel{s.item_off[min(base + 1 + lane, nactive)] - tg};
+            const unsigned starts{__reduce_or_sync(kFull, rel < 32 ? 1u << rel : 0u)};
+            const int item{min(base + __popc(starts & ((2u << lane) - 1u)), nactive - 1)};
+            base += __popc(starts) + (__ballot_sync(kFull, rel == 32) != 0 ? 1 : 0);
+            info[g] = s.item_info[item];
+            at[g] = tg + lane - s.item_off[item];
+            val[g] = 0;
+            state[g] = 0;
+            if (tg + lane >= t_end || at[g] == 0) continue;
+            // Scan position k: the non-zeros left from the bits before it, the
+            // previous coefficient's bit (or the rule for the first position).
+            const int lside{static_cast<int>((info[g] >> 11) & 3u)};
+            const int x{static_cast<int>((info[g] >> 13) & 31u)};
+            const int r{static_cast<int>((info[g] >> 18) & 3u)};
+            const int c{static_cast<int>((info[g] >> 20) & 3u)};
+            const std::uint32_t nz{info[g] & 2047u};
+            const std::uint32_t covered{1u << (2 * lside)};
+            const std::uint32_t k{covered + at[g] - 1};
+            const int w{min(bitmap_word(r, x) + static_cast<int>(k >> 5), 31)};
+            const std::uint32_t m{s.bitmap[c][x >> 2][w]};
+            const std::uint32_t bit{k & 31u};
+            const std::uint32_t left{nz - s.before[c][x >> 2][w] -
+                                     static_cast<std::uint32_t>(__popc(m & ((1u << bit) - 1u)))};
+            const std::uint32_t earlier{bit != 0 ? m << (32 - bit) : s.bitmap[c][x >> 2][max(w - 1, 0)]};
+            const std::uint32_t prev{at[g] == 1 ? (nz > (covered * kCoeffsPerBlock) / 16 ? 0u : 1u) : earlier >> 31};
+            state[g] = (left << 1) | prev;
+            if ((m >> bit) & 1u) {
+                const int raw{s.order[order_base(lside) + static_cast<int>(k)]};
+                const int q{raw >> 6};
+                const std::size_t b{blk0 + static_cast<std::size_t>(r + (q >> lside)) * e.bw + x +
+                                    (q & ((1 << lside) - 1))};
+                val[g] = __ldg(e.ac + (static_cast<std::size_t>(c) * e.nblocks + b) * kCoeffsPerBlock + (raw & 63));
+            }
+        }
+#pragma unroll
+        for (int g{0}; g < kAhead; ++g) {
+            const std::uint32_t t{t0 + 32 * g + lane};
+            if (t >= t_end) continue;
+            const int lside{static_cast<int>((info[g] >> 11) & 3u)};
+            const int c{static_cast<int>((info[g] >> 20) & 3u)};
+            std::uint32_t value;
+            int cl;
+            if (at[g] == 0) {
+                const int x{static_cast<int>((info[g] >> 13) & 31u)};
+                const int r{static_cast<int>((info[g] >> 18) & 3u)};
+                const bool hl{x > 0};
+                const bool ht{st.r0 + r > 0};
+                const std::uint32_t top{ht ? s.nzn[c][r][x] : 0u};
+                const std::uint32_t left{hl ? s.nzn[c][r + 1][x - 1] : 0u};
+                cl = context_cluster(nonzero_context(predict_nonzeros(hl, ht, top, left), block_ctx(c, 8 << lside)));
+                value = info[g] & 2047u;
+            } else {
+                // The context tables and clamps of coeff_tokens.
+                const std::uint32_t l2{static_cast<std::uint32_t>(2 * lside)};
+                const std::uint32_t covered{1u << l2};
+                const std::uint32_t k{covered + at[g] - 1};
+                const std::uint32_t nzi{min(((state[g] >> 1) + covered - 1) >> l2, 63u)};
+                const std::uint32_t z{min((static_cast<std::uint32_t>(s.nz_ctx[nzi]) + s.freq_ctx[min(k >> l2, 63u)]) * 2 +
+                                              (state[g] & 1u),
+                                          static_cast<std::uint32_t>(kZeroDensityCount - 1))};
+                cl = s.zd_cluster[c == 1 ? 0 : 1][z];
+                value = pack_signed(val[g]);
+            }
+            std::uint32_t tok, nb, bits;
+            hybrid_uint(value, tok, nb, bits);
+            atomicAdd(&s.hist[cl * kAcSymbols + tok], 1u);
+            (t < own ? near : far)[t] = pack_ac_token(cl, tok, nb, bits);
+        }
+    }
+    __syncthreads();
+    for (int i{tid}; i < kNumClusters * kAcSymbols; i += kAcThreads) {
+        if (s.hist[i]) atomicAdd(&e.ac_hist[(i / kAcSymbols) * 256 + i % kAcSymbols], s.hist[i]);
     }
 }
 
@@ -1029,16 +1411,15 @@ __device__ __forceinline__ void ac_bits_body(const EntropyDev& e, const unsigned
     const int lane{tid & 31};
     const Stripe st{e.stripes[blk]};
     const GroupGeom gg{ac_group_geom(e, st.group)};
-    const std::uint32_t tbase{e.stripe_tok[2 * blk]};
-    if ((tbase != kNoTokens) != (kSet == kStoredStripes)) return;
-    if (tbase != kNoTokens) {
+    const StripeTokens pool{stripe_tokens(e, st, blk, st.rows * gg.gw)};
+    if ((pool.near != nullptr) != (kSet == kStoredStripes)) return;
+    if (pool.near != nullptr) {
         // Stored tokens: the stripe's whole length goes on its first item
         // (the scan only needs sums at stripe and section starts).
         const std::uint32_t ntok{e.stripe_tok[2 * blk + 1]};
-        const std::uint32_t* pool{e.tok_pool + tbase};
         std::uint32_t sum{0};
         for (std::uint32_t t{static_cast<std::uint32_t>(tid)}; t < ntok; t += kAcThreads) {
-            const std::uint32_t tk{pool[t]};
+            const std::uint32_t tk{*pool.at(t)};
             sum += __ldg(&e.ac_depth[token_table_index(tk)]) + token_extra_count(tk);
         }
         sum = warp_sum(sum);
@@ -1386,7 +1767,10 @@ __device__ __forceinline__ void layout_body(const EntropyDev& e, const unsigned 
         const unsigned long long total{framing + cs};
         sh_head = head_bytes;
         sh_start = framing + head_bytes;
-        sh_status = total > e.out_capacity ? 1ull : 0ull;
+        // 2: the file would reach the tokens kept at the buffer's end (never:
+        // dense_tokens).
+        const unsigned long long dense{e.direct ? 4ull * *e.tok_count : 0ull};
+        sh_status = total > e.out_capacity ? 1ull : (dense != 0 && total + dense > e.out_capacity ? 2ull : 0ull);
         e.result[0] = total;
         e.result[1] = sh_start;
         e.result[2] = sh_status;
@@ -1477,7 +1861,8 @@ __device__ __forceinline__ void ac_emit_body(const EntropyDev& e, const unsigned
     const Stripe st{e.stripes[blk]};
     const GroupGeom gg{ac_group_geom(e, st.group)};
     const int nitems{3 * st.rows * gg.gw};
-    if ((e.stripe_tok[2 * blk] != kNoTokens) != (kSet == kStoredStripes)) return;
+    const StripeTokens pool{stripe_tokens(e, st, blk, st.rows * gg.gw)};
+    if ((pool.near != nullptr) != (kSet == kStoredStripes)) return;
     if (kSet == kUnstoredStripes) stage_stripe(e, st, gg, s);
     if (tid == 0) {
         const Section sec{e.sections[st.section]};
@@ -1494,14 +1879,12 @@ __device__ __forceinline__ void ac_emit_body(const EntropyDev& e, const unsigned
     for (int i{tid}; i < nwords; i += kAcThreads) win[i] = 0;
     unsigned int* words{nwords >= 0 ? win : reinterpret_cast<unsigned int*>(e.out)};
     const unsigned long long base{nwords >= 0 ? (sh_start & 31) : sh_start};
-    const std::uint32_t tbase{e.stripe_tok[2 * blk]};
-    if (tbase != kNoTokens) {
+    if (pool.near != nullptr) {
         // Stored tokens in stream order: their lengths, a CTA scan for their
         // offsets, and their bits, kAcThreads * kPer tokens per round.
         __shared__ std::uint32_t sh_scan[kAcWarps + 1];
         constexpr int kPer{4};
         const std::uint32_t ntok{e.stripe_tok[2 * blk + 1]};
-        const std::uint32_t* pool{e.tok_pool + tbase};
         __syncthreads();
         unsigned long long run{base};
         for (std::uint32_t t0{0}; t0 < ntok; t0 += kAcThreads * kPer) {
@@ -1511,7 +1894,7 @@ __device__ __forceinline__ void ac_emit_body(const EntropyDev& e, const unsigned
 #pragma unroll
             for (int i{0}; i < kPer; ++i) {
                 const std::uint32_t t{t0 + static_cast<std::uint32_t>(tid) * kPer + i};
-                tk[i] = t < ntok ? pool[t] : 0u;
+                tk[i] = t < ntok ? *pool.at(t) : 0u;
                 len[i] = t < ntok ? __ldg(&e.ac_depth[token_table_index(tk[i])]) + token_extra_count(tk[i]) : 0u;
                 local += len[i];
             }
@@ -1752,7 +2135,7 @@ __device__ __forceinline__ int batch_frame(const EntropyBatch& b, int phase, uns
 // one launch: the two kinds are independent within a pass.
 __device__ __forceinline__ void tokens_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
     if (blk < static_cast<unsigned>(e.nstripes)) {
-        ac_tok_body(e, blk, nblk);
+        ac_tok_direct_body(e, blk);
     } else {
         misc_hist_body(e, blk - static_cast<unsigned>(e.nstripes), nblk);
     }
@@ -1805,21 +2188,6 @@ __device__ __forceinline__ bool frame_all_stored(const EntropyDev& e) { return *
             NAME##_body(e, s, 0u);                                                                            \
             __syncthreads();                                                                                  \
         }                                                                                                     \
-    }                                                                                                         \
-    __global__ void __launch_bounds__(kAcThreads) NAME##_batch_kernel(const __grid_constant__ EntropyBatch b) { \
-        const unsigned total{b.begin[kPhaseStripes][b.nframes]};                                              \
-        for (unsigned i{blockIdx.x}; i < total; i += gridDim.x) {                                             \
-            const int f{batch_frame(b, kPhaseStripes, i)};                                                    \
-            if (frame_all_stored(b.frames[f])) {                                                              \
-                /* on to this block's last stripe of frame f */                                               \
-                i += (b.begin[kPhaseStripes][f + 1] - 1 - i) / gridDim.x * gridDim.x;                         \
-                continue;                                                                                     \
-            }                                                                                                 \
-            const unsigned s{i - b.begin[kPhaseStripes][f]};                                                  \
-            if (b.frames[f].stripe_tok[2 * s] != kNoTokens) continue;                                         \
-            NAME##_body(b.frames[f], s, 0u);                                                                  \
-            __syncthreads();                                                                                  \
-        }                                                                                                     \
     }
 
 JXB_UNSTORED_KERNELS(lengths_unstored)
@@ -1834,6 +2202,15 @@ __global__ void __launch_bounds__(256) clear_batch_kernel(const __grid_constant_
     clear_body(b.frames[blockIdx.x], 0u, 1u);
 }
 
+// The token pass of planes given by the caller.
+__global__ void __launch_bounds__(kAcThreads) tokens_staged_kernel(const __grid_constant__ EntropyDev e) {
+    if (blockIdx.x < static_cast<unsigned>(e.nstripes)) {
+        ac_tok_body(e, blockIdx.x);
+    } else {
+        misc_hist_body(e, blockIdx.x - static_cast<unsigned>(e.nstripes), gridDim.x);
+    }
+}
+
 constexpr std::size_t kHistSmem{sizeof(StripeStage) + kNumClusters * kAcSymbols * sizeof(std::uint32_t)};
 constexpr std::size_t kBitsSmem{sizeof(StripeStage)};
 constexpr std::size_t kEmitSmem{sizeof(StripeStage) + kWindowWords * sizeof(unsigned int)};
@@ -1843,7 +2220,10 @@ constexpr std::size_t kEmitStoredSmem{kWindowWords * sizeof(unsigned int) >
                                           ? kWindowWords * sizeof(unsigned int)
                                           : kMiscWindowWords * sizeof(unsigned int) + kMaxDeferred * sizeof(DeferredBlob)};
 // The other items' passes share these launches and their shared memory.
-static_assert(kHistSmem >= (4 * 256 + 2) * sizeof(std::uint32_t), "token pass shared memory");
+constexpr std::size_t kDirectSmem{sizeof(DirectStage)};
+static_assert(kHistSmem >= (4 * 256 + 2) * sizeof(std::uint32_t) && kDirectSmem >= (4 * 256 + 2) * sizeof(std::uint32_t) &&
+                  kDirectSmem <= 48 * 1024,
+              "token pass shared memory");
 
 
 }  // namespace
@@ -1857,16 +2237,20 @@ bool entropy_launch(const EntropyDev& e, void* stream) {
     const unsigned stripes{static_cast<unsigned>(e.nstripes)};
     const std::uint32_t layout_smem{layout_sizes_bytes(e.nsec) + layout_head_bytes(e.nsec)};
     clear_kernel<<<clear_blocks(e.ndc), 256, 0, st>>>(e);  // histograms, first-block counts, pool fill
-    tokens_kernel<<<stripes + misc, kAcThreads, kHistSmem, st>>>(e);
+    if (e.direct) {
+        tokens_kernel<<<stripes + misc, kAcThreads, kDirectSmem, st>>>(e);
+    } else {
+        tokens_staged_kernel<<<stripes + misc, kAcThreads, kHistSmem, st>>>(e);
+    }
     codes_kernel<<<kNumClusters + 2 * e.ndc, 32, sizeof(WarpCodeSmem), st>>>(e);
     lengths_kernel<<<stripes + misc, kAcThreads, 0, st>>>(e);
-    lengths_unstored_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(e);
+    if (!e.direct) lengths_unstored_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(e);
     scan_tile_kernel<<<e.num_tiles, 1024, 0, st>>>(e);
     scan_top_kernel<<<1, 1024, 0, st>>>(e);
     layout_kernel<<<1, kLayoutThreads, layout_smem, st>>>(e);
     zero_body_kernel<<<kZeroBlocks, 256, 0, st>>>(e);
     emit_kernel<<<stripes + misc, kAcThreads, kEmitStoredSmem, st>>>(e);
-    emit_unstored_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(e);
+    if (!e.direct) emit_unstored_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(e);
     return cudaGetLastError() == cudaSuccess;
 }
 
@@ -1877,7 +2261,7 @@ void entropy_batch_plan(EntropyBatch& b) {
         const std::uint32_t per[kEntropyPhases]{static_cast<std::uint32_t>(e.nstripes) +
                                                      (e.ac_first + kMiscItemsPerBlock - 1) / kMiscItemsPerBlock,
                                                  static_cast<std::uint32_t>(kNumClusters + 2 * e.ndc), e.num_tiles,
-                                                 1u, kZeroBlocksBatched, static_cast<std::uint32_t>(e.nstripes)};
+                                                 1u, kZeroBlocksBatched};
         for (int p{0}; p < kEntropyPhases; ++p) b.begin[p][f + 1] = b.begin[p][f] + per[p];
     }
 }
@@ -1894,16 +2278,14 @@ bool entropy_batch_launch(const EntropyBatch& b, void* stream) {
     const int nf{b.nframes};
     const unsigned items{b.begin[kPhaseItems][nf]};
     clear_batch_kernel<<<static_cast<unsigned>(nf), 256, 0, st>>>(b);
-    tokens_batch_kernel<<<items, kAcThreads, kHistSmem, st>>>(b);
+    tokens_batch_kernel<<<items, kAcThreads, kDirectSmem, st>>>(b);
     codes_batch_kernel<<<b.begin[kPhaseCodes][nf], 32, sizeof(WarpCodeSmem), st>>>(b);
     lengths_batch_kernel<<<items, kAcThreads, 0, st>>>(b);
-    lengths_unstored_batch_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(b);
     scan_tile_batch_kernel<<<b.begin[kPhaseScan][nf], 1024, 0, st>>>(b);
     scan_top_batch_kernel<<<static_cast<unsigned>(nf), 1024, 0, st>>>(b);
     layout_batch_kernel<<<static_cast<unsigned>(nf), kLayoutThreads, layout_smem, st>>>(b);
     zero_body_batch_kernel<<<b.begin[kPhaseZero][nf], 256, 0, st>>>(b);
     emit_batch_kernel<<<items, kAcThreads, kEmitStoredSmem, st>>>(b);
-    emit_unstored_batch_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(b);
     return cudaGetLastError() == cudaSuccess;
 }
 
@@ -1951,7 +2333,7 @@ bool entropy_kernels_init() {
                                 static_cast<int>(sizeof(WarpCodeSmem))) == cudaSuccess &&
            cudaFuncSetAttribute(layout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kLayoutSmemLimit)) == cudaSuccess &&
-           cudaFuncSetAttribute(tokens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+           cudaFuncSetAttribute(tokens_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kHistSmem)) == cudaSuccess &&
            cudaFuncSetAttribute(lengths_unstored_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kBitsSmem)) == cudaSuccess &&
@@ -1960,13 +2342,7 @@ bool entropy_kernels_init() {
            cudaFuncSetAttribute(codes_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(sizeof(WarpCodeSmem))) == cudaSuccess &&
            cudaFuncSetAttribute(layout_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kLayoutSmemLimit)) == cudaSuccess &&
-           cudaFuncSetAttribute(tokens_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kHistSmem)) == cudaSuccess &&
-           cudaFuncSetAttribute(lengths_unstored_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kBitsSmem)) == cudaSuccess &&
-           cudaFuncSetAttribute(emit_unstored_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kEmitSmem)) == cudaSuccess;
+                                static_cast<int>(kLayoutSmemLimit)) == cudaSuccess;
 }
 
 }  // namespace jxb

@@ -14,12 +14,12 @@
 //   4. a layout CTA sizes every section, writes the container, headers and
 //      TOC, and places the sections;
 //   5. an emit pass writes every item's bits at its final position.
-// Passes 1, 3 and 5 are one launch each: a CTA per AC stripe (one warp per
-// block-channel while tokenising, stored tokens afterwards), then a CTA per
-// 512 other items (two per thread); passes 3 and 5 take stripes whose
-// tokens did not fit the pool in one more launch each, with their
-// coefficients staged again. A clear kernel zeroes the histograms and the
-// pool fill first.
+// Passes 1, 3 and 5 are one launch each: a CTA per AC stripe (one thread per
+// token), then a CTA per 512 other items (two per thread). Planes given by
+// the caller are tokenised a warp per block-channel instead, and stripes whose
+// tokens did not fit the pool go through passes 3 and 5 in one more launch
+// each, with their coefficients staged again. A clear kernel zeroes the
+// histograms and the pool fill first.
 #pragma once
 
 #include <cstddef>
@@ -73,6 +73,7 @@ struct EntropyDev {
 
     // constant tables
     const std::uint16_t* order;      // natural orders: 64 (DCT8) | 256 (DCT16) | 1024 (DCT32)
+    const std::uint16_t* rank;       // their inverses: scan position of each raw index (direct passes only)
     const std::uint8_t* pre_const;   // DcGroup header bits before the DC code description
     std::uint32_t pre_const_bits;
     const std::uint8_t* mid_const;   // AcMetadata header bits after the count field
@@ -103,14 +104,20 @@ struct EntropyDev {
     unsigned long long* sec_pos;     // [nsec] absolute bit offset of each section in `out`
     unsigned long long* result;      // [4]: total bytes, body start, status, 0
 
-    // AC tokens, written once by the histogram pass and read by the bit-length
-    // and emission passes: each stripe reserves a contiguous run of the pool
-    // (stream order); a stripe that finds the pool full keeps its tokens
-    // unstored and the later passes tokenise its coefficients again.
+    // AC tokens, written once by the token pass in stream order and read by
+    // the bit-length and emission passes. `direct`: the planes come from the
+    // frontend, and each stripe has kTokensPerBlock places a block in the
+    // pool; the tokens of a stripe that has more go to the end of the output
+    // buffer, which the file does not reach. Otherwise (planes given by the
+    // caller, which may break the block layout, and a buffer of any size) each
+    // stripe reserves a contiguous run of the pool; one that finds it full
+    // keeps its tokens unstored and the later passes tokenise its
+    // coefficients again.
+    bool direct;
     std::uint32_t* tok_pool;         // [tok_capacity] packed tokens (pack_ac_token)
     std::uint32_t tok_capacity;
-    std::uint32_t* tok_count;        // [1] pool fill, zeroed per frame
-    std::uint32_t* stripe_tok;       // [2 * nstripes]: pool offset or kNoTokens, token count
+    std::uint32_t* tok_count;        // [1] pool fill, or tokens at the output's end (direct); zeroed per frame
+    std::uint32_t* stripe_tok;       // [2 * nstripes]: place (pool offset or kNoTokens, or dense_tokens offset), token count
     std::uint8_t* out;               // output buffer (container + codestream)
     std::size_t out_capacity;
 };
@@ -120,6 +127,9 @@ constexpr int kScanTile = 4096;
 // Token pool capacity per 8x8 block: 4K frames at distance 0.5 use about 27,
 // at distance 1 about 11.
 constexpr std::uint32_t kTokensPerBlock = 32;
+// A block's tokens at most: three channels of one count and 63 coefficients
+// (DCT8; larger transforms have fewer a block).
+constexpr std::uint32_t kMaxTokensPerBlock = 192;
 constexpr std::uint32_t kNoTokens = 0xffffffffu;
 
 // Shared memory of the layout kernel: one 32-bit size per section, then the
@@ -148,6 +158,7 @@ struct EntropyHostPlan {
     std::vector<std::uint8_t> ac_prefix;
     std::uint32_t ac_prefix_bits{0};
     std::vector<std::uint16_t> order;
+    std::vector<std::uint16_t> rank;  // inverse of each order, concatenated likewise
 };
 EntropyHostPlan entropy_plan(int width, int height);
 
@@ -173,8 +184,7 @@ enum EntropyPhase : int {
     kPhaseScan = 2,     // item scan tiles
     kPhaseFrame = 3,    // one block per frame
     kPhaseZero = 4,     // body zeroing
-    kPhaseStripes = 5,  // AC stripes whose tokens did not fit the pool
-    kEntropyPhases = 6
+    kEntropyPhases = 5
 };
 struct EntropyBatch {
     int nframes;

@@ -277,6 +277,9 @@ EntropyHostPlan entropy_plan(int width, int height) {
             }
         }
         p.order.insert(p.order.end(), out.begin(), out.end());
+        std::vector<std::uint16_t> rank(out.size());
+        for (std::size_t k{0}; k < out.size(); ++k) rank[out[k]] = static_cast<std::uint16_t>(k);
+        p.rank.insert(p.rank.end(), rank.begin(), rank.end());
     }
     return p;
 }
