@@ -1008,6 +1008,7 @@ struct WarpCodeSmem {
     std::uint8_t depth[256];
     std::uint16_t bits[256];
     std::uint16_t used[256];           // compacted list of used symbols
+    alignas(16) std::uint32_t used_cnt[256 + 4];  // their counts, padded to a multiple of four
     std::uint32_t len_count[18];       // depths per code length (canonical codes, header)
     std::uint32_t len_next[18];
     alignas(4) std::uint8_t desc[kDescBytes];
@@ -1044,58 +1045,78 @@ __device__ void warp_create_tree(WarpCodeSmem& s, const std::uint32_t* hist, int
         const int sym{base + lane};
         const bool used{sym < length && hist[sym] != 0};
         const unsigned m{__ballot_sync(kFull, used)};
-        if (used) s.used[n + __popc(m & ((1u << lane) - 1u))] = static_cast<std::uint16_t>(sym);
+        if (used) {
+            const int at{n + __popc(m & ((1u << lane) - 1u))};
+            s.used[at] = static_cast<std::uint16_t>(sym);
+            s.used_cnt[at] = hist[sym];
+        }
         n += __popc(m);
     }
+    constexpr std::uint32_t kInf{0xffffffffu};
+    if (lane < 4) s.used_cnt[n + lane] = kInf;
     __syncwarp();
     if (n < 2) {
         if (n == 1 && lane == 0) depth[s.used[0]] = 1;
         __syncwarp();
         return;
     }
+    // Rank of used symbol i: those with a smaller count, or the same count and
+    // a larger symbol (a later place in the list), come before it.
     for (int i{lane}; i < n; i += 32) {
-        const int sym{s.used[i]};
-        const std::uint32_t c{hist[sym]};
+        const std::uint32_t c{s.used_cnt[i]};
         int rank{0};
-        for (int t{0}; t < n; ++t) {
-            const int ts{s.used[t]};
-            const std::uint32_t ct{hist[ts]};
-            rank += (ct < c || (ct == c && ts > sym)) ? 1 : 0;
+        for (int t{0}; t < n; t += 4) {
+            const uint4 q{*reinterpret_cast<const uint4*>(&s.used_cnt[t])};
+            rank += (q.x < c || (q.x == c && t > i)) ? 1 : 0;
+            rank += (q.y < c || (q.y == c && t + 1 > i)) ? 1 : 0;
+            rank += (q.z < c || (q.z == c && t + 2 > i)) ? 1 : 0;
+            rank += (q.w < c || (q.w == c && t + 3 > i)) ? 1 : 0;
         }
         s.cnt[rank] = c;
-        s.leaf_sym[rank] = static_cast<std::uint16_t>(sym);
+        s.leaf_sym[rank] = s.used[i];
     }
     __syncwarp();
-    // Lane L: floor 2^L, leaf r has count max(cnt[r], 2^L - 1).
-    constexpr std::uint32_t kInf{0xffffffffu};
+    // Lane L: floor 2^L, leaf r has count max(cnt[r], 2^L - 1). The heads of
+    // both queues and the entries behind them are held in registers, so one
+    // step (two picks) waits for one round of loads.
     const std::uint32_t fm1{lane == 31 ? 0x7fffffffu : (1u << lane) - 1u};
     std::uint32_t* icnt{s.icnt + lane};
     std::uint8_t* height{s.height + lane};
     std::int16_t* parent{s.parent + lane};
     int i{0};
     int j{0};
+    std::uint32_t a0{max(s.cnt[0], fm1)};  // leaves i and i + 1 (n is at least 2)
+    std::uint32_t a1{max(s.cnt[1], fm1)};
+    std::uint32_t b0{kInf};                // internal nodes j and j + 1
+    std::uint32_t b1{kInf};
+    int h0{0};
+    int h1{0};
     for (int t{0}; t < n - 1; ++t) {
-        int node[2];
-        std::uint32_t sum{0};
-        int h{0};
-#pragma unroll
-        for (int k{0}; k < 2; ++k) {
-            const std::uint32_t li{i < n ? max(s.cnt[i < n ? i : 0], fm1) : kInf};
-            const std::uint32_t lj{j < t ? icnt[32 * (j < t ? j : 0)] : kInf};
-            const bool leaf{li <= lj};
-            node[k] = leaf ? i : n + j;
-            // Saturating: only floors far above any that can fit reach it.
-            const std::uint32_t v{leaf ? li : lj};
-            sum = sum > kInf - 1u - v ? kInf - 1u : sum + v;
-            const int hk{leaf ? 0 : static_cast<int>(height[32 * (j < t ? j : 0)])};
-            h = max(h, hk);
-            i += leaf ? 1 : 0;
-            j += leaf ? 0 : 1;
-        }
+        const bool leaf0{a0 <= b0};
+        const std::uint32_t a{leaf0 ? a1 : a0};
+        const std::uint32_t b{leaf0 ? b0 : b1};
+        const bool leaf1{a <= b};
+        const std::uint32_t v0{leaf0 ? a0 : b0};
+        const std::uint32_t v1{leaf1 ? a : b};
+        // Saturating: only floors far above any that can fit reach it.
+        const std::uint32_t sum{v0 > kInf - 1u - v1 ? kInf - 1u : v0 + v1};
+        const int h{max(leaf0 ? 0 : h0, leaf1 ? 0 : (leaf0 ? h0 : h1))};
+        parent[32 * (leaf0 ? i : n + j)] = static_cast<std::int16_t>(n + t);
+        i += leaf0 ? 1 : 0;
+        j += leaf0 ? 0 : 1;
+        parent[32 * (leaf1 ? i : n + j)] = static_cast<std::int16_t>(n + t);
+        i += leaf1 ? 1 : 0;
+        j += leaf1 ? 0 : 1;
         icnt[32 * t] = sum;
         height[32 * t] = static_cast<std::uint8_t>(h + 1);
-        parent[32 * node[0]] = static_cast<std::int16_t>(n + t);
-        parent[32 * node[1]] = static_cast<std::int16_t>(n + t);
+        // The next heads; nodes up to t exist (entries of leaves past the
+        // last, and of nodes past t, never win a pick).
+        a0 = i < n ? max(s.cnt[min(i, n - 1)], fm1) : kInf;
+        a1 = i + 1 < n ? max(s.cnt[min(i + 1, n - 1)], fm1) : kInf;
+        b0 = j <= t ? icnt[32 * min(j, t)] : kInf;
+        b1 = j + 1 <= t ? icnt[32 * min(j + 1, t)] : kInf;
+        h0 = height[32 * min(j, t)];
+        h1 = height[32 * min(j + 1, t)];
     }
     const int root_h{static_cast<int>(height[32 * (n - 2)])};
     const unsigned fit{__ballot_sync(kFull, root_h <= limit)};
@@ -1138,13 +1159,12 @@ __device__ void warp_canonical_codes(WarpCodeSmem& s, const std::uint8_t* depth,
         if (d != 0 && (__ffs(peers) - 1) == lane) s.len_count[d] += static_cast<std::uint32_t>(__popc(peers));
     }
     __syncwarp();
-    if (lane == 0) {
-        std::uint32_t code{0};
-        s.len_next[0] = 0;
-        for (int i{1}; i < 16; ++i) {
-            code = (code + (i - 1 == 0 ? 0u : s.len_count[i - 1])) << 1;
-            s.len_next[i] = code;
-        }
+    // First code of each length, next[l] = (next[l - 1] + count[l - 1]) << 1,
+    // as a sum of the shorter lengths' counts in units of 2^-15.
+    {
+        const std::uint32_t share{lane > 0 && lane < 16 ? s.len_count[lane] << (15 - lane) : 0u};
+        const std::uint32_t before{warp_incl_scan(share, lane) - share};
+        if (lane < 16) s.len_next[lane] = before >> (15 - lane);
     }
     __syncwarp();
     const unsigned below{(1u << lane) - 1u};
@@ -1202,46 +1222,30 @@ __device__ void warp_store_complex(WarpCodeSmem& s, int num, BitSink& w, int lan
     __syncwarp();
     warp_create_tree(s, scr.hist, 18, 5, scr.cl_depth, lane);
     warp_canonical_codes(s, scr.cl_depth, 18, scr.cl_bits, lane);
-    std::uint32_t pos{0};
-    if (lane == 0) {
-        std::uint32_t* hist{scr.hist};
-        int num_codes{0};
-        int code{0};
-        for (int i{0}; i < 18; ++i) {
-            if (hist[i]) {
-                if (num_codes == 0) {
-                    code = i;
-                    num_codes = 1;
-                } else if (num_codes == 1) {
-                    num_codes = 2;
-                    break;
-                }
-            }
-        }
-        std::uint8_t* cl_depth{scr.cl_depth};
-        constexpr std::uint8_t kOrder[18]{1, 2, 3, 4, 0, 5, 17, 6, 16, 7, 8, 9, 10, 11, 12, 13, 14, 15};
-        constexpr std::uint8_t kSym[6]{0, 7, 3, 2, 1, 15};
-        constexpr std::uint8_t kLen[6]{2, 4, 3, 2, 2, 4};
-        int to_store{18};
-        if (num_codes > 1) {
-            for (; to_store > 0; --to_store) {
-                if (cl_depth[kOrder[to_store - 1]] != 0) break;
-            }
-        }
-        std::uint32_t skip{0};
-        if (cl_depth[kOrder[0]] == 0 && cl_depth[kOrder[1]] == 0) {
-            skip = 2;
-            if (cl_depth[kOrder[2]] == 0) skip = 3;
-        }
-        w.put(2, skip);
-        for (int i{static_cast<int>(skip)}; i < to_store; ++i) {
-            const int l{cl_depth[kOrder[i]]};
-            w.put(kLen[l], kSym[l]);
-        }
-        if (num_codes == 1) cl_depth[code] = 0;
-        pos = w.pos;
-    }
-    pos = __shfl_sync(kFull, pos, 0);
+    // Code-length-code header: lane i takes entry i of the transmission order
+    // {1, 2, 3, 4, 0, 5, 17, 6, 16, 7, ..., 15} (six bits each below), whose
+    // depth 0..5 is sent as {length, code} {2,0} {4,7} {3,3} {2,2} {2,1} {4,15}
+    // (four bits each).
+    const unsigned used{__ballot_sync(kFull, lane < 18 && scr.hist[lane] != 0)};
+    const int num_codes{__popc(used)};
+    const std::uint64_t lo10{1ull | 2ull << 6 | 3ull << 12 | 4ull << 18 | 0ull << 24 | 5ull << 30 | 17ull << 36 |
+                             6ull << 42 | 16ull << 48 | 7ull << 54};
+    const std::uint64_t hi8{8ull | 9ull << 6 | 10ull << 12 | 11ull << 18 | 12ull << 24 | 13ull << 30 | 14ull << 36 |
+                            15ull << 42};
+    const int entry{lane < 10 ? static_cast<int>((lo10 >> (6 * lane)) & 63u)
+                              : (lane < 18 ? static_cast<int>((hi8 >> (6 * (lane - 10))) & 63u) : 0)};
+    const int l{lane < 18 ? scr.cl_depth[entry] : 0};
+    const unsigned sent{__ballot_sync(kFull, l != 0)};
+    const int to_store{num_codes > 1 ? 32 - __clz(static_cast<int>(sent)) : 18};
+    const int skip{(sent & 3u) != 0 ? 0 : ((sent & 4u) != 0 ? 2 : 3)};
+    const std::uint32_t ln{lane >= skip && lane < to_store ? (0x422342u >> (4 * l)) & 15u : 0u};
+    const std::uint32_t lincl{warp_incl_scan(ln, lane)};
+    std::uint32_t pos{__shfl_sync(kFull, w.pos, 0)};
+    if (lane == 0) or_bits(w.buf, pos, 2, static_cast<std::uint32_t>(skip), w.cap);
+    or_bits(w.buf, pos + 2 + lincl - ln, ln, (0xf12370u >> (4 * l)) & 15u, w.cap);
+    pos += 2 + __shfl_sync(kFull, lincl, 31);
+    __syncwarp();
+    if (num_codes == 1 && lane == 0) scr.cl_depth[__ffs(used) - 1] = 0;
     __syncwarp();
     const std::uint32_t cap{w.cap};
     for (int base{0}; base < new_len; base += 32) {
