@@ -50,6 +50,7 @@ struct cujpegxl_encoder {
     unsigned long long* result_pinned{nullptr};
     std::size_t arena_bytes{0};
     bool pending{false};
+    bool half_launched{false};    // an entropy stage did not launch in full
     bool frontend_planes{false};  // the quantised planes are the frontend's own, not a caller's
     // Learned decisions: the attached network (not owned), its margin and
     // flags, and the per-frame decision buffers in the arena.
@@ -175,8 +176,7 @@ cujpegxl_status validate_config(const cujpegxl_config& c, bool allow_single = fa
     }
     const std::size_t nac{((c.width / 8 + 31) / 32) * static_cast<std::size_t>((c.height / 8 + 31) / 32)};
     if (nac <= 1 && !allow_single) return CUJPEGXL_UNSUPPORTED_RESOLUTION;
-    // The TOC is written in one CTA's shared memory: about 25,000 sections
-    // (1.6 gigapixels) at most.
+    // About 25,000 sections (1.6 gigapixels) at most.
     const std::size_t ndc{((c.width / 8 + 255) / 256) * static_cast<std::size_t>((c.height / 8 + 255) / 256)};
     if (2 + ndc + nac > static_cast<std::size_t>(jxb::kMaxSections)) return CUJPEGXL_UNSUPPORTED_RESOLUTION;
     return CUJPEGXL_OK;
@@ -215,7 +215,7 @@ bool allocate(cujpegxl_encoder* e) {
     const jxb::EntropyHostPlan plan{jxb::entropy_plan(static_cast<int>(W), static_cast<int>(H))};
     const int ndc{static_cast<int>(((bw + 255) / 256) * ((bh + 255) / 256))};
     const int nac{static_cast<int>(((bw + 31) / 32) * ((bh + 31) / 32))};
-    const std::uint32_t tiles{(plan.total_items + jxb::kScanTile - 1) / jxb::kScanTile};
+    const std::size_t units{plan.unit_section.size()};
     const std::size_t out_cap{(jxb::worst_case_output(W, H) + 15) & ~static_cast<std::size_t>(15)};
 
     ArenaPlan a;
@@ -235,12 +235,18 @@ bool allocate(cujpegxl_encoder* e) {
     const std::size_t o_mid{a.take(plan.mid_const.size())};
     const std::size_t o_acp{a.take(plan.ac_prefix.size())};
     const std::size_t o_dcg{a.take(64)};
+    const std::size_t o_msec{a.take(units * 4)};
+    const std::size_t o_zero{a.total};  // from here: zero between encodes
     const std::size_t o_ach{a.take(32 * 256 * 4)};
     const std::size_t o_dch{a.take(static_cast<std::size_t>(ndc) * 256 * 4)};
     const std::size_t o_amh{a.take(static_cast<std::size_t>(ndc) * 256 * 4)};
     const std::size_t o_fb{a.take(static_cast<std::size_t>(ndc) * 4)};
+    const std::size_t o_tokn{a.take(4)};
+    const std::size_t zero_bytes{a.total - o_zero};
+    const std::size_t o_froz{a.take((1 + static_cast<std::size_t>(ndc)) * 4)};
     const std::size_t o_acd{a.take(32 * 256)};
     const std::size_t o_acb{a.take(32 * 256 * 2)};
+    const std::size_t o_code{a.take((32 * 64 + static_cast<std::size_t>(ndc) * 2 * 128) * 4)};
     const std::size_t o_dcd{a.take(static_cast<std::size_t>(ndc) * 256)};
     const std::size_t o_dcb{a.take(static_cast<std::size_t>(ndc) * 256 * 2)};
     const std::size_t o_amd{a.take(static_cast<std::size_t>(ndc) * 256)};
@@ -248,16 +254,16 @@ bool allocate(cujpegxl_encoder* e) {
     const std::size_t o_alpha{a.take(32 * 4)};
     const std::size_t o_desc{a.take(static_cast<std::size_t>(32 + 2 * ndc) * jxb::kDescBytes)};
     const std::size_t o_descb{a.take(static_cast<std::size_t>(32 + 2 * ndc) * 4)};
-    const std::size_t o_ib{a.take(static_cast<std::size_t>(plan.total_items) * 4)};
     const std::size_t o_ip{a.take(static_cast<std::size_t>(plan.total_items) * 4)};
-    const std::size_t o_ts{a.take(static_cast<std::size_t>(tiles) * 4)};
-    const std::size_t o_to{a.take(static_cast<std::size_t>(tiles + 1) * 8)};
+    const std::size_t o_it{a.take(static_cast<std::size_t>(plan.ac_first) * 4)};
+    const std::size_t o_us{a.take(jxb::unit_words(plan) * 4)};
+    const std::size_t o_uo{a.take(jxb::unit_words(plan) * 8)};
+    const std::size_t o_up{a.take(units * 8)};
     const std::size_t o_sp{a.take(plan.sections.size() * 8)};
     const std::size_t o_res{a.take(4 * 8)};
     const std::size_t tok_words{nb * jxb::kTokensPerBlock};
     const std::uint32_t tok_cap{static_cast<std::uint32_t>(std::min<std::size_t>(tok_words, 0xfffffff0u))};
     const std::size_t o_tok{a.take(tok_words * 4)};
-    const std::size_t o_tokn{a.take(4)};
     const std::size_t o_stok{a.take(plan.stripes.size() * 8)};
     const std::size_t o_out{a.take(out_cap)};
     const std::size_t o_nv12{a.take(static_cast<std::size_t>(W) * H * 3 / 2)};
@@ -308,7 +314,11 @@ bool allocate(cujpegxl_encoder* e) {
     ed.nsec = static_cast<int>(plan.sections.size());
     ed.total_items = plan.total_items;
     ed.ac_first = plan.ac_first;
-    ed.num_tiles = tiles;
+    ed.misc_units = plan.misc_units;
+    ed.unit_section = reinterpret_cast<const std::uint32_t*>(b + o_msec);
+    for (int i{0}; i < 4; ++i) ed.head_words[i] = plan.head_words[i];
+    ed.head_bytes = plan.head_bytes;
+    ed.clear_first = false;
     ed.sections = reinterpret_cast<const jxb::Section*>(b + o_sec);
     ed.stripes = reinterpret_cast<const jxb::Stripe*>(b + o_str);
     ed.nstripes = static_cast<int>(plan.stripes.size());
@@ -335,8 +345,10 @@ bool allocate(cujpegxl_encoder* e) {
     ed.dc_hist = reinterpret_cast<std::uint32_t*>(b + o_dch);
     ed.am_hist = reinterpret_cast<std::uint32_t*>(b + o_amh);
     ed.fb_count = reinterpret_cast<std::uint32_t*>(b + o_fb);
+    ed.frozen = reinterpret_cast<std::uint32_t*>(b + o_froz);
     ed.ac_depth = b + o_acd;
     ed.ac_bits = reinterpret_cast<std::uint16_t*>(b + o_acb);
+    ed.code = reinterpret_cast<std::uint32_t*>(b + o_code);
     ed.dc_depth = b + o_dcd;
     ed.dc_bits = reinterpret_cast<std::uint16_t*>(b + o_dcb);
     ed.am_depth = b + o_amd;
@@ -344,11 +356,12 @@ bool allocate(cujpegxl_encoder* e) {
     ed.ac_alpha = reinterpret_cast<std::uint32_t*>(b + o_alpha);
     ed.desc = b + o_desc;
     ed.desc_bits = reinterpret_cast<std::uint32_t*>(b + o_descb);
-    ed.item_bits = reinterpret_cast<std::uint32_t*>(b + o_ib);
     ed.item_pre = reinterpret_cast<std::uint32_t*>(b + o_ip);
-    ed.tile_sum = reinterpret_cast<std::uint32_t*>(b + o_ts);
-    ed.tile_off = reinterpret_cast<unsigned long long*>(b + o_to);
-    ed.sec_pos = reinterpret_cast<unsigned long long*>(b + o_sp);
+    ed.item_tok = reinterpret_cast<std::uint32_t*>(b + o_it);
+    ed.unit_sum = reinterpret_cast<std::uint32_t*>(b + o_us);
+    ed.unit_off = reinterpret_cast<unsigned long long*>(b + o_uo);
+    ed.unit_pos = reinterpret_cast<unsigned long long*>(b + o_up);
+    ed.sec_shift = reinterpret_cast<unsigned long long*>(b + o_sp);
     ed.result = reinterpret_cast<unsigned long long*>(b + o_res);
     ed.tok_pool = reinterpret_cast<std::uint32_t*>(b + o_tok);
     ed.tok_capacity = tok_cap;
@@ -375,6 +388,9 @@ bool allocate(cujpegxl_encoder* e) {
                 cudaSuccess &&
             cudaMemcpy(b + o_acp, plan.ac_prefix.data(), plan.ac_prefix.size(), cudaMemcpyHostToDevice) ==
                 cudaSuccess};
+    ok = ok && cudaMemcpy(b + o_msec, plan.unit_section.data(), units * 4, cudaMemcpyHostToDevice) ==
+                   cudaSuccess &&
+         cudaMemset(b + o_zero, 0, zero_bytes) == cudaSuccess;
     ok = ok && acquire_pinned(reinterpret_cast<void**>(&e->nv12_pinned), static_cast<std::size_t>(W) * H * 3 / 2 + 64);
     if (!ok) {
         release(e);
@@ -408,6 +424,17 @@ bool prepare(cujpegxl_encoder* e) {
     return set_distance(e);
 }
 
+// The entropy stage on the encoder's planes. A sequence that failed to launch
+// half-way leaves histograms that the next one has to clear.
+bool launch_entropy(cujpegxl_encoder* e, std::uint32_t dc_global_bits, bool direct, cudaStream_t st) {
+    jxb::EntropyDev ed{e->ed};
+    ed.dc_global_bits = dc_global_bits;
+    ed.direct = direct;
+    ed.clear_first = e->half_launched;
+    e->half_launched = !jxb::entropy_launch(ed, st);
+    return !e->half_launched;
+}
+
 bool enqueue_frame(cujpegxl_encoder* e, const std::uint8_t* luma, std::size_t lp, const std::uint8_t* chroma,
                    std::size_t cp, std::uint32_t stages = 3u, cudaStream_t stream = nullptr) {
     jxb::FrontendTables ft{};
@@ -431,11 +458,8 @@ bool enqueue_frame(cujpegxl_encoder* e, const std::uint8_t* luma, std::size_t lp
         e->frontend_planes = true;
     }
     if ((stages & 2u) == 0) return true;
-    if (e->frontend_planes) return jxb::entropy_launch(e->ed, st);
-    // The entropy stage alone over planes that no frontend wrote.
-    jxb::EntropyDev ed{e->ed};
-    ed.direct = false;
-    return jxb::entropy_launch(ed, st);
+    // Not direct: the entropy stage alone over planes that no frontend wrote.
+    return launch_entropy(e, e->ed.dc_global_bits, e->frontend_planes, st);
 }
 
 cujpegxl_status finish(cujpegxl_encoder* e, cujpegxl_output* output);
@@ -852,13 +876,10 @@ cujpegxl_status cujpegxl_b200_encode_planes(cujpegxl_encoder* encoder, const cuj
     // The DcGlobal blob now belongs to these planes; force a refresh on the next encode.
     encoder->geo_distance = -1.0f;
     encoder->frontend_planes = false;
-    jxb::EntropyDev ed{encoder->ed};
-    ed.dc_global_bits = nbits;
-    ed.direct = false;
     nz_kernel<<<static_cast<unsigned>((nb + 255) / 256), 256, 0, st>>>(
         encoder->fo.ac, encoder->fo.acs, static_cast<int>(W / 8), static_cast<int>(H / 8), encoder->fo.nzn,
         encoder->fo.nzc);
-    ok = cudaGetLastError() == cudaSuccess && jxb::entropy_launch(ed, st);
+    ok = cudaGetLastError() == cudaSuccess && launch_entropy(encoder, nbits, false, st);
     if (!ok) return CUJPEGXL_INTERNAL_ERROR;
     return finish(encoder, output);
 }
@@ -965,7 +986,7 @@ cujpegxl_status cujpegxl_b200_encoder_memory(cujpegxl_encoder* encoder, size_t* 
     return CUJPEGXL_OK;
 }
 
-uint32_t cujpegxl_b200_kernels_per_encode(void) { return 12u; }
+uint32_t cujpegxl_b200_kernels_per_encode(void) { return 6u; }
 
 void cujpegxl_b200_debug_fail_allocation(uint32_t nth) { g_fail_countdown.store(nth); }
 

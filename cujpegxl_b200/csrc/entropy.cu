@@ -34,17 +34,11 @@ constexpr unsigned kFull = 0xffffffffu;
 // Token channel order Y, X, B over planes stored X, Y, B.
 __device__ __forceinline__ int phys_channel(int p) { return p == 0 ? 1 : (p == 1 ? 0 : 2); }
 
-// Section holding `item`, searched in sections [lo, hi].
-__device__ __forceinline__ int find_section(const Section* secs, int lo, int hi, std::uint32_t item) {
-    while (lo < hi) {
-        const int mid{(lo + hi + 1) >> 1};
-        if (__ldg(&secs[mid].first) <= item) {
-            lo = mid;
-        } else {
-            hi = mid - 1;
-        }
-    }
-    return lo;
+// Section holding `item`, which lies in section s or a little later.
+__device__ __forceinline__ Section section_from(const EntropyDev& e, int& s, std::uint32_t item) {
+    Section sec{e.sections[s]};
+    while (item >= sec.first + sec.count) sec = e.sections[++s];
+    return sec;
 }
 
 struct GroupGeom {
@@ -62,8 +56,9 @@ __device__ __forceinline__ GroupGeom ac_group_geom(const EntropyDev& e, int g) {
 
 __device__ __forceinline__ GroupGeom dc_group_geom(const EntropyDev& e, int g) {
     GroupGeom r;
-    r.bx0 = (g % e.xdg) * kDcGroupBlocks;
-    r.by0 = (g / e.xdg) * kDcGroupBlocks;
+    const int gy{e.xdg == 1 ? g : g / e.xdg};
+    r.bx0 = (g - gy * e.xdg) * kDcGroupBlocks;
+    r.by0 = gy * kDcGroupBlocks;
     r.gw = min(kDcGroupBlocks, e.bw - r.bx0);
     r.gh = min(kDcGroupBlocks, e.bh - r.by0);
     return r;
@@ -71,18 +66,21 @@ __device__ __forceinline__ GroupGeom dc_group_geom(const EntropyDev& e, int g) {
 
 enum TokTable : int { kTabDc = 1, kTabAm = 2 };
 
-__device__ __forceinline__ int misc_hi(const EntropyDev& e) { return e.ndc + 1; }
-
 // ---- items other than AC block-channels -------------------------------------------
 
-// Visits the bits of one non-AC item in stream order: blob(bytes, nbits),
-// varlen(v), count_field(group, nbits), epf(group), first_block(group),
+// a / b for a < 2^23 and b < 2^16: the float quotient is within one of it.
+__device__ __forceinline__ std::uint32_t div_small(std::uint32_t a, std::uint32_t b) {
+    std::uint32_t q{static_cast<std::uint32_t>(__fdividef(static_cast<float>(a), static_cast<float>(b)))};
+    if (q * b > a) --q;
+    if (a - q * b >= b) ++q;
+    return q;
+}
+
+// Visits the bits of non-AC item j of section `sec` in stream order:
+// blob(bytes, nbits), varlen(v), count_field(group, nbits), epf(group), first_block(group),
 // token(table, group, symbol, extra_bits, extra_value).
 template <class V>
-__device__ void visit_misc(const EntropyDev& e, std::uint32_t item, V& v) {
-    const int s{find_section(e.sections, 0, misc_hi(e), item)};
-    const Section sec{e.sections[s]};
-    const std::uint32_t j{item - sec.first};
+__device__ void visit_misc(const EntropyDev& e, const Section& sec, std::uint32_t j, V& v) {
     if (sec.kind == kSecDcGlobal) {
         v.blob(e.dc_global, e.dc_global_bits);
         return;
@@ -100,6 +98,11 @@ __device__ void visit_misc(const EntropyDev& e, std::uint32_t item, V& v) {
     const int g{sec.group};
     const GroupGeom gg{dc_group_geom(e, g)};
     const std::uint32_t n{static_cast<std::uint32_t>(gg.gw * gg.gh)};
+    // Row and column of block b of the group.
+    auto locate = [&](std::uint32_t b, int& x, int& y) {
+        y = static_cast<int>(div_small(b, static_cast<std::uint32_t>(gg.gw)));
+        x = static_cast<int>(b) - y * gg.gw;
+    };
     if (j == 0) {
         v.blob(e.pre_const, e.pre_const_bits);
         return;
@@ -110,10 +113,12 @@ __device__ void visit_misc(const EntropyDev& e, std::uint32_t item, V& v) {
     }
     if (j < 2 + 3 * n) {
         const std::uint32_t sidx{j - 2};
-        const int c{phys_channel(static_cast<int>(sidx / n))};
-        const std::uint32_t bp{sidx % n};
-        const int bx{gg.bx0 + static_cast<int>(bp % gg.gw)};
-        const int by{gg.by0 + static_cast<int>(bp / gg.gw)};
+        const int p{(sidx >= n ? 1 : 0) + (sidx >= 2 * n ? 1 : 0)};
+        const int c{phys_channel(p)};
+        int bx, by;
+        locate(sidx - p * n, bx, by);
+        bx += gg.bx0;
+        by += gg.by0;
         const std::int32_t* plane{e.dc + static_cast<std::size_t>(c) * e.nblocks};
         const std::size_t blk{static_cast<std::size_t>(by) * e.bw + bx};
         const bool hl{bx > gg.bx0};
@@ -151,9 +156,9 @@ __device__ void visit_misc(const EntropyDev& e, std::uint32_t item, V& v) {
         val = m < cwch ? e.ytox[tile] : e.ytob[tile];
     } else if (m < 2 * cwch + 2 * n) {
         const std::uint32_t r{m - 2 * cwch};
-        const std::uint32_t b{r % n};
-        const std::size_t blk{static_cast<std::size_t>(gg.by0 + static_cast<int>(b) / gg.gw) * e.bw +
-                              gg.bx0 + static_cast<int>(b) % gg.gw};
+        int bx, by;
+        locate(r < n ? r : r - n, bx, by);
+        const std::size_t blk{static_cast<std::size_t>(gg.by0 + by) * e.bw + gg.bx0 + bx};
         const int side{e.acs[blk]};
         if (side == 0) return;
         if (r < n) {
@@ -182,9 +187,12 @@ constexpr int kRowSlots = kAcGroupBlocks * kCoeffsPerBlock;      // 2048
 constexpr int kAcSymbols = 64;
 constexpr int kWindowWords = 4096;  // 16 KB of output bits assembled per CTA
 
-__device__ __forceinline__ unsigned long long prefix_at(const EntropyDev& e, std::uint32_t i) {
-    if (i >= e.total_items) return e.tile_off[e.num_tiles];
-    return e.tile_off[i / kScanTile] + e.item_pre[i];
+// Bits before section s (s == nsec: all of them).
+__device__ __forceinline__ unsigned long long section_start(const EntropyDev& e, int s) {
+    if (s >= e.nsec) return e.unit_off[e.misc_units + static_cast<std::uint32_t>(e.nstripes)];
+    const Section sec{e.sections[s]};
+    const unsigned long long off{e.unit_off[sec.unit]};
+    return sec.kind == kSecAcGroup ? off : off + e.item_pre[sec.first];
 }
 
 // ORs `n` (<= 32) bits of `v` at bit position `pos` of a zeroed word array in
@@ -392,9 +400,8 @@ __device__ __forceinline__ std::uint32_t pack_ac_token(int cl, std::uint32_t sym
                                                        std::uint32_t bits) {
     return (bits << 15) | (nb << 11) | (static_cast<std::uint32_t>(cl) << 6) | sym;
 }
-__device__ __forceinline__ std::uint32_t token_table_index(std::uint32_t t) {
-    return ((t >> 6) & 31u) * 256u + (t & 63u);
-}
+// Its entry in EntropyDev::code.
+__device__ __forceinline__ std::uint32_t token_code_index(std::uint32_t t) { return t & 2047u; }
 __device__ __forceinline__ std::uint32_t token_extra_count(std::uint32_t t) { return (t >> 11) & 15u; }
 __device__ __forceinline__ std::uint32_t token_extra_bits(std::uint32_t t) { return t >> 15; }
 
@@ -605,6 +612,7 @@ struct DirectStage {
     // DCT32 are adjacent, so an item's words are contiguous.
     std::uint32_t bitmap[3][kStripeRegions][32];
     std::uint16_t before[3][kStripeRegions][32];     // the item's non-zeros in its earlier words
+    alignas(16) std::uint8_t flag[kAcWarps][32 * 32];  // a warp's non-zeros of one region and plane, a byte each
     std::uint16_t count[kStripeItems];               // tokens of each item
     std::uint32_t info[kStripeItems];                // what a token needs to know of each item (pack_direct_item)
     std::uint32_t item_off[kStripeItems + 33];       // first token of each item that has any, then a sentinel
@@ -713,7 +721,6 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
         }
     }
     for (int i{tid}; i < kNumClusters * kAcSymbols; i += kAcThreads) s.hist[i] = 0;
-    for (int i{tid}; i < 3 * kStripeRegions * 32; i += kAcThreads) (&s.bitmap[0][0][0])[i] = 0;
     __syncthreads();
     if (side != 0) {
         const int lside{side >> 1};
@@ -725,53 +732,68 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
     cp_async_wait_all();
     __syncthreads();
 
-    if (loads) {
-        const int x{tid >> 3};
+    // A warp holds one region's four block rows (a lane an eighth of a block
+    // of each), so it makes that region's bitmaps by itself: plane by plane,
+    // each non-zero stores a byte at its scan position, and lane w gathers
+    // word w from 32 bytes. (ORing the bits in place with shared-memory atomics
+    // took up to 20K cycles for a dense stripe: low frequencies of one
+    // transform share a few words.) The tokens of each item follow: its count
+    // token, then every scan position through its last non-zero; sums over an
+    // item's words are segmented warp scans.
+    static_assert(kStripeRegions == kAcWarps && kAcGroupBlocks / kStripeRegions * (kCoeffsPerBlock / 8) == 32,
+                  "a warp per region");
+    uint4 ranks[kStripeRows];    // scan positions of the lane's eight coefficients of each row
+    std::uint32_t rowinfo[kStripeRows];  // 32 * first bitmap word
+#pragma unroll
+    for (int r{0}; r < kStripeRows; ++r) {
+        const unsigned own{loads && r < st.rows ? s.owner[r][tid >> 3] : kNoOwner};
+        const int lside{own != kNoOwner ? static_cast<int>(own >> 9) : 0};
+        const std::uint16_t* rank{s.rank + order_base(lside) + (own != kNoOwner ? (own >> 5) & 15u : 0u) * kCoeffsPerBlock +
+                                  (tid & 7) * 8};
+        ranks[r] = *reinterpret_cast<const uint4*>(rank);
+        rowinfo[r] = own != kNoOwner ? 32 * (own & 31u) : 0u;
+    }
+    std::uint8_t* flag{s.flag[warp]};
+#pragma unroll
+    for (int c{0}; c < 3; ++c) {
+        reinterpret_cast<uint4*>(flag)[lane] = make_uint4(0, 0, 0, 0);
+        reinterpret_cast<uint4*>(flag)[lane + 32] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
 #pragma unroll
         for (int r{0}; r < kStripeRows; ++r) {
-            if (r >= st.rows) continue;
-            const unsigned own{s.owner[r][x]};
-            if (own == kNoOwner) continue;
-            const int lside{static_cast<int>(own >> 9)};
-            const int covered{1 << (2 * lside)};
-            const std::uint16_t* rank{s.rank + order_base(lside) + ((own >> 5) & 15u) * kCoeffsPerBlock +
-                                      (tid & 7) * 8};
+            const std::uint32_t word[4]{v[c][r].x, v[c][r].y, v[c][r].z, v[c][r].w};
+            if ((word[0] | word[1] | word[2] | word[3]) == 0) continue;
+            const std::uint32_t pos[4]{ranks[r].x, ranks[r].y, ranks[r].z, ranks[r].w};
+            std::uint8_t* at{flag + rowinfo[r]};
 #pragma unroll
-            for (int c{0}; c < 3; ++c) {
-                const std::uint32_t word[4]{v[c][r].x, v[c][r].y, v[c][r].z, v[c][r].w};
-                if ((word[0] | word[1] | word[2] | word[3]) == 0) continue;
-                std::uint32_t* bits{&s.bitmap[c][x >> 2][own & 31u]};
-                // Bit i: coefficient i of the vector is not zero.
-                std::uint32_t set{0};
-#pragma unroll
-                for (int i{0}; i < 8; ++i) {
-                    set |= ((word[i >> 1] >> (16 * (i & 1))) & 0xffffu) != 0 ? 1u << i : 0u;
-                }
-                while (set != 0) {
-                    const int k{rank[__ffs(set) - 1]};
-                    set &= set - 1;
-                    // Positions below `covered` are the low frequencies, never coded here.
-                    if (k >= covered) atomicOr(&bits[k >> 5], 1u << (k & 31));
-                }
+            for (int i{0}; i < 8; ++i) {
+                const std::uint32_t k{(pos[i >> 1] >> (16 * (i & 1))) & 0xffffu};
+                // (The low frequencies, which are not coded here, are zero in
+                // the frontend's planes.)
+                if (((word[i >> 1] >> (16 * (i & 1))) & 0xffffu) != 0) at[k] = 1;
             }
         }
-    }
-    __syncthreads();
-
-    // Tokens of each item: its count token, then every scan position through
-    // its last non-zero. A warp per region and plane, a lane per bitmap word;
-    // sums over an item's words are segmented warp scans.
-    for (int u{warp}; u < 3 * kStripeRegions; u += kAcWarps) {
-        const int c{u / kStripeRegions};
-        const int region{u - c * kStripeRegions};
+        __syncwarp();
+        std::uint32_t m{0};
+#pragma unroll
+        for (int q{0}; q < 2; ++q) {
+            const uint4 b{reinterpret_cast<const uint4*>(flag)[2 * lane + q]};
+            // Four 0/1 bytes to four bits: byte i's product lands in bit 24 + i.
+            const std::uint32_t n[4]{b.x * 0x01020408u >> 24, b.y * 0x01020408u >> 24, b.z * 0x01020408u >> 24,
+                                     b.w * 0x01020408u >> 24};
+#pragma unroll
+            for (int i{0}; i < 4; ++i) m |= n[i] << (16 * q + 4 * i);
+        }
+        __syncwarp();
+        const int region{warp};
         const int z{lane >> 1};
         const int r{((z >> 1) & 1) | ((z >> 2) & 2)};
         const int x{4 * region + ((z & 1) | ((z >> 1) & 2))};
         const unsigned own{r < st.rows && x < gg.gw ? s.owner[r][x] : kNoOwner};
+        s.bitmap[c][region][lane] = m;
         const int lside{own != kNoOwner ? static_cast<int>(own >> 9) : 0};
         const int words{2 << (2 * lside)};
         const int seg{lane & ~(words - 1)};
-        const std::uint32_t m{s.bitmap[c][region][lane]};
         const std::uint32_t pc{static_cast<std::uint32_t>(__popc(m))};
         std::uint32_t sum{pc};
 #pragma unroll
@@ -858,6 +880,7 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
 #pragma unroll
         for (int g{0}; g < kAhead; ++g) {
             const std::uint32_t tg{t0 + 32 * g};
+            if (tg >= t_end) break;
             const std::uint32_t rel{s.item_off[min(base + 1 + lane, nactive)] - tg};
             const unsigned starts{__reduce_or_sync(kFull, rel < 32 ? 1u << rel : 0u)};
             const int item{min(base + __popc(starts & ((2u << lane) - 1u)), nactive - 1)};
@@ -895,7 +918,7 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
 #pragma unroll
         for (int g{0}; g < kAhead; ++g) {
             const std::uint32_t t{t0 + 32 * g + lane};
-            if (t >= t_end) continue;
+            if (t0 + 32 * g >= t_end) break;
             const int lside{static_cast<int>((info[g] >> 11) & 3u)};
             const int c{static_cast<int>((info[g] >> 20) & 3u)};
             std::uint32_t value;
@@ -923,8 +946,16 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
             }
             std::uint32_t tok, nb, bits;
             hybrid_uint(value, tok, nb, bits);
-            atomicAdd(&s.hist[cl * kAcSymbols + tok], 1u);
-            (t < own ? near : far)[t] = pack_ac_token(cl, tok, nb, bits);
+            // Lanes of equal tokens count once: shared-memory atomics on one
+            // address serialise.
+            const unsigned key{t < t_end ? static_cast<unsigned>(cl * kAcSymbols) + tok : 0xffffffffu};
+            const unsigned peers{__match_any_sync(kFull, key)};
+            if (t < t_end) {
+                if (__ffs(static_cast<int>(peers)) - 1 == lane) {
+                    atomicAdd(&s.hist[key], static_cast<unsigned>(__popc(peers)));
+                }
+                (t < own ? near : far)[t] = pack_ac_token(cl, tok, nb, bits);
+            }
         }
     }
     __syncthreads();
@@ -933,15 +964,40 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
     }
 }
 
+// The token of an item other than an AC block-channel, kept from the token
+// pass for the later passes: symbol (7 bits; hybrid-uint (4, 2, 0) symbols of
+// 32-bit values are below 128), extra-bit count (5), extra bits (18), table.
+// kMiscVisit: blobs, counts and wider tokens, which the later passes visit
+// again; kMiscNone: nothing is written for the item.
+constexpr std::uint32_t kMiscVisit = 0x80000000u;
+constexpr std::uint32_t kMiscNone = 0x80000001u;
+constexpr std::uint32_t kMiscExtraBits = 18;
+constexpr int kMiscSymbols = 128;
+__device__ __forceinline__ std::uint32_t pack_misc_token(int tab, std::uint32_t sym, std::uint32_t nb, std::uint32_t bits) {
+    if (nb > kMiscExtraBits) return kMiscVisit;
+    return (tab == kTabAm ? 0x40000000u : 0u) | (bits << 12) | (nb << 7) | sym;
+}
+// Entry of EntropyDev::code where a DC group's DC or AcMetadata symbols start.
+__device__ __forceinline__ int misc_code_base(const EntropyDev& e, bool am, int g) {
+    return kNumClusters * kAcSymbols + ((am ? e.ndc : 0) + g) * kMiscSymbols;
+}
+// Its depth << 16 | code bits, in DC group g.
+__device__ __forceinline__ std::uint32_t misc_code(const EntropyDev& e, int g, std::uint32_t t) {
+    return __ldg(&e.code[misc_code_base(e, (t & 0x40000000u) != 0, g) + (t & 127u)]);
+}
+__device__ __forceinline__ std::uint32_t misc_extra_count(std::uint32_t t) { return (t >> 7) & 31u; }
+__device__ __forceinline__ std::uint32_t misc_extra_bits(std::uint32_t t) { return (t >> 12) & 0x3ffffu; }
+
 struct HistVisitor {
     std::uint32_t* sh_g;      // [2 slots][2 tables][256]
     std::uint32_t* sh_fb;     // [2 slots]
     int g0, g1;
     const EntropyDev* e;
-    __device__ void blob(const std::uint8_t*, std::uint32_t) {}
-    __device__ void varlen(std::uint32_t) {}
-    __device__ void count_field(int, unsigned) {}
-    __device__ void epf(int) {}
+    std::uint32_t kept{kMiscNone};  // what item_tok gets
+    __device__ void blob(const std::uint8_t*, std::uint32_t) { kept = kMiscVisit; }
+    __device__ void varlen(std::uint32_t) { kept = kMiscVisit; }
+    __device__ void count_field(int, unsigned) { kept = kMiscVisit; }
+    __device__ void epf(int) { kept = pack_misc_token(kTabAm, 0, 0, 0); }  // counted by the code pass
     __device__ void first_block(int g) {
         if (g == g0) {
             atomicAdd(&sh_fb[0], 1u);
@@ -951,7 +1007,8 @@ struct HistVisitor {
             atomicAdd(&e->fb_count[g], 1u);
         }
     }
-    __device__ void token(int tab, int g, std::uint32_t sym, std::uint32_t, std::uint32_t) {
+    __device__ void token(int tab, int g, std::uint32_t sym, std::uint32_t nb, std::uint32_t bits) {
+        kept = pack_misc_token(tab, sym, nb, bits);
         const int t{tab == kTabDc ? 0 : 1};
         if (g == g0) {
             atomicAdd(&sh_g[t * 256 + sym], 1u);
@@ -963,27 +1020,35 @@ struct HistVisitor {
     }
 };
 
-// Other items per CTA of the item passes (256 threads, two items each).
-constexpr std::uint32_t kMiscItemsPerBlock = 512;
+// Other items per thread of the item passes.
 constexpr int kMiscPerThread = 2;
+static_assert(kMiscItemsPerUnit == kMiscPerThread * kAcThreads, "a unit of other items is one CTA's");
 
-__device__ __forceinline__ void misc_hist_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+__device__ __forceinline__ void misc_hist_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char misc_smem[];
     std::uint32_t* sh_g{reinterpret_cast<std::uint32_t*>(misc_smem)};  // [4 * 256]
     std::uint32_t* sh_fb{sh_g + 4 * 256};                              // [2]
     if (threadIdx.x < 2) sh_fb[threadIdx.x] = 0;
     for (int i{static_cast<int>(threadIdx.x)}; i < 4 * 256; i += blockDim.x) sh_g[i] = 0;
-    const std::uint32_t first{blk * kMiscItemsPerBlock};
-    const std::uint32_t last{min(first + kMiscItemsPerBlock, e.ac_first) - 1};
-    const Section s0{e.sections[find_section(e.sections, 0, misc_hi(e), first)]};
-    const Section s1{e.sections[find_section(e.sections, 0, misc_hi(e), last)]};
+    const std::uint32_t first{blk * kMiscItemsPerUnit};
+    const std::uint32_t last{min(first + kMiscItemsPerUnit, e.ac_first) - 1};
+    const int sfirst{static_cast<int>(e.unit_section[blk])};
+    const Section s0{e.sections[sfirst]};
+    int slast{sfirst};
+    const Section s1{section_from(e, slast, last)};
     HistVisitor v{sh_g, sh_fb, s0.kind == kSecDcGroup ? s0.group : -1,
                   s1.kind == kSecDcGroup && s1.group != s0.group ? s1.group : -2, &e};
     __syncthreads();
 #pragma unroll
     for (int k{0}; k < kMiscPerThread; ++k) {
         const std::uint32_t item{first + threadIdx.x + k * blockDim.x};
-        if (item < e.ac_first) visit_misc(e, item, v);
+        if (item < e.ac_first) {
+            int sat{sfirst};
+            const Section sec{section_from(e, sat, item)};
+            v.kept = kMiscNone;
+            visit_misc(e, sec, item - sec.first, v);
+            e.item_tok[item] = v.kept;
+        }
     }
     __syncthreads();
     for (int i{static_cast<int>(threadIdx.x)}; i < 4 * 256; i += blockDim.x) {
@@ -1298,12 +1363,12 @@ __device__ void warp_build_and_store(WarpCodeSmem& s, int length, BitSink& w, in
 // One single-warp CTA per histogram (the 32 AC clusters, then the DC and the
 // AcMetadata histogram of every DC group): the construction is a long serial
 // chain on lane 0, so each chain gets an SM to itself.
-__device__ __forceinline__ void codes_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+__device__ __forceinline__ void codes_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char code_smem[];
     const int lane{static_cast<int>(threadIdx.x) & 31};
     WarpCodeSmem& s{*reinterpret_cast<WarpCodeSmem*>(code_smem)};
     int idx;
-    const std::uint32_t* src;
+    std::uint32_t* src;
     std::uint8_t* dst_depth;
     std::uint16_t* dst_bits;
     bool clustered;
@@ -1336,6 +1401,19 @@ __device__ __forceinline__ void codes_body(const EntropyDev& e, const unsigned b
     std::uint32_t hv[8];
 #pragma unroll
     for (int k{0}; k < 8; ++k) hv[k] = src[lane + 32 * k];  // all eight loads in flight at once
+    // Leave the histograms and counters zeroed for the next frame; the passes
+    // after this one read the counters' frozen copies.
+#pragma unroll
+    for (int k{0}; k < 8; ++k) src[lane + 32 * k] = 0;
+    if (lane == 0 && blk == 0) {
+        e.frozen[0] = *e.tok_count;
+        *e.tok_count = 0;
+    }
+    if (lane == 0 && idx >= 32 + e.ndc) {
+        const int g{idx - 32 - e.ndc};
+        e.frozen[1 + g] = e.fb_count[g];
+        e.fb_count[g] = 0;
+    }
 #pragma unroll
     for (int k{0}; k < 8; ++k) {
         const int i{lane + 32 * k};
@@ -1371,6 +1449,10 @@ __device__ __forceinline__ void codes_body(const EntropyDev& e, const unsigned b
         dst_depth[i] = s.depth[i];
         dst_bits[i] = s.bits[i];
     }
+    std::uint32_t* code{e.code + (clustered ? idx * kAcSymbols : kNumClusters * kAcSymbols + (idx - 32) * kMiscSymbols)};
+    for (int i{lane}; i < (clustered ? kAcSymbols : kMiscSymbols); i += 32) {
+        code[i] = (static_cast<std::uint32_t>(s.depth[i]) << 16) | s.bits[i];
+    }
 }
 
 // One histogram through the device builder (test hook): `length` symbols,
@@ -1399,42 +1481,42 @@ __global__ void __launch_bounds__(32) prefix_code_test_kernel(const std::uint32_
     if (lane == 0) *nbits = w.overflow ? 0xffffffffu : w.pos;
 }
 
-// ---- pass 3: bit lengths and scan ----------------------------------------------------
+// ---- pass 3: bit lengths, scan and layout ----------------------------------------------------
 
-// Which stripes a launch of the AC bit-length or emission pass takes: those
-// whose tokens are stored (no staging, small shared memory) or the others
-// (staged coefficients, tokenised again).
-enum StripeSet : int { kStoredStripes = 0, kUnstoredStripes = 1 };
+// Bits of a stripe whose tokens are stored: the sum over its tokens. (Only
+// the start of a stripe is ever looked up, so its items get no prefixes.)
+__device__ __forceinline__ void ac_bits_stored_body(const EntropyDev& e, const unsigned blk) {
+    __shared__ std::uint32_t sh_sum[kAcWarps];
+    const int tid{static_cast<int>(threadIdx.x)};
+    const Stripe st{e.stripes[blk]};
+    const StripeTokens pool{stripe_tokens(e, st, blk, st.rows * st.cols)};
+    if (pool.near == nullptr) return;  // summed by the pass over unstored stripes
+    const std::uint32_t ntok{e.stripe_tok[2 * blk + 1]};
+    std::uint32_t sum{0};
+#pragma unroll 4
+    for (std::uint32_t t{static_cast<std::uint32_t>(tid)}; t < ntok; t += kAcThreads) {
+        const std::uint32_t tk{*pool.at(t)};
+        sum += (__ldg(&e.code[token_code_index(tk)]) >> 16) + token_extra_count(tk);
+    }
+    sum = warp_sum(sum);
+    if ((tid & 31) == 0) sh_sum[tid >> 5] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        std::uint32_t total{0};
+        for (int w{0}; w < kAcWarps; ++w) total += sh_sum[w];
+        e.unit_sum[e.misc_units + blk] = total;
+    }
+}
 
-template <int kSet>
-__device__ __forceinline__ void ac_bits_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+// Bits of a stripe whose tokens are not stored, and each item's prefix.
+__device__ __forceinline__ void ac_bits_unstored_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char ac_smem[];
     StripeStage& s{*reinterpret_cast<StripeStage*>(ac_smem)};
-    __shared__ std::uint32_t sh_sum[kAcWarps];
+    __shared__ std::uint32_t sh_scan[kAcWarps + 1];
     const int tid{static_cast<int>(threadIdx.x)};
     const int lane{tid & 31};
     const Stripe st{e.stripes[blk]};
     const GroupGeom gg{ac_group_geom(e, st.group)};
-    const StripeTokens pool{stripe_tokens(e, st, blk, st.rows * gg.gw)};
-    if ((pool.near != nullptr) != (kSet == kStoredStripes)) return;
-    if (pool.near != nullptr) {
-        // Stored tokens: the stripe's whole length goes on its first item
-        // (the scan only needs sums at stripe and section starts).
-        const std::uint32_t ntok{e.stripe_tok[2 * blk + 1]};
-        std::uint32_t sum{0};
-        for (std::uint32_t t{static_cast<std::uint32_t>(tid)}; t < ntok; t += kAcThreads) {
-            const std::uint32_t tk{*pool.at(t)};
-            sum += __ldg(&e.ac_depth[token_table_index(tk)]) + token_extra_count(tk);
-        }
-        sum = warp_sum(sum);
-        if (lane == 0) sh_sum[tid >> 5] = sum;
-        __syncthreads();
-        const int nitems{3 * st.rows * gg.gw};
-        std::uint32_t total{0};
-        for (int w{0}; w < kAcWarps; ++w) total += sh_sum[w];
-        for (int j{tid}; j < nitems; j += kAcThreads) e.item_bits[st.item0 + j] = j == 0 ? total : 0u;
-        return;
-    }
     stage_stripe(e, st, gg, s);
     __syncthreads();
     const int nitems{3 * st.rows * gg.gw};
@@ -1462,7 +1544,14 @@ __device__ __forceinline__ void ac_bits_body(const EntropyDev& e, const unsigned
         if (lane == 0) s.aux[j] += total;
     }
     __syncthreads();
-    for (int j{tid}; j < nitems; j += kAcThreads) e.item_bits[st.item0 + j] = s.aux[j];
+    const int j0{2 * tid};
+    const std::uint32_t b0{j0 < nitems ? s.aux[j0] : 0u};
+    const std::uint32_t b1{j0 + 1 < nitems ? s.aux[j0 + 1] : 0u};
+    std::uint32_t total{0};
+    const std::uint32_t off{cta_exclusive_scan(b0 + b1, sh_scan, total)};
+    if (j0 < nitems) e.item_pre[st.item0 + j0] = off;
+    if (j0 + 1 < nitems) e.item_pre[st.item0 + j0 + 1] = off + b0;
+    if (tid == 0) e.unit_sum[e.misc_units + blk] = total;
 }
 
 struct BitsVisitor {
@@ -1486,130 +1575,36 @@ struct BitsVisitor {
     }
 };
 
-__device__ __forceinline__ void misc_bits_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+// Bits of a unit of other items, and each item's prefix in it; thread t takes
+// items 2t and 2t + 1.
+__device__ __forceinline__ void misc_bits_body(const EntropyDev& e, const unsigned blk) {
+    __shared__ std::uint32_t sh_scan[kAcWarps + 1];
+    const std::uint32_t item0{blk * kMiscItemsPerUnit + kMiscPerThread * threadIdx.x};
+    std::uint32_t bits[kMiscPerThread]{};
+    std::uint32_t tok[kMiscPerThread];
+#pragma unroll
+    for (int k{0}; k < kMiscPerThread; ++k) tok[k] = item0 + k < e.ac_first ? e.item_tok[item0 + k] : kMiscNone;
+    int sat{static_cast<int>(e.unit_section[blk])};
 #pragma unroll
     for (int k{0}; k < kMiscPerThread; ++k) {
-        const std::uint32_t item{blk * kMiscItemsPerBlock + threadIdx.x + k * blockDim.x};
-        if (item >= e.ac_first) return;
-        BitsVisitor v{&e, 0};
-        visit_misc(e, item, v);
-        e.item_bits[item] = v.total;
+        if (tok[k] == kMiscNone) continue;
+        const Section sec{section_from(e, sat, item0 + k)};
+        if (tok[k] == kMiscVisit) {
+            BitsVisitor v{&e, 0};
+            visit_misc(e, sec, item0 + k - sec.first, v);
+            bits[k] = v.total;
+        } else {
+            bits[k] = (misc_code(e, sec.group, tok[k]) >> 16) + misc_extra_count(tok[k]);
+        }
     }
+    std::uint32_t total{0};
+    const std::uint32_t off{cta_exclusive_scan(bits[0] + bits[1], sh_scan, total)};
+    if (item0 < e.ac_first) e.item_pre[item0] = off;
+    if (item0 + 1 < e.ac_first) e.item_pre[item0 + 1] = off + bits[0];
+    if (threadIdx.x == 0) e.unit_sum[blk] = total;
 }
 
-// Exclusive scan of item_bits inside tiles of kScanTile items (1024 threads x 4).
-__device__ __forceinline__ void scan_tile_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    __shared__ std::uint32_t warp_sums[32];
-    const std::uint32_t base{blk * kScanTile + threadIdx.x * 4};
-    std::uint32_t v[4];
-    std::uint32_t local{0};
-#pragma unroll
-    for (int k{0}; k < 4; ++k) {
-        v[k] = base + k < e.total_items ? e.item_bits[base + k] : 0u;
-        local += v[k];
-    }
-    const int lane{static_cast<int>(threadIdx.x) & 31};
-    const int warp{static_cast<int>(threadIdx.x) >> 5};
-    std::uint32_t incl{local};
-#pragma unroll
-    for (int off{1}; off < 32; off <<= 1) {
-        const std::uint32_t t{__shfl_up_sync(kFull, incl, off)};
-        if (lane >= off) incl += t;
-    }
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const std::uint32_t ws{warp_sums[lane]};
-        std::uint32_t wi{ws};
-#pragma unroll
-        for (int off{1}; off < 32; off <<= 1) {
-            const std::uint32_t t{__shfl_up_sync(kFull, wi, off)};
-            if (lane >= off) wi += t;
-        }
-        warp_sums[lane] = wi - ws;
-        if (lane == 31) e.tile_sum[blk] = wi;
-    }
-    __syncthreads();
-    std::uint32_t run{warp_sums[warp] + incl - local};
-#pragma unroll
-    for (int k{0}; k < 4; ++k) {
-        if (base + k < e.total_items) e.item_pre[base + k] = run;
-        run += v[k];
-    }
-}
-
-__device__ __forceinline__ void scan_top_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    __shared__ unsigned long long warp_sums[32];
-    __shared__ unsigned long long carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane{static_cast<int>(threadIdx.x) & 31};
-    const int warp{static_cast<int>(threadIdx.x) >> 5};
-    for (std::uint32_t base{0}; base < e.num_tiles; base += 1024) {
-        const std::uint32_t i{base + threadIdx.x};
-        const unsigned long long x{i < e.num_tiles ? e.tile_sum[i] : 0ull};
-        unsigned long long incl{x};
-#pragma unroll
-        for (int off{1}; off < 32; off <<= 1) {
-            const unsigned long long t{__shfl_up_sync(kFull, incl, off)};
-            if (lane >= off) incl += t;
-        }
-        if (lane == 31) warp_sums[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const unsigned long long ws{warp_sums[lane]};
-            unsigned long long wi{ws};
-#pragma unroll
-            for (int off{1}; off < 32; off <<= 1) {
-                const unsigned long long t{__shfl_up_sync(kFull, wi, off)};
-                if (lane >= off) wi += t;
-            }
-            warp_sums[lane] = wi - ws;
-        }
-        __syncthreads();
-        if (i < e.num_tiles) e.tile_off[i] = carry + warp_sums[warp] + incl - x;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += warp_sums[31] + incl;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) e.tile_off[e.num_tiles] = carry;
-}
-
-
-// ---- pass 4: layout --------------------------------------------------------------
-
-struct U32Dist {
-    bool direct;
-    std::uint32_t v;
-    std::uint32_t extra;
-};
-
-__device__ void put_u32(BitSink& w, const U32Dist* d, std::uint32_t value) {
-    std::uint32_t best{0};
-    std::uint32_t best_bits{64};
-    for (std::uint32_t s{0}; s < 4; ++s) {
-        if (d[s].direct) {
-            if (d[s].v == value) {
-                best = s;
-                best_bits = 2;
-                break;
-            }
-            continue;
-        }
-        if (value < d[s].v || static_cast<unsigned long long>(value) >=
-                                  static_cast<unsigned long long>(d[s].v) + (1ull << d[s].extra)) {
-            continue;
-        }
-        if (2 + d[s].extra < best_bits) {
-            best = s;
-            best_bits = 2 + d[s].extra;
-        }
-    }
-    w.put(2, best);
-    if (!d[best].direct) w.put(d[best].extra, value - d[best].v);
-}
-
-constexpr int kLayoutThreads = 256;
+// ---- pass 4: layout ---------------------------------------------------------------
 
 // TOC entry of a section of `bytes` bytes: U32 with selectors 0 + 10 bits,
 // 1024 + 14, 17408 + 22, 4211712 + 30 (src/bitstream/codestream.cc:16-18, 91-98);
@@ -1631,8 +1626,11 @@ __device__ __forceinline__ void toc_entry(std::uint32_t bytes, std::uint32_t& nb
     field = sel | ((bytes - base) << 2);
 }
 
-// Block-wide exclusive scan of one 64-bit value per thread; returns the
-// thread's offset and sets `total`.
+constexpr int kLayoutThreads = 1024;
+constexpr int kLayoutWarps = kLayoutThreads / 32;
+
+// Block-wide exclusive scan of one 64-bit value per thread of the layout CTA;
+// returns the thread's offset and sets `total`.
 __device__ unsigned long long block_scan(unsigned long long v, unsigned long long* warp_sums,
                                          unsigned long long& total) {
     const int lane{static_cast<int>(threadIdx.x) & 31};
@@ -1645,189 +1643,207 @@ __device__ unsigned long long block_scan(unsigned long long v, unsigned long lon
     }
     if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
-    if (warp == 0) {
-        const int nw{static_cast<int>(blockDim.x) >> 5};
-        const unsigned long long ws{lane < nw ? warp_sums[lane] : 0ull};
-        unsigned long long wi{ws};
+    // Every warp scans the warps' sums itself.
+    const unsigned long long x{warp_sums[lane]};
+    unsigned long long sums{x};
 #pragma unroll
-        for (int off{1}; off < 32; off <<= 1) {
-            const unsigned long long t{__shfl_up_sync(kFull, wi, off)};
-            if (lane >= off) wi += t;
-        }
-        if (lane < nw) warp_sums[lane] = wi - ws;
-        if (lane == nw - 1) warp_sums[32] = wi;
+    for (int off{1}; off < 32; off <<= 1) {
+        const unsigned long long t{__shfl_up_sync(kFull, sums, off)};
+        if (lane >= off) sums += t;
     }
+    const unsigned long long before{__shfl_sync(kFull, sums - x, warp)};
+    total = __shfl_sync(kFull, sums, 31);
     __syncthreads();
-    const unsigned long long off{warp_sums[warp] + incl - v};
-    total = warp_sums[32];
-    __syncthreads();
-    return off;
+    return before + incl - v;
 }
 
-// Sizes the sections, then writes the codestream headers and frame header
-// (one thread), the TOC (every thread its own entries, placed by a scan of
-// their bit lengths), the container framing and the section positions
-// (src/bitstream/codestream.cc:57-135, src/bitstream/container.cc:35-62).
-// Dynamic shared memory: the section sizes, then the header words
-// (layout_head_bytes).
-__device__ __forceinline__ void layout_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    extern __shared__ __align__(16) unsigned char layout_smem[];
-    __shared__ unsigned long long scan_sums[33];
-    __shared__ unsigned long long sh_start, sh_status, sh_head;
-    __shared__ std::uint32_t sh_toc_start;
-    auto* sec_bytes{reinterpret_cast<std::uint32_t*>(layout_smem)};
-    const std::uint32_t head_cap{layout_head_bytes(e.nsec)};
-    std::uint8_t* head{layout_smem + layout_sizes_bytes(e.nsec)};
-    auto* head_words{reinterpret_cast<unsigned int*>(head)};
+// Zeroes word w of the output, or those of its bytes that lie in the file.
+__device__ __forceinline__ void zero_out_word(const EntropyDev& e, unsigned long long w, unsigned long long file_bytes) {
+    if (4 * w + 4 <= file_bytes) {
+        reinterpret_cast<std::uint32_t*>(e.out)[w] = 0;
+    } else {
+        for (unsigned long long b{4 * w}; b < file_bytes; ++b) e.out[b] = 0;
+    }
+}
+
+// Scans the units, sizes the sections, places sections and units, and writes
+// the container framing, the codestream headers and the TOC
+// (src/bitstream/codestream.cc:57-135, src/bitstream/container.cc:35-62). The
+// emission ORs its bits into the words that units or sections share, so those
+// are zeroed here; a unit stores the words it has to itself.
+//
+// One CTA per frame. Its time is that of its chains of dependent loads, so
+// sections and units are looked up two levels deep and loads go ahead of
+// stores.
+__device__ __forceinline__ void layout_body(const EntropyDev& e) {
+    __shared__ unsigned long long scan_sums[kLayoutWarps];
     const int tid{static_cast<int>(threadIdx.x)};
-    for (std::uint32_t i{static_cast<std::uint32_t>(tid)}; i < head_cap / 4; i += kLayoutThreads) head_words[i] = 0;
-    // With one AC group the four sections are one combined TOC entry: their
-    // bits follow each other with no padding between them
-    // (tools/bitstream/vardct_frame.cc:414-449).
+    const std::uint32_t units{e.misc_units + static_cast<std::uint32_t>(e.nstripes)};
+    // This thread's sections (a contiguous run of TOC entries): what their
+    // starts depend on, loaded while the units are scanned. With one AC group
+    // the four sections are one combined TOC entry: their bits follow each
+    // other with no padding between them (tools/bitstream/vardct_frame.cc:414-449).
     const bool single{e.nac == 1};
     const int ntoc{single ? 1 : e.nsec};
-    if (single) {
-        if (tid == 0) {
-            const unsigned long long bits{prefix_at(e, e.total_items) - prefix_at(e, 0)};
-            sec_bytes[0] = static_cast<std::uint32_t>((bits + 7) / 8);
-        }
-    } else {
-        for (int s{tid}; s < e.nsec; s += kLayoutThreads) {
-            const Section sec{e.sections[s]};
-            const unsigned long long bits{prefix_at(e, sec.first + sec.count) - prefix_at(e, sec.first)};
-            sec_bytes[s] = static_cast<std::uint32_t>((bits + 7) / 8);
-        }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        BitSink w{head, 0, head_cap * 8, false};
-        const U32Dist dim[4]{{false, 1, 9}, {false, 1, 13}, {false, 1, 18}, {false, 1, 30}};
-        w.put(8, 0xFF);
-        w.put(8, 0x0A);
-        const std::uint32_t W{static_cast<std::uint32_t>(e.width)};
-        const std::uint32_t H{static_cast<std::uint32_t>(e.height)};
-        const bool small{W % 8 == 0 && H % 8 == 0 && W <= 256 && H <= 256};
-        w.put(1, small ? 1 : 0);
-        if (small) w.put(5, H / 8 - 1); else put_u32(w, dim, H);
-        w.put(3, 0);
-        if (small) w.put(5, W / 8 - 1); else put_u32(w, dim, W);
-        w.put(1, 1);  // ImageMetadata all_default
-        w.put(1, 1);  // transform data all_default
-        w.pos = (w.pos + 7) & ~7u;
-        // FrameHeader: regular VarDCT frame, upsampling 1, x/b qm scale 2, one
-        // pass, no custom size, replace blending, last, unnamed, default loop filter.
-        w.put(1, 0);
-        w.put(2, 0);
-        w.put(1, 0);
-        w.put(2, 0);
-        w.put(2, 0);
-        w.put(3, 2);
-        w.put(3, 2);
-        w.put(2, 0);
-        w.put(1, 0);
-        w.put(2, 0);
-        w.put(1, 1);
-        w.put(2, 0);
-        w.put(1, 1);
-        w.put(2, 0);
-        w.put(1, 0);  // TOC without permutation
-        w.pos = (w.pos + 7) & ~7u;
-        sh_toc_start = w.pos;
-    }
-    __syncthreads();
-    // Each thread takes a contiguous run of TOC entries.
     const int per{(ntoc + kLayoutThreads - 1) / kLayoutThreads};
     const int lo{min(ntoc, tid * per)};
     const int hi{min(ntoc, lo + per)};
+    // Unit offsets, four units per thread and round (unit_sum and unit_off
+    // have room for whole vectors of four).
+    unsigned long long carry{0};
+    for (std::uint32_t u0{0}; u0 < units; u0 += kLayoutThreads * 4) {
+        const std::uint32_t at{u0 + static_cast<std::uint32_t>(tid) * 4};
+        uint4 x{at < units ? *reinterpret_cast<const uint4*>(e.unit_sum + at) : make_uint4(0, 0, 0, 0)};
+        if (at + 1 >= units) x.y = 0;
+        if (at + 2 >= units) x.z = 0;
+        if (at + 3 >= units) x.w = 0;
+        unsigned long long total{0};
+        const unsigned long long off{
+            carry + block_scan(static_cast<unsigned long long>(x.x) + x.y + x.z + x.w, scan_sums, total)};
+        if (at < units) {
+            auto* dst{reinterpret_cast<ulonglong2*>(e.unit_off + at)};
+            dst[0] = make_ulonglong2(off, off + x.x);
+            dst[1] = make_ulonglong2(off + x.x + x.y, off + x.x + x.y + x.z);
+        }
+        carry += total;
+    }
+    __syncthreads();
+    if (tid == 0) e.unit_off[units] = carry;
+    __syncthreads();
+
+    std::uint32_t nb{0};  // of the last entry: of the only one in all but the largest frames
+    std::uint32_t field{0};
     unsigned long long my_bits{0};
     unsigned long long my_bytes{0};
+    unsigned long long start{lo < hi ? section_start(e, lo) : 0ull};
     for (int s{lo}; s < hi; ++s) {
-        std::uint32_t nb, field;
-        toc_entry(sec_bytes[s], nb, field);
+        const unsigned long long next{section_start(e, single ? e.nsec : s + 1)};
+        const std::uint32_t bytes{static_cast<std::uint32_t>((next - start + 7) / 8)};
+        start = next;
+        toc_entry(bytes, nb, field);
         my_bits += nb;
-        my_bytes += sec_bytes[s];
+        my_bytes += bytes;
+        e.sec_shift[s] = bytes;
     }
     unsigned long long toc_bits{0};
     unsigned long long body{0};
-    const unsigned long long bit_off{block_scan(my_bits, scan_sums, toc_bits)};
+    const unsigned long long toc_off{block_scan(my_bits, scan_sums, toc_bits)};
     const unsigned long long byte_off{block_scan(my_bytes, scan_sums, body)};
-    {
-        unsigned long long p{sh_toc_start + bit_off};
-        for (int s{lo}; s < hi; ++s) {
-            std::uint32_t nb, field;
-            toc_entry(sec_bytes[s], nb, field);
-            const std::uint32_t off{static_cast<std::uint32_t>(p & 31)};
-            atomicOr(&head_words[p >> 5], field << off);
-            if (off + nb > 32) atomicOr(&head_words[(p >> 5) + 1], field >> (32 - off));
-            p += nb;
-        }
-    }
-    __syncthreads();
+    const unsigned long long head{e.head_bytes + (toc_bits + 7) / 8};
+    const unsigned long long cs{head + body};
+    const bool large{cs >= 0x100000000ull - 8};
+    const unsigned long long framing{32ull + (large ? 16 : 8)};
+    const unsigned long long file{framing + cs};
+    // 2: the file would reach the tokens kept at the buffer's end (never:
+    // dense_tokens).
+    const unsigned long long dense{e.direct ? 4ull * e.frozen[0] : 0ull};
+    const unsigned long long status{
+        file > e.out_capacity ? 1ull : (dense != 0 && file + dense > e.out_capacity ? 2ull : 0ull)};
     if (tid == 0) {
-        const unsigned long long head_bytes{(sh_toc_start + toc_bits + 7) / 8};
-        const unsigned long long cs{head_bytes + body};
-        const bool large{cs >= 0x100000000ull - 8};
-        const unsigned long long framing{32ull + (large ? 16 : 8)};
-        const unsigned long long total{framing + cs};
-        sh_head = head_bytes;
-        sh_start = framing + head_bytes;
-        // 2: the file would reach the tokens kept at the buffer's end (never:
-        // dense_tokens).
-        const unsigned long long dense{e.direct ? 4ull * *e.tok_count : 0ull};
-        sh_status = total > e.out_capacity ? 1ull : (dense != 0 && total + dense > e.out_capacity ? 2ull : 0ull);
-        e.result[0] = total;
-        e.result[1] = sh_start;
-        e.result[2] = sh_status;
-        if (sh_status == 0) {
-            const std::uint8_t hdr[32]{0, 0, 0, 0x0c, 'J', 'X', 'L', ' ', 0x0d, 0x0a, 0x87, 0x0a, 0, 0, 0, 0x14,
-                                       'f', 't', 'y', 'p', 'j', 'x', 'l', ' ', 0, 0, 0, 0, 'j', 'x', 'l', ' '};
-            for (int i{0}; i < 32; ++i) e.out[i] = hdr[i];
-            std::size_t at{32};
-            const unsigned long long box{cs + (large ? 16 : 8)};
-            const std::uint32_t sf{large ? 1u : static_cast<std::uint32_t>(box)};
-            for (int i{0}; i < 4; ++i) e.out[at++] = static_cast<std::uint8_t>(sf >> (8 * (3 - i)));
-            e.out[at++] = 'j';
-            e.out[at++] = 'x';
-            e.out[at++] = 'l';
-            e.out[at++] = 'c';
-            if (large) {
-                for (int i{0}; i < 8; ++i) e.out[at++] = static_cast<std::uint8_t>(box >> (8 * (7 - i)));
-            }
+        e.result[0] = file;
+        e.result[1] = framing + head;
+        e.result[2] = status;
+    }
+    if (status != 0) return;
+
+    // Each section's shift from its bits' place in the scan to their place in
+    // the file (sections are padded to whole bytes, but not the combined ones).
+    if (single) {
+        for (int s{tid}; s < e.nsec; s += kLayoutThreads) e.sec_shift[s] = 8 * (framing + head);
+    } else {
+        unsigned long long pos{framing + head + byte_off};
+        start = lo < hi ? section_start(e, lo) : 0ull;
+        for (int s{lo}; s < hi; ++s) {
+            const unsigned long long bytes{e.sec_shift[s]};
+            e.sec_shift[s] = 8 * pos - start;
+            pos += bytes;
+            if (s + 1 < hi) start = section_start(e, s + 1);
         }
     }
     __syncthreads();
-    if (sh_status != 0) return;
-    if (single) {
-        const unsigned long long base{prefix_at(e, 0)};
-        for (int s{tid}; s < e.nsec; s += kLayoutThreads) {
-            e.sec_pos[s] = sh_start * 8 + (prefix_at(e, e.sections[s].first) - base);
+    // Unit positions; the words that hold a unit's first or last bit. Four
+    // units' loads at a time, ahead of their stores.
+    for (std::uint32_t u0{static_cast<std::uint32_t>(tid)}; u0 < units; u0 += 4 * kLayoutThreads) {
+        unsigned long long pos[4];
+        std::uint32_t bits[4];
+        std::uint32_t sec[4];
+#pragma unroll
+        for (int k{0}; k < 4; ++k) {
+            const std::uint32_t u{min(u0 + k * kLayoutThreads, units - 1)};
+            sec[k] = e.unit_section[u];
+            pos[k] = e.unit_off[u];
+            bits[k] = e.unit_sum[u];
         }
-    } else {
-        unsigned long long pos{sh_start + byte_off};
-        for (int s{lo}; s < hi; ++s) {
-            e.sec_pos[s] = pos * 8;
-            pos += sec_bytes[s];
+#pragma unroll
+        for (int k{0}; k < 4; ++k) pos[k] += e.sec_shift[sec[k]];
+#pragma unroll
+        for (int k{0}; k < 4; ++k) {
+            const std::uint32_t u{u0 + k * kLayoutThreads};
+            if (u >= units) break;
+            e.unit_pos[u] = pos[k];
+            // A unit of several sections has its last bit elsewhere, in words
+            // zeroed below; the one found here is then some other word of the body.
+            const unsigned long long last{(pos[k] + (bits[k] != 0 ? bits[k] - 1 : 0)) >> 5};
+            zero_out_word(e, pos[k] >> 5, file);
+            zero_out_word(e, last, file);
         }
     }
-    const unsigned long long framing{sh_start - sh_head};
-    for (unsigned long long i{static_cast<unsigned long long>(tid)}; i < sh_head; i += kLayoutThreads) {
-        e.out[framing + i] = head[i];
+    // Sections that start inside a unit: the emission ORs that unit's part of
+    // them bit by bit, and the section before them ends there. A warp each.
+    for (int s{1 + (tid >> 5)}; s < e.ndc + 2; s += kLayoutWarps) {
+        const Section sec{e.sections[s]};
+        if (sec.first % kMiscItemsPerUnit == 0) continue;
+        const std::uint32_t end{min(sec.first + sec.count, (sec.unit + 1) * kMiscItemsPerUnit)};
+        const unsigned long long from{section_start(e, s)};
+        const unsigned long long to{end < sec.first + sec.count ? e.unit_off[sec.unit + 1] : section_start(e, s + 1)};
+        const unsigned long long shift{e.sec_shift[s]};
+        for (unsigned long long w{((shift + from) >> 5) + (tid & 31)}; w < (shift + to + 31) >> 5; w += 32) {
+            zero_out_word(e, w, file);
+        }
+        if ((tid & 31) == 0) zero_out_word(e, (e.sec_shift[s - 1] + from - 1) >> 5, file);
+    }
+    const unsigned long long head_w0{framing / 4};
+    for (unsigned long long w{head_w0 + tid}; 4 * w < framing + head; w += kLayoutThreads) zero_out_word(e, w, file);
+    __syncthreads();
+
+    // Container framing in bytes, headers and TOC ORed in.
+    if (tid < 48) {
+        constexpr std::uint8_t kHead[32]{0, 0, 0, 0x0c, 'J', 'X', 'L', ' ', 0x0d, 0x0a, 0x87, 0x0a, 0, 0, 0, 0x14,
+                                         'f', 't', 'y', 'p', 'j', 'x', 'l', ' ', 0, 0, 0, 0, 'j', 'x', 'l', ' '};
+        constexpr std::uint8_t kBox[4]{'j', 'x', 'l', 'c'};
+        const unsigned long long box{cs + (large ? 16 : 8)};
+        const std::uint32_t sf{large ? 1u : static_cast<std::uint32_t>(box)};
+        if (tid < 32) {
+            e.out[tid] = kHead[tid];
+        } else if (tid < 36) {
+            e.out[tid] = static_cast<std::uint8_t>(sf >> (8 * (35 - tid)));
+        } else if (tid < 40) {
+            e.out[tid] = kBox[tid - 36];
+        } else if (large) {
+            e.out[tid] = static_cast<std::uint8_t>(box >> (8 * (47 - tid)));
+        }
+    }
+    auto* words{reinterpret_cast<unsigned int*>(e.out)};
+    if (tid < 4 && e.head_words[tid] != 0) atomicOr(&words[head_w0 + tid], e.head_words[tid]);
+    unsigned long long p{8 * (framing + e.head_bytes) + toc_off};
+    for (int s{lo}; s < hi; ++s) {
+        if (hi - lo > 1) {
+            const unsigned long long from{section_start(e, s)};
+            toc_entry(static_cast<std::uint32_t>((section_start(e, s + 1) - from + 7) / 8), nb, field);
+        }
+        const std::uint32_t off{static_cast<std::uint32_t>(p & 31)};
+        atomicOr(&words[p >> 5], field << off);
+        if (off + nb > 32) atomicOr(&words[(p >> 5) + 1], field >> (32 - off));
+        p += nb;
     }
 }
 
-__device__ __forceinline__ void zero_body_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    if (e.result[2] != 0) return;
-    const unsigned long long start{e.result[1]};
-    const unsigned long long end{e.result[0]};
-    const unsigned long long a{(start + 15) & ~15ull};
-    const unsigned long long stride{static_cast<unsigned long long>(nblk) * blockDim.x};
-    const unsigned long long tid{static_cast<unsigned long long>(blk) * blockDim.x + threadIdx.x};
-    if (tid < a - start && start + tid < end) e.out[start + tid] = 0;
-    const unsigned long long nvec{end > a ? (end - a) / 16 : 0};
-    uint4* v{reinterpret_cast<uint4*>(e.out + a)};
-    for (unsigned long long i{tid}; i < nvec; i += stride) v[i] = make_uint4(0, 0, 0, 0);
-    const unsigned long long tail{a + nvec * 16};
-    if (tail + tid < end && tid < 16) e.out[tail + tid] = 0;
+__device__ __forceinline__ void lengths_body(const EntropyDev& e, const unsigned blk) {
+    if (blk < static_cast<unsigned>(e.nstripes)) {
+        ac_bits_stored_body(e, blk);
+    } else {
+        misc_bits_body(e, blk - static_cast<unsigned>(e.nstripes));
+    }
 }
 
 // ---- pass 5: emission ------------------------------------------------------------
@@ -1847,82 +1863,119 @@ __device__ void flush_window(const unsigned int* win, int nwords, unsigned int* 
     }
 }
 
-// Writes a stripe's tokens. The stripe's bits are contiguous in its section;
-// they are assembled in a shared-memory window and written out with plain
-// stores (global atomics only when the stripe exceeds the window).
-template <int kSet>
-__device__ __forceinline__ void ac_emit_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+// Where a unit's bits go: a shared-memory window of the words they touch, or,
+// when those exceed the window, the output itself, whose words between the
+// unit's first and last (zeroed by the layout) the CTA zeroes here. `base` is
+// the unit's first bit in `words`.
+struct EmitTarget {
+    unsigned int* words;
+    unsigned long long base;
+    unsigned long long w0;  // first word of the unit in the output
+    int window;             // words of the window, -1 without one
+};
+
+__device__ __forceinline__ EmitTarget emit_target(const EntropyDev& e, unsigned long long pos, std::uint32_t bits,
+                                                  unsigned int* win, int capacity) {
+    auto* out{reinterpret_cast<unsigned int*>(e.out)};
+    const unsigned long long w0{pos >> 5};
+    const unsigned long long nw{bits == 0 ? 0ull : ((pos + bits + 31) >> 5) - w0};
+    if (nw <= static_cast<unsigned long long>(capacity)) {
+        for (int i{static_cast<int>(threadIdx.x)}; i < static_cast<int>(nw); i += blockDim.x) win[i] = 0;
+        return {win, pos & 31, w0, static_cast<int>(nw)};
+    }
+    for (unsigned long long w{w0 + 1 + threadIdx.x}; w + 1 < w0 + nw; w += blockDim.x) out[w] = 0;
+    return {out, pos, w0, -1};
+}
+
+// Writes a stored stripe's tokens, in stream order: their lengths, a CTA scan
+// for their offsets, and their bits, eight consecutive tokens per thread and
+// round gathered into whole words on the way to the window.
+//
+// Latency-bound: one round (2048 tokens; a stripe of a 4K frame at distance 1
+// has some 1400) is a pool load, the scan and the stores, where rounds of four
+// tokens with two or three ORs each into shared memory took several. The code
+// table is copied to shared memory while the first tokens load.
+__device__ __forceinline__ void ac_emit_stored_body(const EntropyDev& e, const unsigned blk) {
+    extern __shared__ __align__(16) unsigned char ac_smem[];
+    unsigned int* win{reinterpret_cast<unsigned int*>(ac_smem)};                     // [kWindowWords]
+    auto* code{reinterpret_cast<std::uint32_t*>(ac_smem + kWindowWords * 4)};        // [32][64]
+    __shared__ std::uint32_t sh_scan[kAcWarps + 1];
+    constexpr int kPer{8};
+    const std::uint32_t tid{threadIdx.x};
+    const Stripe st{e.stripes[blk]};
+    const StripeTokens pool{stripe_tokens(e, st, blk, st.rows * st.cols)};
+    if (pool.near == nullptr || e.result[2] != 0) return;
+    const std::uint32_t ntok{e.stripe_tok[2 * blk + 1]};
+    const unsigned long long pos{e.unit_pos[e.misc_units + blk]};
+    const std::uint32_t bits{e.unit_sum[e.misc_units + blk]};
+    for (int i{static_cast<int>(tid)}; i < kNumClusters * kAcSymbols / 4; i += kAcThreads) {
+        reinterpret_cast<uint4*>(code)[i] = __ldg(reinterpret_cast<const uint4*>(e.code) + i);
+    }
+    const EmitTarget to{emit_target(e, pos, bits, win, kWindowWords)};
+    __syncthreads();
+    unsigned long long run{to.base};
+    for (std::uint32_t t0{0}; t0 < ntok; t0 += kAcThreads * kPer) {
+        const std::uint32_t t{t0 + tid * kPer};
+        std::uint32_t tk[kPer];
+        std::uint32_t cd[kPer];
+        std::uint32_t local{0};
+        // A thread's eight tokens lie on one side of the split. Direct places
+        // are 16-byte aligned, reserved runs may not be.
+        const std::uint32_t* src{pool.at(t)};
+        if (t + kPer <= ntok && (reinterpret_cast<std::uintptr_t>(src) & 15u) == 0) {
+            const uint4 a{reinterpret_cast<const uint4*>(src)[0]};
+            const uint4 b{reinterpret_cast<const uint4*>(src)[1]};
+            tk[0] = a.x; tk[1] = a.y; tk[2] = a.z; tk[3] = a.w;
+            tk[4] = b.x; tk[5] = b.y; tk[6] = b.z; tk[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i{0}; i < kPer; ++i) tk[i] = t + i < ntok ? src[i] : 0u;
+        }
+#pragma unroll
+        for (int i{0}; i < kPer; ++i) {
+            cd[i] = t + i < ntok ? code[token_code_index(tk[i])] : 0u;
+            local += (cd[i] >> 16) + (t + i < ntok ? token_extra_count(tk[i]) : 0u);
+        }
+        std::uint32_t total{0};
+        const unsigned long long at{run + cta_exclusive_scan(local, sh_scan, total)};
+        unsigned int* w{to.words + (at >> 5)};
+        unsigned long long acc{0};
+        std::uint32_t fill{static_cast<std::uint32_t>(at & 31)};
+#pragma unroll
+        for (int i{0}; i < kPer; ++i) {
+            if (t + i >= ntok) break;
+            const std::uint32_t depth{cd[i] >> 16};
+            const std::uint32_t v{(cd[i] & 0xffffu) | (token_extra_bits(tk[i]) << depth)};
+            acc |= static_cast<unsigned long long>(v) << fill;  // at most 15 + 13 bits on at most 31
+            fill += depth + token_extra_count(tk[i]);
+            if (fill >= 32) {
+                atomicOr(w++, static_cast<unsigned int>(acc));
+                acc >>= 32;
+                fill -= 32;
+            }
+        }
+        if (acc != 0) atomicOr(w, static_cast<unsigned int>(acc));
+        run += total;
+    }
+    __syncthreads();
+    if (to.window > 0) flush_window(win, to.window, reinterpret_cast<unsigned int*>(e.out), to.w0);
+}
+
+// Tokenises an unstored stripe again and writes its tokens.
+__device__ __forceinline__ void ac_emit_unstored_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char ac_smem[];
     StripeStage& s{*reinterpret_cast<StripeStage*>(ac_smem)};
-    // Stored stripes need no staging: their window starts the allocation.
-    unsigned int* win{reinterpret_cast<unsigned int*>(ac_smem + (kSet == kStoredStripes ? 0 : sizeof(StripeStage)))};
-    __shared__ unsigned long long sh_start;
-    __shared__ unsigned long long sh_p0;
-    __shared__ int sh_words;
-    if (e.result[2] != 0) return;
+    unsigned int* win{reinterpret_cast<unsigned int*>(ac_smem + sizeof(StripeStage))};
     const int tid{static_cast<int>(threadIdx.x)};
     const int lane{tid & 31};
     const Stripe st{e.stripes[blk]};
     const GroupGeom gg{ac_group_geom(e, st.group)};
     const int nitems{3 * st.rows * gg.gw};
-    const StripeTokens pool{stripe_tokens(e, st, blk, st.rows * gg.gw)};
-    if ((pool.near != nullptr) != (kSet == kStoredStripes)) return;
-    if (kSet == kUnstoredStripes) stage_stripe(e, st, gg, s);
-    if (tid == 0) {
-        const Section sec{e.sections[st.section]};
-        const unsigned long long p0{prefix_at(e, st.item0)};
-        const unsigned long long start{e.sec_pos[st.section] + (p0 - prefix_at(e, sec.first))};
-        const unsigned long long bits{prefix_at(e, st.item0 + static_cast<std::uint32_t>(nitems)) - p0};
-        const unsigned long long nw{bits == 0 ? 0ull : ((start + bits + 31) >> 5) - (start >> 5)};
-        sh_start = start;
-        sh_p0 = p0;
-        sh_words = nw <= static_cast<unsigned long long>(kWindowWords) ? static_cast<int>(nw) : -1;
-    }
+    stage_stripe(e, st, gg, s);
+    const EmitTarget to{
+        emit_target(e, e.unit_pos[e.misc_units + blk], e.unit_sum[e.misc_units + blk], win, kWindowWords)};
     __syncthreads();
-    const int nwords{sh_words};
-    for (int i{tid}; i < nwords; i += kAcThreads) win[i] = 0;
-    unsigned int* words{nwords >= 0 ? win : reinterpret_cast<unsigned int*>(e.out)};
-    const unsigned long long base{nwords >= 0 ? (sh_start & 31) : sh_start};
-    if (pool.near != nullptr) {
-        // Stored tokens in stream order: their lengths, a CTA scan for their
-        // offsets, and their bits, kAcThreads * kPer tokens per round.
-        __shared__ std::uint32_t sh_scan[kAcWarps + 1];
-        constexpr int kPer{4};
-        const std::uint32_t ntok{e.stripe_tok[2 * blk + 1]};
-        __syncthreads();
-        unsigned long long run{base};
-        for (std::uint32_t t0{0}; t0 < ntok; t0 += kAcThreads * kPer) {
-            std::uint32_t tk[kPer];
-            std::uint32_t len[kPer];
-            std::uint32_t local{0};
-#pragma unroll
-            for (int i{0}; i < kPer; ++i) {
-                const std::uint32_t t{t0 + static_cast<std::uint32_t>(tid) * kPer + i};
-                tk[i] = t < ntok ? *pool.at(t) : 0u;
-                len[i] = t < ntok ? __ldg(&e.ac_depth[token_table_index(tk[i])]) + token_extra_count(tk[i]) : 0u;
-                local += len[i];
-            }
-            std::uint32_t total{0};
-            unsigned long long at{run + cta_exclusive_scan(local, sh_scan, total)};
-#pragma unroll
-            for (int i{0}; i < kPer; ++i) {
-                if (len[i] == 0) continue;
-                const std::uint32_t idx{token_table_index(tk[i])};
-                const std::uint32_t d{__ldg(&e.ac_depth[idx])};
-                put_bits_at(words, at, d, __ldg(&e.ac_bits[idx]));
-                const std::uint32_t nb{token_extra_count(tk[i])};
-                if (nb) put_bits_at(words, at + d, nb, token_extra_bits(tk[i]));
-                at += len[i];
-            }
-            run += total;
-        }
-        __syncthreads();
-        if (nwords > 0) flush_window(win, nwords, reinterpret_cast<unsigned int*>(e.out), sh_start >> 5);
-        return;
-    }
-    for (int j{tid}; j < nitems; j += kAcThreads) {
-        s.aux[j] = static_cast<std::uint32_t>(prefix_at(e, st.item0 + static_cast<std::uint32_t>(j)) - sh_p0);
-    }
+    for (int j{tid}; j < nitems; j += kAcThreads) s.aux[j] = e.item_pre[st.item0 + j];
     __syncthreads();
     for (int j{tid}; j < nitems; j += kAcThreads) {
         const StripeItem it{stripe_item(s, gg.gw, j)};
@@ -1931,9 +1984,9 @@ __device__ __forceinline__ void ac_emit_body(const EntropyDev& e, const unsigned
         std::uint32_t tok, nb, bits;
         count_token(s, st, it, cl, tok, nb, bits);
         const std::uint32_t d{__ldg(&e.ac_depth[cl * 256 + tok])};
-        const unsigned long long at{base + s.aux[j]};
-        put_bits_at(words, at, d, __ldg(&e.ac_bits[cl * 256 + tok]));
-        if (nb) put_bits_at(words, at + d, nb, bits);
+        const unsigned long long at{to.base + s.aux[j]};
+        put_bits_at(to.words, at, d, __ldg(&e.ac_bits[cl * 256 + tok]));
+        if (nb) put_bits_at(to.words, at + d, nb, bits);
         if (it.nz != 0) {
             s.active[atomicAdd(&s.nactive, 1)] = static_cast<std::uint16_t>(j);
             s.aux[j] += d + nb;  // coefficient tokens start after the count token
@@ -1943,21 +1996,21 @@ __device__ __forceinline__ void ac_emit_body(const EntropyDev& e, const unsigned
     for (int a{tid >> 5}; a < s.nactive; a += kAcWarps) {
         const int j{s.active[a]};
         const StripeItem it{stripe_item(s, gg.gw, j)};
-        unsigned long long pos{base + s.aux[j]};
+        unsigned long long pos{to.base + s.aux[j]};
         coeff_tokens(s, it, lane, [&](bool has, int cl, std::uint32_t sym, std::uint32_t nb, std::uint32_t bits) {
             const std::uint32_t d{has ? __ldg(&e.ac_depth[cl * 256 + sym]) : 0u};
             const std::uint32_t tb{has ? d + nb : 0u};
             const std::uint32_t incl{warp_incl_scan(tb, lane)};
             if (has) {
                 const unsigned long long at{pos + incl - tb};
-                put_bits_at(words, at, d, __ldg(&e.ac_bits[cl * 256 + sym]));
-                if (nb) put_bits_at(words, at + d, nb, bits);
+                put_bits_at(to.words, at, d, __ldg(&e.ac_bits[cl * 256 + sym]));
+                if (nb) put_bits_at(to.words, at + d, nb, bits);
             }
             pos += __shfl_sync(kFull, incl, 31);
         });
     }
     __syncthreads();
-    if (nwords > 0) flush_window(win, nwords, reinterpret_cast<unsigned int*>(e.out), sh_start >> 5);
+    if (to.window > 0) flush_window(win, to.window, reinterpret_cast<unsigned int*>(e.out), to.w0);
 }
 
 // A header blob long enough to be written by the whole CTA (the AcGlobal
@@ -2012,7 +2065,7 @@ struct EmitVisitor {
         put(4, nb);
         put(nb, v - (1u << nb));
     }
-    __device__ void count_field(int g, unsigned nbits) { put(nbits, e->fb_count[g] - 1); }
+    __device__ void count_field(int g, unsigned nbits) { put(nbits, e->frozen[1 + g] - 1); }
     __device__ void epf(int g) { put(e->am_depth[g * 256], e->am_bits[g * 256]); }
     __device__ void first_block(int) {}
     __device__ void token(int tab, int g, std::uint32_t sym, std::uint32_t nb, std::uint32_t bits) {
@@ -2025,46 +2078,55 @@ struct EmitVisitor {
 
 constexpr int kMiscWindowWords = 2048;
 
-// One thread per non-AC item; the bits of the block's items that share the
-// first item's section are assembled in a shared-memory window.
-__device__ __forceinline__ void misc_emit_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+// One unit of other items, two per thread; the bits of the items that share the
+// first item's section go through a shared-memory window.
+__device__ __forceinline__ void misc_emit_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char misc_smem[];
     unsigned int* win{reinterpret_cast<unsigned int*>(misc_smem)};                              // [kMiscWindowWords]
     DeferredBlob* deferred{reinterpret_cast<DeferredBlob*>(misc_smem + kMiscWindowWords * 4)};  // [kMaxDeferred]
-    __shared__ unsigned long long sh_start;
-    __shared__ std::uint32_t sh_end;
-    __shared__ int sh_words;
     __shared__ int sh_ndeferred;
     if (e.result[2] != 0) return;
-    const std::uint32_t first{blk * kMiscItemsPerBlock};
-    if (threadIdx.x == 0) {
-        sh_ndeferred = 0;
-        const int s0{find_section(e.sections, 0, misc_hi(e), first)};
-        const Section sec{e.sections[s0]};
-        const std::uint32_t end{min(min(first + kMiscItemsPerBlock, sec.first + sec.count), e.ac_first)};
-        const unsigned long long p0{prefix_at(e, first)};
-        const unsigned long long start{e.sec_pos[s0] + (p0 - prefix_at(e, sec.first))};
-        const unsigned long long bits{prefix_at(e, end) - p0};
-        const unsigned long long nw{bits == 0 ? 0ull : ((start + bits + 31) >> 5) - (start >> 5)};
-        sh_start = start;
-        sh_end = end;
-        sh_words = nw <= static_cast<unsigned long long>(kMiscWindowWords) ? static_cast<int>(nw) : -1;
-    }
+    const std::uint32_t first{blk * kMiscItemsPerUnit};
+    const int sfirst{static_cast<int>(e.unit_section[blk])};
+    const Section sec0{e.sections[sfirst]};
+    const unsigned long long pos0{e.unit_pos[blk]};
+    if (threadIdx.x == 0) sh_ndeferred = 0;
+    const bool whole{sec0.first + sec0.count >= min(first + kMiscItemsPerUnit, e.ac_first)};
+    const std::uint32_t bits{whole ? e.unit_sum[blk]
+                                   : static_cast<std::uint32_t>(section_start(e, sfirst + 1) - e.unit_off[blk])};
+    const EmitTarget to{emit_target(e, pos0, bits, win, kMiscWindowWords)};
     __syncthreads();
-    const int nwords{sh_words};
-    for (int i{static_cast<int>(threadIdx.x)}; i < nwords; i += blockDim.x) win[i] = 0;
-    __syncthreads();
+    std::uint32_t tok[kMiscPerThread];
+    std::uint32_t pre[kMiscPerThread];
 #pragma unroll
     for (int k{0}; k < kMiscPerThread; ++k) {
-        const std::uint32_t item{first + threadIdx.x + k * blockDim.x};
-        if (item < e.ac_first) {
-            const int s{find_section(e.sections, 0, misc_hi(e), item)};
-            const Section sec{e.sections[s]};
-            const unsigned long long pos{e.sec_pos[s] + (prefix_at(e, item) - prefix_at(e, sec.first))};
-            const bool in_window{nwords >= 0 && item < sh_end};
-            EmitVisitor v{&e, in_window ? win : reinterpret_cast<unsigned int*>(e.out),
-                          in_window ? pos - ((sh_start >> 5) << 5) : pos, deferred, &sh_ndeferred};
-            visit_misc(e, item, v);
+        const std::uint32_t item{first + threadIdx.x + k * kAcThreads};
+        tok[k] = item < e.ac_first ? e.item_tok[item] : kMiscNone;
+        pre[k] = item < e.ac_first ? e.item_pre[item] : 0u;
+    }
+#pragma unroll
+    for (int k{0}; k < kMiscPerThread; ++k) {
+        if (tok[k] == kMiscNone) continue;
+        const std::uint32_t item{first + threadIdx.x + k * kAcThreads};
+        int sat{sfirst};
+        const Section sec{section_from(e, sat, item)};
+        unsigned int* words{to.words};
+        unsigned long long pos{to.base + pre[k]};
+        if (sat != sfirst) {
+            words = reinterpret_cast<unsigned int*>(e.out);
+            pos = e.sec_shift[sat] + e.unit_off[blk] + pre[k];
+        }
+        if (tok[k] == kMiscVisit) {
+            EmitVisitor v{&e, words, pos, deferred, &sh_ndeferred};
+            visit_misc(e, sec, item - sec.first, v);
+        } else {
+            // At most 15 + 18 bits on at most 31: two words.
+            const std::uint32_t cd{misc_code(e, sec.group, tok[k])};
+            const unsigned long long v{((cd & 0xffffu) |
+                                        (static_cast<unsigned long long>(misc_extra_bits(tok[k])) << (cd >> 16)))
+                                       << (pos & 31)};
+            if (static_cast<unsigned int>(v) != 0) atomicOr(&words[pos >> 5], static_cast<unsigned int>(v));
+            if ((v >> 32) != 0) atomicOr(&words[(pos >> 5) + 1], static_cast<unsigned int>(v >> 32));
         }
     }
     __syncthreads();
@@ -2081,10 +2143,9 @@ __device__ __forceinline__ void misc_emit_body(const EntropyDev& e, const unsign
         }
     }
     __syncthreads();
-    if (nwords > 0) flush_window(win, nwords, reinterpret_cast<unsigned int*>(e.out), sh_start >> 5);
+    if (to.window > 0) flush_window(win, to.window, reinterpret_cast<unsigned int*>(e.out), to.w0);
 }
 
-// Clears a frame's histograms and counters (the first step of every encode).
 // Zeroes a frame's histograms, first-block counts and token-pool fill; block
 // blk of nblk takes every nblk-th 256-word stretch.
 __device__ __forceinline__ void clear_body(const EntropyDev& e, unsigned blk, unsigned nblk) {
@@ -2104,18 +2165,13 @@ __host__ __device__ constexpr unsigned clear_blocks(int ndc) { return 1u + stati
 
 // ---- kernels: one frame per launch, and every frame of a batch per launch -----------
 
-// Blocks of a single-frame launch of the body-zeroing pass.
-constexpr unsigned kZeroBlocks = 296;
-// Blocks per frame of the body-zeroing pass in a batched launch.
-constexpr unsigned kZeroBlocksBatched = 32;
-
-#define JXB_ENTROPY_KERNELS(NAME, BOUNDS, PHASE, NBLK)                                                     \
+#define JXB_ENTROPY_KERNELS(NAME, BOUNDS, PHASE)                                                           \
     __global__ void BOUNDS NAME##_kernel(const __grid_constant__ EntropyDev e) {                              \
-        NAME##_body(e, blockIdx.x, gridDim.x);                                                                \
+        NAME##_body(e, blockIdx.x);                                                                           \
     }                                                                                                         \
     __global__ void BOUNDS NAME##_batch_kernel(const __grid_constant__ EntropyBatch b) {                      \
         const int f{batch_frame(b, PHASE, blockIdx.x)};                                                      \
-        NAME##_body(b.frames[f], blockIdx.x - b.begin[PHASE][f], NBLK);                                       \
+        NAME##_body(b.frames[f], blockIdx.x - b.begin[PHASE][f]);                                             \
     }
 
 // Frame of block `blk` of a batched launch of `phase` (binary search over the
@@ -2137,44 +2193,30 @@ __device__ __forceinline__ int batch_frame(const EntropyBatch& b, int phase, uns
 // The three item passes run the AC stripes (blocks 0 .. nstripes - 1, the
 // long ones, scheduled first) and the other items (the blocks after them) as
 // one launch: the two kinds are independent within a pass.
-__device__ __forceinline__ void tokens_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+__device__ __forceinline__ void tokens_body(const EntropyDev& e, const unsigned blk) {
     if (blk < static_cast<unsigned>(e.nstripes)) {
         ac_tok_direct_body(e, blk);
     } else {
-        misc_hist_body(e, blk - static_cast<unsigned>(e.nstripes), nblk);
+        misc_hist_body(e, blk - static_cast<unsigned>(e.nstripes));
     }
 }
-__device__ __forceinline__ void lengths_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
+__device__ __forceinline__ void emit_body(const EntropyDev& e, const unsigned blk) {
     if (blk < static_cast<unsigned>(e.nstripes)) {
-        ac_bits_body<kStoredStripes>(e, blk, nblk);
+        ac_emit_stored_body(e, blk);
     } else {
-        misc_bits_body(e, blk - static_cast<unsigned>(e.nstripes), nblk);
+        misc_emit_body(e, blk - static_cast<unsigned>(e.nstripes));
     }
-}
-__device__ __forceinline__ void emit_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    if (blk < static_cast<unsigned>(e.nstripes)) {
-        ac_emit_body<kStoredStripes>(e, blk, nblk);
-    } else {
-        misc_emit_body(e, blk - static_cast<unsigned>(e.nstripes), nblk);
-    }
-}
-// Stripes whose tokens did not fit the pool, with their coefficients staged
-// (their CTAs return at once for stored stripes).
-__device__ __forceinline__ void lengths_unstored_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    ac_bits_body<kUnstoredStripes>(e, blk, nblk);
-}
-__device__ __forceinline__ void emit_unstored_body(const EntropyDev& e, const unsigned blk, const unsigned nblk) {
-    ac_emit_body<kUnstoredStripes>(e, blk, nblk);
 }
 
-JXB_ENTROPY_KERNELS(tokens, __launch_bounds__(kAcThreads), kPhaseItems, 0u)
-JXB_ENTROPY_KERNELS(codes, __launch_bounds__(32), kPhaseCodes, 0u)
-JXB_ENTROPY_KERNELS(lengths, __launch_bounds__(kAcThreads), kPhaseItems, 0u)
-JXB_ENTROPY_KERNELS(scan_tile, __launch_bounds__(1024), kPhaseScan, 0u)
-JXB_ENTROPY_KERNELS(scan_top, __launch_bounds__(1024), kPhaseFrame, 0u)
-JXB_ENTROPY_KERNELS(layout, __launch_bounds__(kLayoutThreads), kPhaseFrame, 0u)
-JXB_ENTROPY_KERNELS(zero_body, __launch_bounds__(256), kPhaseZero, kZeroBlocksBatched)
-JXB_ENTROPY_KERNELS(emit, __launch_bounds__(kAcThreads), kPhaseItems, 0u)
+JXB_ENTROPY_KERNELS(tokens, __launch_bounds__(kAcThreads, 3), kPhaseItems)
+JXB_ENTROPY_KERNELS(codes, __launch_bounds__(32), kPhaseCodes)
+JXB_ENTROPY_KERNELS(lengths, __launch_bounds__(kAcThreads, 8), kPhaseItems)
+__global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const __grid_constant__ EntropyDev e) { layout_body(e); }
+__global__ void __launch_bounds__(kLayoutThreads) layout_batch_kernel(const __grid_constant__ EntropyBatch b) {
+    layout_body(b.frames[blockIdx.x]);
+}
+// Five CTAs per SM (latency-bound: the window and code table fill the rest).
+JXB_ENTROPY_KERNELS(emit, __launch_bounds__(kAcThreads, 5), kPhaseItems)
 // Stripes whose tokens did not fit the pool are rare, so their passes run on
 // a few resident CTAs that skip the stored stripes with one load each.
 constexpr unsigned kUnstoredCtas = 148;
@@ -2182,28 +2224,28 @@ constexpr unsigned kUnstoredCtas = 148;
 // Every stripe adds its token count to the pool fill whether or not it fits,
 // so a frame has an unstored stripe exactly when its final fill exceeds the
 // capacity; a frame without one is passed over after one load.
-__device__ __forceinline__ bool frame_all_stored(const EntropyDev& e) { return *e.tok_count <= e.tok_capacity; }
+__device__ __forceinline__ bool frame_all_stored(const EntropyDev& e) { return e.frozen[0] <= e.tok_capacity; }
 
-#define JXB_UNSTORED_KERNELS(NAME)                                                                         \
-    __global__ void __launch_bounds__(kAcThreads) NAME##_kernel(const __grid_constant__ EntropyDev e) {       \
-        if (frame_all_stored(e)) return;                                                                      \
-        for (unsigned s{blockIdx.x}; s < static_cast<unsigned>(e.nstripes); s += gridDim.x) {                 \
-            if (e.stripe_tok[2 * s] != kNoTokens) continue;                                                   \
-            NAME##_body(e, s, 0u);                                                                            \
-            __syncthreads();                                                                                  \
-        }                                                                                                     \
+__global__ void __launch_bounds__(kAcThreads) lengths_unstored_kernel(const __grid_constant__ EntropyDev e) {
+    if (frame_all_stored(e)) return;
+    for (unsigned s{blockIdx.x}; s < static_cast<unsigned>(e.nstripes); s += gridDim.x) {
+        if (e.stripe_tok[2 * s] != kNoTokens) continue;
+        ac_bits_unstored_body(e, s);
+        __syncthreads();
     }
-
-JXB_UNSTORED_KERNELS(lengths_unstored)
-JXB_UNSTORED_KERNELS(emit_unstored)
-#undef JXB_UNSTORED_KERNELS
+}
+__global__ void __launch_bounds__(kAcThreads) emit_unstored_kernel(const __grid_constant__ EntropyDev e) {
+    if (frame_all_stored(e) || e.result[2] != 0) return;
+    for (unsigned s{blockIdx.x}; s < static_cast<unsigned>(e.nstripes); s += gridDim.x) {
+        if (e.stripe_tok[2 * s] != kNoTokens) continue;
+        ac_emit_unstored_body(e, s);
+        __syncthreads();
+    }
+}
 #undef JXB_ENTROPY_KERNELS
 
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ EntropyDev e) {
     clear_body(e, blockIdx.x, gridDim.x);
-}
-__global__ void __launch_bounds__(256) clear_batch_kernel(const __grid_constant__ EntropyBatch b) {
-    clear_body(b.frames[blockIdx.x], 0u, 1u);
 }
 
 // The token pass of planes given by the caller.
@@ -2211,18 +2253,17 @@ __global__ void __launch_bounds__(kAcThreads) tokens_staged_kernel(const __grid_
     if (blockIdx.x < static_cast<unsigned>(e.nstripes)) {
         ac_tok_body(e, blockIdx.x);
     } else {
-        misc_hist_body(e, blockIdx.x - static_cast<unsigned>(e.nstripes), gridDim.x);
+        misc_hist_body(e, blockIdx.x - static_cast<unsigned>(e.nstripes));
     }
 }
 
 constexpr std::size_t kHistSmem{sizeof(StripeStage) + kNumClusters * kAcSymbols * sizeof(std::uint32_t)};
 constexpr std::size_t kBitsSmem{sizeof(StripeStage)};
 constexpr std::size_t kEmitSmem{sizeof(StripeStage) + kWindowWords * sizeof(unsigned int)};
-// Emission of stored stripes and other items: the larger of their windows.
-constexpr std::size_t kEmitStoredSmem{kWindowWords * sizeof(unsigned int) >
-                                              kMiscWindowWords * sizeof(unsigned int) + kMaxDeferred * sizeof(DeferredBlob)
-                                          ? kWindowWords * sizeof(unsigned int)
-                                          : kMiscWindowWords * sizeof(unsigned int) + kMaxDeferred * sizeof(DeferredBlob)};
+// Emission of stored stripes (window and code table) and of other items.
+constexpr std::size_t kEmitStoredSmem{(kWindowWords + kNumClusters * kAcSymbols) * sizeof(unsigned int)};
+static_assert(kEmitStoredSmem >= kMiscWindowWords * sizeof(unsigned int) + kMaxDeferred * sizeof(DeferredBlob),
+              "emission shared memory");
 // The other items' passes share these launches and their shared memory.
 constexpr std::size_t kDirectSmem{sizeof(DirectStage)};
 static_assert(kHistSmem >= (4 * 256 + 2) * sizeof(std::uint32_t) && kDirectSmem >= (4 * 256 + 2) * sizeof(std::uint32_t) &&
@@ -2237,23 +2278,18 @@ static_assert(sizeof(EntropyBatch) <= 32000, "a batched entropy launch's paramet
 bool entropy_launch(const EntropyDev& e, void* stream) {
     if (e.nsec > kMaxSections) return false;
     cudaStream_t st{static_cast<cudaStream_t>(stream)};
-    const unsigned misc{(e.ac_first + kMiscItemsPerBlock - 1) / kMiscItemsPerBlock};
-    const unsigned stripes{static_cast<unsigned>(e.nstripes)};
-    const std::uint32_t layout_smem{layout_sizes_bytes(e.nsec) + layout_head_bytes(e.nsec)};
-    clear_kernel<<<clear_blocks(e.ndc), 256, 0, st>>>(e);  // histograms, first-block counts, pool fill
+    const unsigned units{e.misc_units + static_cast<unsigned>(e.nstripes)};
+    if (e.clear_first) clear_kernel<<<clear_blocks(e.ndc), 256, 0, st>>>(e);
     if (e.direct) {
-        tokens_kernel<<<stripes + misc, kAcThreads, kDirectSmem, st>>>(e);
+        tokens_kernel<<<units, kAcThreads, kDirectSmem, st>>>(e);
     } else {
-        tokens_staged_kernel<<<stripes + misc, kAcThreads, kHistSmem, st>>>(e);
+        tokens_staged_kernel<<<units, kAcThreads, kHistSmem, st>>>(e);
     }
     codes_kernel<<<kNumClusters + 2 * e.ndc, 32, sizeof(WarpCodeSmem), st>>>(e);
-    lengths_kernel<<<stripes + misc, kAcThreads, 0, st>>>(e);
     if (!e.direct) lengths_unstored_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(e);
-    scan_tile_kernel<<<e.num_tiles, 1024, 0, st>>>(e);
-    scan_top_kernel<<<1, 1024, 0, st>>>(e);
-    layout_kernel<<<1, kLayoutThreads, layout_smem, st>>>(e);
-    zero_body_kernel<<<kZeroBlocks, 256, 0, st>>>(e);
-    emit_kernel<<<stripes + misc, kAcThreads, kEmitStoredSmem, st>>>(e);
+    lengths_kernel<<<units, kAcThreads, 0, st>>>(e);
+    layout_kernel<<<1, kLayoutThreads, 0, st>>>(e);
+    emit_kernel<<<units, kAcThreads, kEmitStoredSmem, st>>>(e);
     if (!e.direct) emit_unstored_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(e);
     return cudaGetLastError() == cudaSuccess;
 }
@@ -2262,33 +2298,24 @@ void entropy_batch_plan(EntropyBatch& b) {
     for (int p{0}; p < kEntropyPhases; ++p) b.begin[p][0] = 0;
     for (int f{0}; f < b.nframes; ++f) {
         const EntropyDev& e{b.frames[f]};
-        const std::uint32_t per[kEntropyPhases]{static_cast<std::uint32_t>(e.nstripes) +
-                                                     (e.ac_first + kMiscItemsPerBlock - 1) / kMiscItemsPerBlock,
-                                                 static_cast<std::uint32_t>(kNumClusters + 2 * e.ndc), e.num_tiles,
-                                                 1u, kZeroBlocksBatched};
+        const std::uint32_t per[kEntropyPhases]{e.misc_units + static_cast<std::uint32_t>(e.nstripes),
+                                                 static_cast<std::uint32_t>(kNumClusters + 2 * e.ndc)};
         for (int p{0}; p < kEntropyPhases; ++p) b.begin[p][f + 1] = b.begin[p][f] + per[p];
     }
 }
 
 bool entropy_batch_launch(const EntropyBatch& b, void* stream) {
     if (b.nframes <= 0 || b.nframes > kEntropyBatchFrames) return false;
-    std::uint32_t layout_smem{0};
     for (int f{0}; f < b.nframes; ++f) {
-        const EntropyDev& e{b.frames[f]};
-        if (e.nsec > kMaxSections) return false;
-        layout_smem = std::max(layout_smem, layout_sizes_bytes(e.nsec) + layout_head_bytes(e.nsec));
+        if (b.frames[f].nsec > kMaxSections) return false;
     }
     cudaStream_t st{static_cast<cudaStream_t>(stream)};
     const int nf{b.nframes};
     const unsigned items{b.begin[kPhaseItems][nf]};
-    clear_batch_kernel<<<static_cast<unsigned>(nf), 256, 0, st>>>(b);
     tokens_batch_kernel<<<items, kAcThreads, kDirectSmem, st>>>(b);
     codes_batch_kernel<<<b.begin[kPhaseCodes][nf], 32, sizeof(WarpCodeSmem), st>>>(b);
     lengths_batch_kernel<<<items, kAcThreads, 0, st>>>(b);
-    scan_tile_batch_kernel<<<b.begin[kPhaseScan][nf], 1024, 0, st>>>(b);
-    scan_top_batch_kernel<<<static_cast<unsigned>(nf), 1024, 0, st>>>(b);
-    layout_batch_kernel<<<static_cast<unsigned>(nf), kLayoutThreads, layout_smem, st>>>(b);
-    zero_body_batch_kernel<<<b.begin[kPhaseZero][nf], 256, 0, st>>>(b);
+    layout_batch_kernel<<<static_cast<unsigned>(nf), kLayoutThreads, 0, st>>>(b);
     emit_batch_kernel<<<items, kAcThreads, kEmitStoredSmem, st>>>(b);
     return cudaGetLastError() == cudaSuccess;
 }
@@ -2335,8 +2362,6 @@ bool entropy_kernels_init() {
     if (cudaMemcpyToSymbol(g_coeff_ctx, ctx, sizeof(ctx)) != cudaSuccess) return false;
     return cudaFuncSetAttribute(codes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(sizeof(WarpCodeSmem))) == cudaSuccess &&
-           cudaFuncSetAttribute(layout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kLayoutSmemLimit)) == cudaSuccess &&
            cudaFuncSetAttribute(tokens_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kHistSmem)) == cudaSuccess &&
            cudaFuncSetAttribute(lengths_unstored_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2344,9 +2369,7 @@ bool entropy_kernels_init() {
            cudaFuncSetAttribute(emit_unstored_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kEmitSmem)) == cudaSuccess &&
            cudaFuncSetAttribute(codes_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(sizeof(WarpCodeSmem))) == cudaSuccess &&
-           cudaFuncSetAttribute(layout_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kLayoutSmemLimit)) == cudaSuccess;
+                                static_cast<int>(sizeof(WarpCodeSmem))) == cudaSuccess;
 }
 
 }  // namespace jxb

@@ -10,16 +10,17 @@
 //      the 32 cluster histograms and stored once in a token pool; the other
 //      items fill the per-DC-group DC and AcMetadata histograms;
 //   2. prefix codes built on the device, one warp per histogram;
-//   3. bit-length pass over all items, then a two-level exclusive scan;
-//   4. a layout CTA sizes every section, writes the container, headers and
-//      TOC, and places the sections;
+//   3. bit-length pass over all items: each unit (an AC stripe or 512 other
+//      items, the work of one CTA) sums and scans its own;
+//   4. a layout CTA scans the units, sizes every section, writes the
+//      container, headers and TOC, and places sections and units;
 //   5. an emit pass writes every item's bits at its final position.
-// Passes 1, 3 and 5 are one launch each: a CTA per AC stripe (one thread per
+// Passes 1, 3 and 5 are one launch each: a CTA per AC stripe (one lane per
 // token), then a CTA per 512 other items (two per thread). Planes given by
 // the caller are tokenised a warp per block-channel instead, and stripes whose
 // tokens did not fit the pool go through passes 3 and 5 in one more launch
-// each, with their coefficients staged again. A clear kernel zeroes the
-// histograms and the pool fill first.
+// each, with their coefficients staged again. The code pass leaves the
+// histograms and counters zeroed for the next frame.
 #pragma once
 
 #include <cstddef>
@@ -35,18 +36,20 @@ struct Section {
     std::uint32_t count;   // items in the section
     int kind;
     int group;             // DC or AC group index
+    std::uint32_t unit;    // unit that holds the first item
 };
 
 // Up to kStripeRows block rows of one AC group: the unit one CTA stages in
 // shared memory for the AC passes. Rows start at multiples of 4 inside the
 // group, so every DCT16/DCT32 transform lies inside one stripe.
 constexpr int kStripeRows = 4;
-struct Stripe {
+struct alignas(16) Stripe {
     std::uint32_t item0;   // global index of the stripe's first item
     std::int32_t section;  // section index of the AC group
     std::uint16_t group;   // AC group index
     std::uint8_t r0;       // first block row inside the group
     std::uint8_t rows;     // block rows, 1..kStripeRows
+    std::uint32_t cols;    // blocks per row
 };
 
 // Geometry and per-frame device state of the entropy stage. All pointers are
@@ -56,10 +59,11 @@ struct EntropyDev {
     int width, height, bw, bh, nblocks, xg, nac, xdg, ndc, cmw, nsec;
     std::uint32_t total_items;
     std::uint32_t ac_first;          // first item of the first AcGroup; AC block-channels follow
-    std::uint32_t num_tiles;         // scan tiles of kScanTile items
+    std::uint32_t misc_units;        // units of the items before ac_first; the stripes' units follow
     const Section* sections;
     const Stripe* stripes;
     int nstripes;
+    const std::uint32_t* unit_section;  // [misc_units + nstripes] section that holds each unit's first item
 
     // inputs (frontend outputs)
     const std::int16_t* ac;
@@ -82,14 +86,25 @@ struct EntropyDev {
     std::uint32_t ac_prefix_bits;
     const std::uint8_t* dc_global;   // DcGlobal section bits (per distance)
     std::uint32_t dc_global_bits;
+    std::uint32_t head_words[4];     // codestream header up to the TOC: signature, sizes, frame header
+    std::uint32_t head_bytes;
 
-    // per-frame scratch
+    // Per-frame scratch. The histograms and counters (ac_hist to tok_count)
+    // are zero between encodes: the passes that read them last clear them (with
+    // clear_first, for scratch without that history, a kernel clears them
+    // before the first pass).
+    bool clear_first;
     std::uint32_t* ac_hist;          // [32][256]
     std::uint32_t* dc_hist;          // [ndc][256]
     std::uint32_t* am_hist;          // [ndc][256]
-    std::uint32_t* fb_count;         // [ndc]
+    std::uint32_t* fb_count;         // [ndc] first blocks counted by the token pass
+    std::uint32_t* tok_count;        // [1] pool fill, or tokens at the output's end (direct)
+    std::uint32_t* frozen;           // [1 + ndc] tok_count and fb_count as the code pass found them
     std::uint8_t* ac_depth;          // [32][256]
     std::uint16_t* ac_bits;
+    // Depth << 16 | code bits of each symbol: [32][64] AC, then [ndc][128] DC
+    // and [ndc][128] AcMetadata.
+    std::uint32_t* code;
     std::uint8_t* dc_depth;          // [ndc][256]
     std::uint16_t* dc_bits;
     std::uint8_t* am_depth;          // [ndc][256]
@@ -97,11 +112,12 @@ struct EntropyDev {
     std::uint32_t* ac_alpha;         // [32]
     std::uint8_t* desc;              // [32 + 2*ndc][kDescBytes] code descriptions
     std::uint32_t* desc_bits;        // [32 + 2*ndc]
-    std::uint32_t* item_bits;        // [total_items]
-    std::uint32_t* item_pre;         // [total_items] exclusive prefix within its scan tile
-    std::uint32_t* tile_sum;         // [num_tiles]
-    unsigned long long* tile_off;    // [num_tiles + 1]
-    unsigned long long* sec_pos;     // [nsec] absolute bit offset of each section in `out`
+    std::uint32_t* item_pre;         // [total_items] exclusive prefix of the bits within the item's unit
+    std::uint32_t* item_tok;         // [ac_first] tokens of the items before the AC groups (pack_misc_token)
+    std::uint32_t* unit_sum;         // [unit_words] bits of each unit
+    unsigned long long* unit_off;    // [unit_words] bits before each unit, then their total
+    unsigned long long* unit_pos;    // [misc_units + nstripes] absolute bit offset of each unit in `out`
+    unsigned long long* sec_shift;   // [nsec] from a bit's place in the scan to its place in `out`
     unsigned long long* result;      // [4]: total bytes, body start, status, 0
 
     // AC tokens, written once by the token pass in stream order and read by
@@ -116,14 +132,14 @@ struct EntropyDev {
     bool direct;
     std::uint32_t* tok_pool;         // [tok_capacity] packed tokens (pack_ac_token)
     std::uint32_t tok_capacity;
-    std::uint32_t* tok_count;        // [1] pool fill, or tokens at the output's end (direct); zeroed per frame
     std::uint32_t* stripe_tok;       // [2 * nstripes]: place (pool offset or kNoTokens, or dense_tokens offset), token count
     std::uint8_t* out;               // output buffer (container + codestream)
     std::size_t out_capacity;
 };
 
 constexpr int kDescBytes = 256;
-constexpr int kScanTile = 4096;
+// Items of a unit that is not an AC stripe.
+constexpr std::uint32_t kMiscItemsPerUnit = 512;
 // Token pool capacity per 8x8 block: 4K frames at distance 0.5 use about 27,
 // at distance 1 about 11.
 constexpr std::uint32_t kTokensPerBlock = 32;
@@ -132,23 +148,18 @@ constexpr std::uint32_t kTokensPerBlock = 32;
 constexpr std::uint32_t kMaxTokensPerBlock = 192;
 constexpr std::uint32_t kNoTokens = 0xffffffffu;
 
-// Shared memory of the layout kernel: one 32-bit size per section, then the
-// codestream header, which is at most 64 bytes before the TOC plus 4 bytes
-// per TOC entry.
-__host__ __device__ constexpr std::uint32_t layout_sizes_bytes(int nsec) {
-    return (static_cast<std::uint32_t>(nsec) * 4 + 15) & ~15u;
-}
-__host__ __device__ constexpr std::uint32_t layout_head_bytes(int nsec) {
-    return 64 + static_cast<std::uint32_t>(nsec) * 4;
-}
-constexpr std::uint32_t kLayoutSmemLimit = 200 * 1024;
-constexpr int kMaxSections = static_cast<int>(kLayoutSmemLimit / 8) - 16;
+// Sections of a frame at most (25,000: 1.6 gigapixels).
+constexpr int kMaxSections = 25584;
 
 // Builds the constant header blobs and section table for a geometry. Fills the
 // host-side vectors; the caller uploads them.
 struct EntropyHostPlan {
     std::vector<Section> sections;
     std::vector<Stripe> stripes;
+    std::uint32_t misc_units{0};
+    std::vector<std::uint32_t> unit_section;
+    std::uint32_t head_words[4]{};
+    std::uint32_t head_bytes{0};
     std::uint32_t total_items{0};
     std::uint32_t ac_first{0};
     std::vector<std::uint8_t> pre_const;
@@ -179,12 +190,9 @@ bool entropy_launch(const EntropyDev& e, void* stream);
 // begin[phase][f + 1] - 1. The frames live in the launch's parameter block.
 constexpr int kEntropyBatchFrames = 64;
 enum EntropyPhase : int {
-    kPhaseItems = 0,    // item passes: one block per AC stripe, then one per 512 other items
-    kPhaseCodes = 1,    // prefix codes: one block per histogram
-    kPhaseScan = 2,     // item scan tiles
-    kPhaseFrame = 3,    // one block per frame
-    kPhaseZero = 4,     // body zeroing
-    kEntropyPhases = 5
+    kPhaseItems = 0,  // item passes: one block per AC stripe, then one per 512 other items
+    kPhaseCodes = 1,  // prefix codes: one block per histogram
+    kEntropyPhases = 2
 };
 struct EntropyBatch {
     int nframes;
@@ -197,6 +205,9 @@ void entropy_batch_plan(EntropyBatch& b);
 
 // Enqueues every frame's entropy stage on `stream` (b planned).
 bool entropy_batch_launch(const EntropyBatch& b, void* stream);
+
+// Entries of unit_sum and unit_off: the units and one more, in whole vectors of four.
+inline std::size_t unit_words(const EntropyHostPlan& p) { return (p.unit_section.size() + 4) & ~std::size_t{3}; }
 
 // The device prefix-code builder on one histogram of `length` (1..256)
 // symbols, synchronously on the current device (test hook): depths, codes and

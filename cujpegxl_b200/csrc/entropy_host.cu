@@ -190,7 +190,7 @@ EntropyHostPlan entropy_plan(int width, int height) {
     const int xdg{(bw + 255) / 256};
     const int ydg{(bh + 255) / 256};
     std::uint32_t at{0};
-    p.sections.push_back({at, 1, kSecDcGlobal, 0});
+    p.sections.push_back({at, 1, kSecDcGlobal, 0, 0});
     at += 1;
     for (int g{0}; g < xdg * ydg; ++g) {
         const int gw{std::min(256, bw - (g % xdg) * 256)};
@@ -198,26 +198,73 @@ EntropyHostPlan entropy_plan(int width, int height) {
         const std::uint32_t n{static_cast<std::uint32_t>(gw * gh)};
         const std::uint32_t cwch{static_cast<std::uint32_t>(((gw + 7) / 8) * ((gh + 7) / 8))};
         const std::uint32_t cnt{5 + 6 * n + 2 * cwch};
-        p.sections.push_back({at, cnt, kSecDcGroup, g});
+        p.sections.push_back({at, cnt, kSecDcGroup, g, at / kMiscItemsPerUnit});
         at += cnt;
     }
-    p.sections.push_back({at, 65, kSecAcGlobal, 0});
+    p.sections.push_back({at, 65, kSecAcGlobal, 0, at / kMiscItemsPerUnit});
     at += 65;
     p.ac_first = at;
+    for (std::uint32_t first{0}, sec{0}; first < p.ac_first; first += kMiscItemsPerUnit) {
+        while (first >= p.sections[sec].first + p.sections[sec].count) ++sec;
+        p.unit_section.push_back(sec);
+        ++p.misc_units;
+    }
     for (int g{0}; g < xg * yg; ++g) {
         const int gw{std::min(32, bw - (g % xg) * 32)};
         const int gh{std::min(32, bh - (g / xg) * 32)};
         const std::uint32_t cnt{static_cast<std::uint32_t>(3 * gw * gh)};
         const int sec{static_cast<int>(p.sections.size())};
+        const std::uint32_t unit{static_cast<std::uint32_t>(p.unit_section.size())};
         for (int r0{0}; r0 < gh; r0 += kStripeRows) {
             const int rows{std::min(kStripeRows, gh - r0)};
             p.stripes.push_back({at + static_cast<std::uint32_t>(3 * gw * r0), sec, static_cast<std::uint16_t>(g),
-                                 static_cast<std::uint8_t>(r0), static_cast<std::uint8_t>(rows)});
+                                 static_cast<std::uint8_t>(r0), static_cast<std::uint8_t>(rows),
+                                 static_cast<std::uint32_t>(gw)});
+            p.unit_section.push_back(static_cast<std::uint32_t>(sec));
         }
-        p.sections.push_back({at, cnt, kSecAcGroup, g});
+        p.sections.push_back({at, cnt, kSecAcGroup, g, unit});
         at += cnt;
     }
     p.total_items = at;
+
+    {
+        // Codestream header (src/bitstream/codestream.cc:57-90): signature,
+        // SizeHeader, ImageMetadata and transform data all default.
+        HostBits hb;
+        BitSink& w{hb.w};
+        auto size = [&](std::uint32_t v) {
+            // U32(1 + u(9), 1 + u(13), 1 + u(18), 1 + u(30)), the shortest that holds v.
+            constexpr std::uint32_t kExtra[4]{9, 13, 18, 30};
+            std::uint32_t sel{0};
+            while (v - 1 >= (1u << kExtra[sel])) ++sel;
+            w.put(2, sel);
+            w.put(kExtra[sel], v - 1);
+        };
+        const std::uint32_t W{static_cast<std::uint32_t>(width)};
+        const std::uint32_t H{static_cast<std::uint32_t>(height)};
+        w.put(8, 0xFF);
+        w.put(8, 0x0A);
+        const bool small{W % 8 == 0 && H % 8 == 0 && W <= 256 && H <= 256};
+        w.put(1, small ? 1 : 0);
+        if (small) w.put(5, H / 8 - 1); else size(H);
+        w.put(3, 0);
+        if (small) w.put(5, W / 8 - 1); else size(W);
+        w.put(1, 1);
+        w.put(1, 1);
+        w.pos = (w.pos + 7) & ~7u;
+        // FrameHeader: regular VarDCT frame, upsampling 1, x/b qm scale 2, one
+        // pass, no custom size, replace blending, last, unnamed, default loop
+        // filter; then a TOC without permutation.
+        constexpr std::uint32_t kFrame[15][2]{{1, 0}, {2, 0}, {1, 0}, {2, 0}, {2, 0}, {3, 2}, {3, 2}, {2, 0},
+                                              {1, 0}, {2, 0}, {1, 1}, {2, 0}, {1, 1}, {2, 0}, {1, 0}};
+        for (const auto& f : kFrame) w.put(f[0], f[1]);
+        w.pos = (w.pos + 7) & ~7u;
+        p.head_bytes = w.pos / 8;
+        const std::vector<std::uint8_t> bytes{hb.bytes()};
+        for (std::size_t i{0}; i < p.head_bytes && i < bytes.size(); ++i) {
+            p.head_words[i / 4] |= static_cast<std::uint32_t>(bytes[i]) << (8 * (i % 4));
+        }
+    }
 
     {
         HostBits hb;

@@ -107,7 +107,7 @@ cujpegxl_status cujpegxl_b200_encode_planes_noalloc(const cujpegxl_b200_device_p
     const std::size_t nb{static_cast<std::size_t>(bw) * bh};
     const jxb::EntropyHostPlan plan{jxb::entropy_plan(W, H)};
     const int ndc{((bw + 255) / 256) * ((bh + 255) / 256)};
-    const std::uint32_t tiles{(plan.total_items + jxb::kScanTile - 1) / jxb::kScanTile};
+    const std::size_t units{plan.unit_section.size()};
     std::uint32_t dcg_bits{0};
     const std::vector<std::uint8_t> dcg{jxb::dc_global_bits(global_scale, quant_dc, &dcg_bits)};
 
@@ -126,9 +126,13 @@ cujpegxl_status cujpegxl_b200_encode_planes_noalloc(const cujpegxl_b200_device_p
     e.nsec = static_cast<int>(plan.sections.size());
     e.total_items = plan.total_items;
     e.ac_first = plan.ac_first;
-    e.num_tiles = tiles;
+    e.misc_units = plan.misc_units;
+    for (int i{0}; i < 4; ++i) e.head_words[i] = plan.head_words[i];
+    e.head_bytes = plan.head_bytes;
+    e.clear_first = true;  // the array last served another geometry
     auto* sections{c.take<jxb::Section>(plan.sections.size())};
     auto* stripes{c.take<jxb::Stripe>(plan.stripes.size())};
+    auto* unit_section{c.take<std::uint32_t>(units)};
     auto* order{c.take<std::uint16_t>(plan.order.size())};
     auto* pre{c.take<std::uint8_t>(plan.pre_const.size())};
     auto* mid{c.take<std::uint8_t>(plan.mid_const.size())};
@@ -140,8 +144,11 @@ cujpegxl_status cujpegxl_b200_encode_planes_noalloc(const cujpegxl_b200_device_p
     e.dc_hist = c.take<std::uint32_t>(static_cast<std::size_t>(ndc) * 256);
     e.am_hist = c.take<std::uint32_t>(static_cast<std::size_t>(ndc) * 256);
     e.fb_count = c.take<std::uint32_t>(static_cast<std::size_t>(ndc));
+    e.tok_count = c.take<std::uint32_t>(1);
+    e.frozen = c.take<std::uint32_t>(1 + static_cast<std::size_t>(ndc));
     e.ac_depth = c.take<std::uint8_t>(32 * 256);
     e.ac_bits = c.take<std::uint16_t>(32 * 256);
+    e.code = c.take<std::uint32_t>(32 * 64 + static_cast<std::size_t>(ndc) * 2 * 128);
     e.dc_depth = c.take<std::uint8_t>(static_cast<std::size_t>(ndc) * 256);
     e.dc_bits = c.take<std::uint16_t>(static_cast<std::size_t>(ndc) * 256);
     e.am_depth = c.take<std::uint8_t>(static_cast<std::size_t>(ndc) * 256);
@@ -149,13 +156,13 @@ cujpegxl_status cujpegxl_b200_encode_planes_noalloc(const cujpegxl_b200_device_p
     e.ac_alpha = c.take<std::uint32_t>(32);
     e.desc = c.take<std::uint8_t>(static_cast<std::size_t>(32 + 2 * ndc) * jxb::kDescBytes);
     e.desc_bits = c.take<std::uint32_t>(static_cast<std::size_t>(32 + 2 * ndc));
-    e.item_bits = c.take<std::uint32_t>(plan.total_items);
     e.item_pre = c.take<std::uint32_t>(plan.total_items);
-    e.tile_sum = c.take<std::uint32_t>(tiles);
-    e.tile_off = c.take<unsigned long long>(tiles + 1);
-    e.sec_pos = c.take<unsigned long long>(plan.sections.size());
+    e.item_tok = c.take<std::uint32_t>(plan.ac_first);
+    e.unit_sum = c.take<std::uint32_t>(jxb::unit_words(plan));
+    e.unit_off = c.take<unsigned long long>(jxb::unit_words(plan));
+    e.unit_pos = c.take<unsigned long long>(units);
+    e.sec_shift = c.take<unsigned long long>(plan.sections.size());
     e.result = c.take<unsigned long long>(4);
-    e.tok_count = c.take<std::uint32_t>(1);
     e.stripe_tok = c.take<std::uint32_t>(2 * plan.stripes.size());
     if (!c.ok) return CUJPEGXL_UNSUPPORTED_RESOLUTION;
     // The rest of the array holds AC tokens; stripes that find it full are
@@ -165,6 +172,7 @@ cujpegxl_status cujpegxl_b200_encode_planes_noalloc(const cujpegxl_b200_device_p
     e.tok_pool = reinterpret_cast<std::uint32_t*>(base + (tok_at < kScratchBytes ? tok_at : 0));
 
     e.sections = sections;
+    e.unit_section = unit_section;
     e.stripes = stripes;
     e.nstripes = static_cast<int>(plan.stripes.size());
     e.order = order;
@@ -195,6 +203,8 @@ cujpegxl_status cujpegxl_b200_encode_planes_noalloc(const cujpegxl_b200_device_p
                         cudaMemcpyHostToDevice, st) == cudaSuccess &&
         cudaMemcpyAsync(stripes, plan.stripes.data(), plan.stripes.size() * sizeof(jxb::Stripe),
                         cudaMemcpyHostToDevice, st) == cudaSuccess &&
+        cudaMemcpyAsync(unit_section, plan.unit_section.data(), units * 4, cudaMemcpyHostToDevice, st) ==
+            cudaSuccess &&
         cudaMemcpyAsync(order, plan.order.data(), plan.order.size() * 2, cudaMemcpyHostToDevice, st) == cudaSuccess &&
         cudaMemcpyAsync(pre, plan.pre_const.data(), plan.pre_const.size(), cudaMemcpyHostToDevice, st) == cudaSuccess &&
         cudaMemcpyAsync(mid, plan.mid_const.data(), plan.mid_const.size(), cudaMemcpyHostToDevice, st) == cudaSuccess &&
