@@ -74,6 +74,23 @@ __constant__ float2 c_dct8[32];
 __constant__ float2 c_dct16[128];
 __constant__ float2 c_dct32[512];
 
+// The selection bases folded for the bounded selection: element
+// (parity * N/4 + j) * N/2 + t holds {basis[k][t], basis[k + 2][t]} with
+// k = parity + 4j, for t < N/2 (basis[k][N-1-t] is +-basis[k][t] by parity, up
+// to the rounding that kFold of c_bound covers).
+// DCT8's are constants of its unrolled passes; DCT16's and DCT32's are read
+// from shared memory by passes rolled over the coefficient pairs (a third of
+// the code, which every launch fetches anew).
+__constant__ float2 c_fold8[16];
+// Error-bound coefficients of the bounded selection per size (bound_init).
+struct SelectBound {
+    float pixel;   // per unit of the largest centred pixel or row output
+    float column;  // per unit of the centre, for row frequency 0 in the column pass
+    float weight;  // largest reciprocal weight
+    float span;    // largest weight
+};
+__constant__ SelectBound c_bound[3];
+
 template <int N, bool kSel>
 __device__ __forceinline__ float2 basis2(int i) {
     if (kSel) {
@@ -84,13 +101,9 @@ __device__ __forceinline__ float2 basis2(int i) {
 
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
-// Rate-proxy table entries kept in shared memory: quantised magnitudes below
-// this are by far the most frequent.
-constexpr int kLog2Cached = 256;
-
 struct Small {
     float pre[256];       // AQ pre-erosion cells, 16x16 over the tile
-    float log2_small[kLog2Cached];  // log2f(1 + i), the first entries of the rate table
+    float2 fold[64 + 256];  // folded bases of the bounded selection: DCT16, DCT32 (fold_entry)
     float cost8[64];
     float cost16[16];
     float cost32[4];
@@ -104,6 +117,14 @@ struct Small {
     signed char acs[64];
     int n32, n16, n8;
     signed char net[4];   // learned split class of each 32x32 region, -1 = RD heuristic
+    // The bounded selection's costs and how far each can be from the exact
+    // one, the two halves of each DCT32 apart; the largest centred pixel of
+    // each region; and whether the bounds left the region undecided.
+    float2 near8[64];
+    float2 near16[16];
+    float2 near32[4][2];
+    float spread[4];
+    unsigned char undecided[4];
     float2 pow_lut[6];    // factor table of jx_pow24_2, for the packed sRGB transfer
 };
 
@@ -311,23 +332,21 @@ __device__ __forceinline__ void row_pass(const float* src, float* dst) {
 // (block_ac_cost, src/transform_select_impl.cuh:80-106). Kept out of line:
 // the unrolled column passes call it from hundreds of sites, and one shared
 // body keeps their code small enough for the instruction caches.
-__device__ __noinline__ float2 sel_cost_nonzero(float coeff, float scaled, float w, float qgsf, const float* l2t,
-                                                const float* l2s) {
+__device__ __noinline__ float2 sel_cost_nonzero(float coeff, float scaled, float w, float qgsf, const float* l2t) {
     const float q{rintf(scaled / w)};
     const float err{(q * w) / qgsf - coeff};
     float rt{0.0f};
     if (q != 0.0f) {
         int a{static_cast<int>(fabsf(q))};
         a = a < kLog2TableSize ? a : kLog2TableSize - 1;
-        rt = 1.0f + (a < kLog2Cached ? l2s[a] : l2t[a]);
+        rt = 1.0f + l2t[a];
     }
     return make_float2(err * err, rt);
 }
 
 template <int N, int Y0, int Y1>
 __device__ __forceinline__ void sel_col(const float* rows_fx, float* cd_fx, float* cr_fx, int fx,
-                                        float qgsf, const float* wsel, const float* l2t,
-                                        const float* l2s) {
+                                        float qgsf, const float* wsel, const float* l2t) {
     static_assert(Y0 % 2 == 0 && Y1 % 2 == 0, "pairs of frequencies");
     float2 rr[N];
 #pragma unroll
@@ -362,7 +381,7 @@ __device__ __forceinline__ void sel_col(const float* rows_fx, float* cd_fx, floa
                     // rate.
                     d = h == 0 ? sq2.x : sq2.y;
                 } else {
-                    const float2 dr{sel_cost_nonzero(coeff, scaled, w, qgsf, l2t, l2s)};
+                    const float2 dr{sel_cost_nonzero(coeff, scaled, w, qgsf, l2t)};
                     d = dr.x;
                     rt = dr.y;
                 }
@@ -412,6 +431,193 @@ __device__ __forceinline__ void dct_col(const float* rows_fx, __half* coef, int 
         const int lb{(fby + q / side) * 8 + fbx + q % side};
         *reinterpret_cast<__half2*>(coef + lb * kCoefBlock + (raw & 63)) = __floats2half2_rn(c2.x, c2.y);
     }
+}
+
+// ---- Bounded transform selection ---------------------------------------------
+//
+// The RD decisions compare sums of costs, and a comparison whose two sides
+// differ by more than their possible errors comes out the same however the
+// sums were formed. So the costs are first computed the cheap way (pixels less
+// a centre value, even/odd folded DCT passes with FMA, quantisation by
+// reciprocal weights, hardware log2, sums in any order), each with a bound on
+// its distance from the host twin's float cost; a region whose decisions the
+// bounds settle is done, and the others go through the exact passes.
+//
+// The bound. All in units scaled by qgsf; u = 2^-24; m the centre, D the
+// largest |pixel - m| of the region. A chain of products and sums without FMA
+// is off by at most u times the sum of its products' and partial sums'
+// magnitudes. With pixel = m + d the partial sums of row frequency k are at
+// most |m| P_k(c) + D B_k(c), P_k(c) = |sum_{t<=c} b_k[t]|, B_k(c) =
+// sum_{t<=c} |b_k[t]|: hence FrontendTables::sel_centre (B_k + sum_c P_k(c)
+// per frequency) and SelectBound::pixel (the largest B_k + sum_c B_k(c) for
+// the host twin's chain, N/4 + 4 for the folded one in two accumulators, and
+// the basis's asymmetry). Row frequency 0 keeps the centre in its outputs,
+// which its column pass sees again (::column, the largest sel_centre of
+// k >= 1). With R the largest row output of a column (less the centre), every
+// coefficient is within
+//   delta = sel_centre m + pixel (D + R) [+ column m for row frequency 0]
+// and, quantised, within theta = delta + 10 u R of the host twin's (its
+// scaling, division and product round once each). |t| closer than theta / w to
+// a half-integer may then round the other way, which moves the rate by at most
+// 2 (0 <-> 1; less above) and the error term, near half a weight w, by at most
+// 2 theta; every other error term is off by at most theta, so the distortion
+// sum by at most 2 theta sqrt(n D2) + n theta^2 (Cauchy-Schwarz; D2 the sum of
+// n squares) and, per close call, theta w + 3 theta^2. Sums of non-negative
+// terms and the logarithms are covered by a relative 2e-5.
+
+__device__ __forceinline__ float log2_hw(float v) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));  // every v here is at least 1
+    return r;
+}
+
+// Two coefficients' sums over the N/2 folded samples, in two chains; `fold`
+// their basis entries in shared memory (DCT16, DCT32).
+template <int N>
+__device__ __forceinline__ float2 fold_dot(const float2* fold, const float2 (&h)[N / 2]) {
+    float2 a{0.0f, 0.0f};
+    float2 b{0.0f, 0.0f};
+#pragma unroll
+    for (int t{0}; t < N / 2; t += 2) {
+        const float4 f{*reinterpret_cast<const float4*>(fold + t)};
+        a = __ffma2_rn(make_float2(f.x, f.y), h[t], a);
+        b = __ffma2_rn(make_float2(f.z, f.w), h[t + 1], b);
+    }
+    return __fadd2_rn(a, b);
+}
+__device__ __forceinline__ float2 fold_dot8(int at, const float2 (&h)[4]) {
+    float2 a{__fmul2_rn(c_fold8[at], h[0])};
+#pragma unroll
+    for (int t{1}; t < 4; ++t) a = __ffma2_rn(c_fold8[at + t], h[t], a);
+    return a;
+}
+
+// Row stride of the folded passes' scratch.
+template <int N>
+constexpr int kNearStride = N == 32 ? 36 : N + 1;
+
+// Folded row pass of parities [P0, P1): frequencies k of those parities of the
+// scaled centred row to dst[k * kNearStride]; the largest centred pixel.
+template <int N, int P0, int P1>
+__device__ __forceinline__ float near_row(const float* src, const float2* fold, float scale, float centre, float* dst) {
+    float2 x[N / 2];
+    float big{0.0f};
+#pragma unroll
+    for (int c{0}; c < N; c += 4) {
+        const float4 v{*reinterpret_cast<const float4*>(src + c)};
+        x[c / 2] = __ffma2_rn(make_float2(v.x, v.y), f2dup(scale), f2dup(-centre));
+        x[c / 2 + 1] = __ffma2_rn(make_float2(v.z, v.w), f2dup(scale), f2dup(-centre));
+    }
+    if (N == 32 && P0 == 0) {
+#pragma unroll
+        for (int c{0}; c < N / 2; ++c) big = fmaxf(big, fmaxf(fabsf(x[c].x), fabsf(x[c].y)));
+    }
+#pragma unroll
+    for (int par{P0}; par < P1; ++par) {
+        float2 h[N / 2];
+#pragma unroll
+        for (int t{0}; t < N / 2; t += 2) {
+            const float2 lo{x[t / 2]};
+            const float2 hi{make_float2(x[N / 2 - 1 - t / 2].y, x[N / 2 - 1 - t / 2].x)};
+            const float2 f{par == 0 ? __fadd2_rn(lo, hi) : __fadd2_rn(lo, f2neg(hi))};
+            h[t] = dup2(f.x);
+            h[t + 1] = dup2(f.y);
+        }
+#pragma unroll (N == 8 ? 2 : 1)
+        for (int j{0}; j < N / 4; ++j) {
+            const int at{(par * (N / 4) + j) * (N / 2)};
+            float2 a;
+            if constexpr (N == 8) {
+                a = fold_dot8(at, h);
+            } else {
+                a = fold_dot<N>(fold + at, h);
+            }
+            dst[(par + 4 * j) * kNearStride<N>] = a.x;
+            dst[(par + 4 * j + 2) * kNearStride<N>] = a.y;
+        }
+    }
+    return big;
+}
+
+// Folded column pass of parities [P0, P1) of row frequency fx, quantised and
+// costed; returns {cost, bound} of these coefficients. Weights of frequencies
+// (k, k + 2) as {1/w, 1/w', w, w'}, zero for the low-frequency corner.
+template <int N, int P0, int P1>
+__device__ __forceinline__ float2 near_col(const float* rows_fx, const float2* fold, int fx, const float4* weights,
+                                           const float* centre_bound, float centre, float spread, float inv_scale2) {
+    constexpr int kSize{N == 8 ? 0 : (N == 16 ? 1 : 2)};
+    constexpr float kU{5.9604645e-8f};
+    constexpr float kMagic{12582912.0f};  // 1.5 * 2^23: adding it rounds to integers
+    float x[N];
+    float big{0.0f};
+    if constexpr (N == 32) {
+#pragma unroll
+        for (int r{0}; r < N; r += 4) {  // 16-byte aligned (kNearStride)
+            const float4 v{*reinterpret_cast<const float4*>(rows_fx + r)};
+            x[r] = v.x;
+            x[r + 1] = v.y;
+            x[r + 2] = v.z;
+            x[r + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int r{0}; r < N; ++r) x[r] = rows_fx[r];
+    }
+#pragma unroll
+    for (int r{0}; r < N; ++r) big = fmaxf(big, fabsf(x[r]));
+    const SelectBound sb{c_bound[kSize]};
+    const float delta{(centre_bound[fx] + (fx == 0 ? sb.column : 0.0f)) * centre + sb.pixel * (spread + big)};
+    const float theta{delta + 10.0f * kU * big};
+    float2 dist{0.0f, 0.0f};
+    float rate{0.0f};
+    // A quantum beyond the rate table or the rounding trick: undecidable here.
+    // Neither is one whose error may reach a whole quantum.
+    float flips{big * sb.weight > 4.0e5f || theta * sb.weight > 0.25f ? 1.0e9f : 0.0f};
+#pragma unroll
+    for (int par{P0}; par < P1; ++par) {
+        float2 h[N / 2];
+#pragma unroll
+        for (int t{0}; t < N / 2; ++t) h[t] = dup2(par == 0 ? x[t] + x[N - 1 - t] : x[t] - x[N - 1 - t]);
+#pragma unroll (N == 8 ? 2 : 1)
+        for (int j{0}; j < N / 4; ++j) {
+            const int at{(par * (N / 4) + j) * (N / 2)};
+            float2 a;
+            if constexpr (N == 8) {
+                a = fold_dot8(at, h);
+            } else {
+                a = fold_dot<N>(fold + at, h);
+            }
+            const float4 w{weights[(par * (N / 4) + j) * N + fx]};
+            const float2 inv{w.x, w.y};
+            const float2 q{__fmul2_rn(a, inv)};
+            const float2 qi{__fadd2_rn(__fadd2_rn(q, f2dup(kMagic)), f2dup(-kMagic))};
+            const float2 e{__fadd2_rn(q, f2neg(qi))};
+            const float2 ew{__fmul2_rn(e, make_float2(w.z, w.w))};
+            dist = __ffma2_rn(ew, ew, dist);
+            const float2 edge{__ffma2_rn(f2dup(-theta), inv, f2dup(0.5f))};
+            flips += (fabsf(e.x) > edge.x ? 2.0f : 0.0f) + (fabsf(e.y) > edge.y ? 2.0f : 0.0f);
+            const float2 mag{fabsf(qi.x), fabsf(qi.y)};
+            if (mag.x + mag.y != 0.0f) {
+                rate += (fminf(mag.x, 1.0f) + log2_hw(1.0f + mag.x)) + (fminf(mag.y, 1.0f) + log2_hw(1.0f + mag.y));
+            }
+        }
+    }
+    constexpr float kN2{static_cast<float>(N * N)};
+    constexpr float kCount{static_cast<float>(N / 2 * (P1 - P0))};
+    const float d2{dist.x + dist.y};
+    const float off{theta * (2.0f * sqrtf(kCount * d2) + kCount * theta + flips * (theta + sb.span))};
+    const float cost{kN2 * inv_scale2 * d2 + kSelectLambda * rate};
+    return make_float2(cost, 1.01f * kN2 * inv_scale2 * off + kSelectLambda * flips + 2.0e-5f * cost);
+}
+
+// Sum of both components over groups of kLanes adjacent lanes.
+template <int kLanes>
+__device__ __forceinline__ float2 group_sum2(float2 v) {
+#pragma unroll
+    for (int off{1}; off < kLanes; off <<= 1) {
+        v = __fadd2_rn(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.y, off)));
+    }
+    return v;
 }
 
 // One CfL sum of a side-N first block lb over its non-LLF coefficients
@@ -538,11 +744,11 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     {
         const int cw{W >> 1};
         const int ch{H >> 1};
-        // The rate-table entry and the learned class are loaded here and
-        // stored after the window, so that their latency overlaps the
-        // window's.
-        static_assert(kLog2Cached == kThreads, "one cached rate-table entry per thread");
-        const float log2_entry{tb.log2_1p[tid]};
+        // The folded bases and the learned class are loaded here and stored
+        // after the window, so that their latency overlaps the window's.
+        static_assert(64 + 256 <= 2 * kThreads, "two basis entries per thread");
+        const float2 fold_a{tb.fold[tid]};
+        const float2 fold_b{tid < 64 ? tb.fold[kThreads + tid] : make_float2(0.0f, 0.0f)};
         signed char net_entry{-1};
         if (tid < 4) {
             const int rw{(bw + 3) >> 2};
@@ -640,7 +846,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 }
             }
         }
-        sm.log2_small[tid] = log2_entry;
+        sm.fold[tid] = fold_a;
+        if (tid < 64) sm.fold[kThreads + tid] = fold_b;
         if (tid < 4) sm.net[tid] = net_entry;
 #pragma unroll
         for (int k{0}; k < 6; ++k) {
@@ -877,20 +1084,201 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     float* crate{smem + 9216};     // per-coefficient rate contributions
     const float qg{sc.qgsf_select};
     // Regions inside the image that the network did not decide need the RD
-    // costs; when there are none the cost passes are skipped altogether.
+    // costs: first the bounded ones (not when the exact costs are dumped).
     unsigned inimg{0};
 #pragma unroll
     for (int ri{0}; ri < 4; ++ri) {
         inimg |= (bx0 + 4 * (ri & 1) < bw && by0 + 4 * (ri >> 1) < bh ? 1u : 0u) << ri;
     }
-    if ((inimg & ~dmask) != 0u) {
+    // Warps 4-7 clear the non-zero counters and CfL sums and finish
+    // each block's quant field from its AQ sums.
+    if (tid >= 128) {
+        for (int i{tid - 128}; i < 192; i += 128) {
+            sm.nz[i >> 6][i & 63] = 0;
+            sm.cfl[i >> 6][i & 63] = 0.0f;  // blocks that are not first blocks add zero
+        }
+    }
+    if (tid >= 128 && tid < 192) {
+        // Quant field of block lb from its AQ sums (src/frontend_fused.cu:177-201).
+        const int lb{tid - 128};
+        if (((qmask >> region_of_block(lb)) & 1u) != 0) {
+            sm.qf[lb] = in.net_qf[static_cast<std::size_t>(by0 + (lb >> 3)) * bw + bx0 + (lb & 7)];
+        } else if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh) {
+            const float hf_sum{sm.aq_sums[0][lb]};
+            const float gamma_overall{sm.aq_sums[1][lb] * (0.5f / 64.0f)};
+            float blue_sum{sm.aq_sums[2][lb]};
+            const float aq{sm.aq_sums[3][lb]};
+            if (blue_sum >= 32.0f * kBlueLimit) {
+                blue_sum = 64.0f * kBlueLimit - blue_sum;
+            }
+            if (blue_sum >= kBlueMaxLimit * kBlueLimit) {
+                blue_sum = kBlueMaxLimit * kBlueLimit;
+            }
+            float ov{compute_mask(aq)};
+            ov = ov + jx_fma(hf_sum, kHfMul, kHfAdd);
+            ov = jx_fma(kGammaLogMul, jx_log2(gamma_overall), ov);
+            ov = jx_fma(blue_sum, kBlueMul, ov);
+            const float qval{jx_fma(jx_exp(ov), sc.mul_pb, sc.add_pb)};
+            int qi{static_cast<int>(jx_fma(qval, sc.inv_global_scale, 0.5f))};
+            qi = qi < 1 ? 1 : (qi > kQuantMax ? kQuantMax : qi);
+            sm.qf[lb] = qi;
+        }
+    }
+    unsigned exact{inimg & ~dmask};  // regions for the exact passes
+    if (exact != 0u && out.dbg_cost == nullptr) {
+        // Row passes of all three sizes, then their column passes, two phases
+        // in all: every item is independent, and costs are summed in registers
+        // and across lanes. (The exact passes take nine phases, with every
+        // coefficient's two cost terms through shared memory.) Bound by issue
+        // and latency as the rest of the tile; at 4K the selection of a pair
+        // of tiles went from 37.7K cycles to 19K (rows 5.5K, columns 13K,
+        // decisions 0.7K), and about 1% of the regions, at distance 1 on the
+        // synthetic frame, go on to the exact passes (25K for a pair of tiles
+        // that has one); the launch went from 0.40 to 0.34 ms.
+        constexpr int kRows16{4608};
+        constexpr int kRows32{kRows16 + 16 * 272};
+        static_assert(kRows32 % 4 == 0 && kRows32 + 4 * 32 * kNearStride<32> <= kRegionAFloats, "row scratch of the bounded selection");
+        auto centre_of = [&](int ri) { return SY[((ri >> 1) * 32 + 16) * kSs + (ri & 1) * 32 + 16] * qg; };
+#pragma unroll
+        for (int h{0}; h < 2; ++h) {
+            const int k{tid + h * kThreads};
+            const int lb{k >> 3};
+            const int r{k & 7};
+            if (((exact >> region_of_block(lb)) & 1u) != 0) {
+                near_row<8, 0, 2>(SY + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, nullptr, qg, centre_of(region_of_block(lb)),
+                                  rows + lb * 72 + r);
+            }
+        }
+        {
+            const int qd{tid >> 4};
+            const int r{tid & 15};
+            const int ri{((qd >> 3) << 1) | ((qd & 3) >> 1)};
+            if (((exact >> ri) & 1u) != 0) {
+                near_row<16, 0, 2>(SY + ((qd >> 2) * 16 + r) * kSs + (qd & 3) * 16, sm.fold, qg, centre_of(ri),
+                                   rows + kRows16 + qd * 272 + r);
+            }
+        }
+        {
+            // A warp per region and parity.
+            const int ri{tid >> 6};
+            const int r{tid & 31};
+            if (((exact >> ri) & 1u) != 0) {
+                const float* src{SY + ((ri >> 1) * 32 + r) * kSs + (ri & 1) * 32};
+                float* dst{rows + kRows32 + ri * 32 * kNearStride<32> + r};
+                if ((tid & 32) == 0) {
+                    const float big{near_row<32, 0, 1>(src, sm.fold + 64, qg, centre_of(ri), dst)};
+                    const unsigned most{__reduce_max_sync(0xffffffffu, __float_as_uint(big))};
+                    if (lane == 0) sm.spread[ri] = __uint_as_float(most);
+                } else {
+                    near_row<32, 1, 2>(src, sm.fold + 64, qg, centre_of(ri), dst);
+                }
+            }
+        }
+        tile_sync(bar);
+        const float inv_scale2{1.0f / (qg * qg)};
+        {
+            const int ri{tid >> 6};
+            const int fx{tid & 31};
+            if (((exact >> ri) & 1u) != 0) {
+                const float* src{rows + kRows32 + (ri * 32 + fx) * kNearStride<32>};
+                const float c{fabsf(centre_of(ri))};
+                const float2 v{group_sum2<32>(
+                    (tid & 32) == 0 ? near_col<32, 0, 1>(src, sm.fold + 64, fx, tb.sel_pairs + 160, tb.sel_centre + 24, c,
+                                                         sm.spread[ri], inv_scale2)
+                                    : near_col<32, 1, 2>(src, sm.fold + 64, fx, tb.sel_pairs + 160, tb.sel_centre + 24, c,
+                                                         sm.spread[ri], inv_scale2))};
+                if (lane == 0) sm.near32[ri][(tid >> 5) & 1] = v;
+            }
+        }
+        {
+            const int qd{tid >> 4};
+            const int fx{tid & 15};
+            const int ri{((qd >> 3) << 1) | ((qd & 3) >> 1)};
+            const bool on{((exact >> ri) & 1u) != 0};
+            float2 v{0.0f, 0.0f};
+            if (on) {
+                v = near_col<16, 0, 2>(rows + kRows16 + qd * 272 + fx * 17, sm.fold, fx, tb.sel_pairs + 32, tb.sel_centre + 8,
+                                       fabsf(centre_of(ri)), sm.spread[ri], inv_scale2);
+            }
+            v = group_sum2<16>(v);
+            if (on && fx == 0) sm.near16[qd] = v;
+        }
+#pragma unroll
+        for (int h{0}; h < 2; ++h) {
+            const int k{tid + h * kThreads};
+            const int lb{k >> 3};
+            const int fx{k & 7};
+            const int ri{region_of_block(lb)};
+            const bool on{((exact >> ri) & 1u) != 0};
+            float2 v{0.0f, 0.0f};
+            if (on) {
+                v = near_col<8, 0, 2>(rows + lb * 72 + fx * 9, nullptr, fx, tb.sel_pairs, tb.sel_centre, fabsf(centre_of(ri)), sm.spread[ri],
+                                      inv_scale2);
+            }
+            v = group_sum2<8>(v);
+            if (on && fx == 0) sm.near8[lb] = v;
+        }
+        tile_sync(bar);
+        // Decisions, a warp per region and a lane per block, four lanes to a
+        // quad: the comparisons of 4d on [cost - bound, cost + bound].
+        if (warp < 4) {
+            const int ri{warp};
+            const int quad{(lane >> 2) & 3};
+            const int dx{(quad & 1) * 2 + (lane & 1)};
+            const int dy{(quad >> 1) * 2 + ((lane >> 1) & 1)};
+            const int lbx{(ri & 1) * 4 + dx};
+            const int lby{(ri >> 1) * 4 + dy};
+            const bool inside{bx0 + lbx < bw && by0 + lby < bh};
+            const int qx{bx0 + (lbx & ~1)};
+            const int qy{by0 + (lby & ~1)};
+            const bool quad_in{qx < bw && qy < bh};
+            const bool fit16{qx + 2 <= bw && qy + 2 <= bh};
+            const int rx{bx0 + (ri & 1) * 4};
+            const int ry{by0 + (ri >> 1) * 4};
+            const bool fit32{rx + 4 <= bw && ry + 4 <= bh};
+            const float2 sum8{group_sum2<4>(inside ? sm.near8[lby * 8 + lbx] : make_float2(0.0f, 0.0f))};
+            const float2 c16{sm.near16[(lby >> 1) * 4 + (lbx >> 1)]};
+            const float gap{c16.x - (sum8.x + kSelectSplitEps)};
+            const float room{c16.y + sum8.y + 1.0e-9f};
+            const bool take16{fit16 && gap <= -room};
+            const bool unsure{quad_in && fit16 && !take16 && !(gap > room)};
+            // The split's cost between lo and hi, whichever way an unsure quad goes.
+            float2 lohi{0.0f, 0.0f};
+            if (quad_in) {
+                const float2 r16{c16.x - c16.y, c16.x + c16.y};
+                const float2 r8{sum8.x - sum8.y, sum8.x + sum8.y};
+                lohi = unsure ? make_float2(fminf(r16.x, r8.x), fmaxf(r16.y, r8.y)) : (take16 ? r16 : r8);
+            }
+            lohi = __fadd2_rn(lohi, make_float2(__shfl_xor_sync(0xffffffffu, lohi.x, 4),
+                                                __shfl_xor_sync(0xffffffffu, lohi.y, 4)));
+            lohi = __fadd2_rn(lohi, make_float2(__shfl_xor_sync(0xffffffffu, lohi.x, 8),
+                                                __shfl_xor_sync(0xffffffffu, lohi.y, 8)));
+            const float2 c32{__fadd2_rn(sm.near32[ri][0], sm.near32[ri][1])};
+            const bool any_unsure{__any_sync(0xffffffffu, unsure) != 0};
+            const bool take32{fit32 && c32.x + c32.y + 1.0e-9f <= lohi.x + kSelectSplitEps};
+            const bool split{!any_unsure && (!fit32 || c32.x - c32.y > lohi.y + kSelectSplitEps + 1.0e-9f)};
+            if (((exact >> ri) & 1u) != 0) {
+                if (lane < 16 && inside && (take32 || split)) {
+                    sm.acs[lby * 8 + lbx] = static_cast<signed char>(
+                        take32 ? (lane == 0 ? 32 : 0) : (take16 ? ((lane & 3) == 0 ? 16 : 0) : 8));
+                }
+                if (lane == 0) sm.undecided[ri] = take32 || split ? 0 : 1;
+            }
+        }
+        tile_sync(bar);
+        unsigned left{0};
+#pragma unroll
+        for (int ri{0}; ri < 4; ++ri) left |= (((exact >> ri) & 1u) != 0 && sm.undecided[ri] != 0 ? 1u : 0u) << ri;
+        exact = left;
+    }
+    if (exact != 0u) {
         // 4a. DCT8 candidates: one per block inside the image.
         for (int k{tid}; k < 512; k += kThreads) {
             const int lb{k >> 3};
             const int r{k & 7};
             const int lbx{lb & 7};
             const int lby{lb >> 3};
-            if (bx0 + lbx < bw && by0 + lby < bh && ((dmask >> region_of_block(lb)) & 1u) == 0) {
+            if (bx0 + lbx < bw && by0 + lby < bh && ((exact >> region_of_block(lb)) & 1u) != 0) {
                 row_pass<8, 0, 8, true>(SY + (lby * 8 + r) * kSs + lbx * 8, rows + lb * 72 + r);
             }
         }
@@ -899,9 +1287,9 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int lb{k >> 3};
             const int fx{k & 7};
             if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh &&
-                ((dmask >> region_of_block(lb)) & 1u) == 0) {
+                ((exact >> region_of_block(lb)) & 1u) != 0) {
                 sel_col<8, 0, 8>(rows + lb * 72 + fx * 9, cdist + lb * 72 + fx * 9,
-                                 crate + lb * 72 + fx * 9, fx, qg, tb.sel_weight, tb.log2_1p, sm.log2_small);
+                                 crate + lb * 72 + fx * 9, fx, qg, tb.sel_weight, tb.log2_1p);
             }
         }
         tile_sync(bar);
@@ -909,7 +1297,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
 #pragma unroll 2
         for (int lb{warp}; lb < 64; lb += kThreads / 32) {
             if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh &&
-                ((dmask >> region_of_block(lb)) & 1u) == 0) {
+                ((exact >> region_of_block(lb)) & 1u) != 0) {
                 const int i0{lb * 72 + (lane >> 3) * 9 + (lane & 7)};
                 const int i1{lb * 72 + ((lane + 32) >> 3) * 9 + (lane & 7)};
                 const float2 DR{warp_tree2(
@@ -928,7 +1316,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int qx{qd & 3};
             const int qy{qd >> 2};
             if (bx0 + 2 * qx + 2 <= bw && by0 + 2 * qy + 2 <= bh &&
-                ((dmask >> (((qy >> 1) << 1) | (qx >> 1))) & 1u) == 0) {
+                ((exact >> (((qy >> 1) << 1) | (qx >> 1))) & 1u) != 0) {
                 row_pass<16, 0, 16, true>(SY + (qy * 16 + r) * kSs + qx * 16, rows + qd * 272 + r);
             }
         }
@@ -937,16 +1325,16 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int qd{k >> 4};
             const int fx{k & 15};
             if (bx0 + 2 * (qd & 3) + 2 <= bw && by0 + 2 * (qd >> 2) + 2 <= bh &&
-                ((dmask >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) == 0) {
+                ((exact >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) != 0) {
                 sel_col<16, 0, 16>(rows + qd * 272 + fx * 17, cdist + qd * 272 + fx * 17,
                                    crate + qd * 272 + fx * 17, fx, qg, tb.sel_weight + 1024,
-                                   tb.log2_1p, sm.log2_small);
+                                   tb.log2_1p);
             }
         }
         tile_sync(bar);
         for (int qd{warp}; qd < 16; qd += kThreads / 32) {
             if (bx0 + 2 * (qd & 3) + 2 <= bw && by0 + 2 * (qd >> 2) + 2 <= bh &&
-                ((dmask >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) == 0) {
+                ((exact >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) != 0) {
                 // Distortion (x) and rate (y) as packed pairs, each in the
                 // host twin's order.
                 float2 p[8];
@@ -975,7 +1363,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const bool hi{(k & 32) != 0};
             const int rx{ri & 1};
             const int ry{ri >> 1};
-            if (bx0 + 4 * rx + 4 <= bw && by0 + 4 * ry + 4 <= bh && ((dmask >> ri) & 1u) == 0) {
+            if (bx0 + 4 * rx + 4 <= bw && by0 + 4 * ry + 4 <= bh && ((exact >> ri) & 1u) != 0) {
                 const float* src{SY + (ry * 32 + r) * kSs + rx * 32};
                 float* dst{rows + ri * 1056 + r};
                 if (hi) {
@@ -991,14 +1379,14 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int fx{k & 31};
             const bool hi{(k & 32) != 0};
             if (bx0 + 4 * (ri & 1) + 4 <= bw && by0 + 4 * (ri >> 1) + 4 <= bh &&
-                ((dmask >> ri) & 1u) == 0) {
+                ((exact >> ri) & 1u) != 0) {
                 const float* src{rows + ri * 1056 + fx * 33};
                 float* cd{cdist + ri * 1056 + fx * 33};
                 float* cr{crate + ri * 1056 + fx * 33};
                 if (hi) {
-                    sel_col<32, 16, 32>(src, cd, cr, fx, qg, tb.sel_weight + 2048, tb.log2_1p, sm.log2_small);
+                    sel_col<32, 16, 32>(src, cd, cr, fx, qg, tb.sel_weight + 2048, tb.log2_1p);
                 } else {
-                    sel_col<32, 0, 16>(src, cd, cr, fx, qg, tb.sel_weight + 2048, tb.log2_1p, sm.log2_small);
+                    sel_col<32, 0, 16>(src, cd, cr, fx, qg, tb.sel_weight + 2048, tb.log2_1p);
                 }
             }
         }
@@ -1006,7 +1394,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
         if (warp < 4) {
             const int ri{warp};
             if (bx0 + 4 * (ri & 1) + 4 <= bw && by0 + 4 * (ri >> 1) + 4 <= bh &&
-                ((dmask >> ri) & 1u) == 0) {
+                ((exact >> ri) & 1u) != 0) {
                 // Distortion (x) and rate (y) as packed pairs, each in the
                 // host twin's order.
                 float2 p[8];
@@ -1032,6 +1420,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
         }
     }
+    // Decided regions of the network and of the exact passes.
+    if ((dmask | exact) != 0u) {
     // 4d. RD decision per region (src/transform_select_impl.cuh:130-201), by
     // lane 0 of warp ri, which wrote cost32[ri] itself (the DCT8 and DCT16
     // costs are older than the last barrier).
@@ -1060,7 +1450,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                     sm.acs[(rly + dy) * 8 + rlx + dx] = a;
                 }
             }
-        } else if (rbx < bw && rby < bh) {
+        } else if (((exact >> ri) & 1u) != 0) {
             constexpr float kInf{1.0e30f};
             const bool fit32{rbx + 4 <= bw && rby + 4 <= bh};
             const float c32{fit32 ? sm.cost32[ri] : kInf};
@@ -1123,41 +1513,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
         }
     }
-    // Warps 4-7 meanwhile clear the non-zero counters and CfL sums and finish
-    // each block's quant field from its AQ sums.
-    if (tid >= 128) {
-        for (int i{tid - 128}; i < 192; i += 128) {
-            sm.nz[i >> 6][i & 63] = 0;
-            sm.cfl[i >> 6][i & 63] = 0.0f;  // blocks that are not first blocks add zero
-        }
+        tile_sync(bar);
     }
-    if (tid >= 128 && tid < 192) {
-        // Quant field of block lb from its AQ sums (src/frontend_fused.cu:177-201).
-        const int lb{tid - 128};
-        if (((qmask >> region_of_block(lb)) & 1u) != 0) {
-            sm.qf[lb] = in.net_qf[static_cast<std::size_t>(by0 + (lb >> 3)) * bw + bx0 + (lb & 7)];
-        } else if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh) {
-            const float hf_sum{sm.aq_sums[0][lb]};
-            const float gamma_overall{sm.aq_sums[1][lb] * (0.5f / 64.0f)};
-            float blue_sum{sm.aq_sums[2][lb]};
-            const float aq{sm.aq_sums[3][lb]};
-            if (blue_sum >= 32.0f * kBlueLimit) {
-                blue_sum = 64.0f * kBlueLimit - blue_sum;
-            }
-            if (blue_sum >= kBlueMaxLimit * kBlueLimit) {
-                blue_sum = kBlueMaxLimit * kBlueLimit;
-            }
-            float ov{compute_mask(aq)};
-            ov = ov + jx_fma(hf_sum, kHfMul, kHfAdd);
-            ov = jx_fma(kGammaLogMul, jx_log2(gamma_overall), ov);
-            ov = jx_fma(blue_sum, kBlueMul, ov);
-            const float qval{jx_fma(jx_exp(ov), sc.mul_pb, sc.add_pb)};
-            int qi{static_cast<int>(jx_fma(qval, sc.inv_global_scale, 0.5f))};
-            qi = qi < 1 ? 1 : (qi > kQuantMax ? kQuantMax : qi);
-            sm.qf[lb] = qi;
-        }
-    }
-    tile_sync(bar);
     if (out.dbg_cost != nullptr) {
         for (int lb{tid}; lb < 64; lb += kThreads) {
             const int lbx{lb & 7};
@@ -1635,6 +1992,13 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
 }  // namespace
 
+// Entry [k][t] of the selection basis: the double-precision DCT-II basis
+// narrowed to float.
+static float selection_basis(int n, int k, int t) {
+    const double g{k == 0 ? 1.0 / n : 1.4142135623730950488 / n};
+    return static_cast<float>(g * std::cos(3.14159265358979323846 * (t + 0.5) * k / n));
+}
+
 FrontendScalars frontend_scalars(float distance, std::uint32_t* global_scale,
                                  std::uint32_t* quant_dc) {
     // Quantiser calibration (src/quant_calibration.h:49-88).
@@ -1692,6 +2056,60 @@ FrontendScalars frontend_scalars(float distance, std::uint32_t* global_scale,
     return s;
 }
 
+namespace {
+
+// Folded selection bases and the error-bound coefficients of the bounded
+// selection, from the bases the exact passes use. sw: the selection weights;
+// centre_bound: FrontendTables::sel_centre; folds: FrontendTables::fold.
+bool bound_init(const std::vector<float>& sw, float* centre_bound, std::vector<float>* folds) {
+    constexpr double kU{1.0 / 16777216.0};
+    SelectBound bounds[3]{};
+    for (int n : {8, 16, 32}) {
+        const int si{n == 8 ? 0 : (n == 16 ? 1 : 2)};
+        std::vector<float> fold(static_cast<std::size_t>(n) * n / 2);
+        double pixel{0.0}, column{0.0}, skew{0.0};
+        for (int k{0}; k < n; ++k) {
+            double part{0.0}, mag{0.0}, parts{0.0}, mags{0.0}, asym{0.0};
+            for (int t{0}; t < n; ++t) {
+                const double b{selection_basis(n, k, t)};
+                const double mirror{selection_basis(n, k, n - 1 - t) * ((k & 1) != 0 ? -1.0 : 1.0)};
+                part += b;
+                mag += std::fabs(b);
+                parts += std::fabs(part);
+                mags += mag;
+                asym += std::fabs(b - mirror);
+                if (t < n / 2) {
+                    const int p{(k & 1) * (n / 4) + k / 4};
+                    fold[2 * (p * (n / 2) + t) + ((k >> 1) & 1)] = static_cast<float>(b);
+                }
+            }
+            // Each basis row's magnitudes sum to at most 1 (so a pass hands on
+            // the errors of the one before), and a centre outside frequency
+            // 0 leaves what the row's rounded entries sum to; the margin
+            // covers second-order terms.
+            const double bound{1.02 * (kU * (mag + parts) + (k > 0 ? 2.0 * std::fabs(part) : 0.0))};
+            centre_bound[n - 8 + k] = static_cast<float>(bound);
+            if (k > 0) column = std::max(column, bound);
+            pixel = std::max(pixel, mag + mags + n / 4 + 4);
+            skew = std::max(skew, asym);
+        }
+        bounds[si].pixel = static_cast<float>(1.02 * (kU * pixel + 2.0 * skew));
+        bounds[si].column = static_cast<float>(column);
+        for (int i{0}; i < n * n; ++i) {
+            bounds[si].weight = std::max(bounds[si].weight, 1.0f / sw[si * 1024 + i]);
+            bounds[si].span = std::max(bounds[si].span, sw[si * 1024 + i]);
+        }
+        if (n > 8) {
+            folds->insert(folds->end(), fold.begin(), fold.end());
+        } else if (cudaMemcpyToSymbol(c_fold8, fold.data(), fold.size() * sizeof(float)) != cudaSuccess) {
+            return false;
+        }
+    }
+    return cudaMemcpyToSymbol(c_bound, bounds, sizeof(bounds)) == cudaSuccess;
+}
+
+}  // namespace
+
 bool frontend_tables_init(FrontendTables* tables) {
     // Bases.
     for (int n : {8, 16, 32}) {
@@ -1699,11 +2117,10 @@ bool frontend_tables_init(FrontendTables* tables) {
         std::vector<float> sel(static_cast<std::size_t>(n) * n);
         std::vector<float> dct(static_cast<std::size_t>(n) * n);
         for (int k{0}; k < n; ++k) {
-            const double g{k == 0 ? 1.0 / n : 1.4142135623730950488 / n};
             const float gf{k == 0 ? 1.0f / n : 1.4142135623730951f / n};
             for (int t{0}; t < n; ++t) {
                 const int at{2 * ((k >> 1) * n + t) + (k & 1)};
-                sel[at] = static_cast<float>(g * std::cos(3.14159265358979323846 * (t + 0.5) * k / n));
+                sel[at] = selection_basis(n, k, t);
                 const float arg{3.14159265358979323846f * (t + 0.5f) * k / n};
                 dct[at] = gf * std::cos(arg);
             }
@@ -1740,6 +2157,29 @@ bool frontend_tables_init(FrontendTables* tables) {
             }
         }
     }
+    std::vector<float> centre(8 + 16 + 32);
+    std::vector<float> folds;
+    if (!bound_init(sw, centre.data(), &folds)) return false;
+    // Weight pairs of the bounded selection: {1/w, 1/w', w, w'} of
+    // frequencies (k, k + 2), k = parity + 4j, at [parity * N/4 + j][fx];
+    // zeros in the low-frequency corner.
+    std::vector<float> pairs(4 * (32 + 128 + 512), 0.0f);
+    for (int n : {8, 16, 32}) {
+        const int si{n == 8 ? 0 : (n == 16 ? 1 : 2)};
+        const int at{n == 8 ? 0 : (n == 16 ? 32 : 160)};
+        for (int p{0}; p < n / 2; ++p) {
+            const int k{(p < n / 4 ? 0 : 1) + 4 * (p % (n / 4))};
+            for (int fx{0}; fx < n; ++fx) {
+                for (int h{0}; h < 2; ++h) {
+                    const int fy{k + 2 * h};
+                    if (fx < n / 8 && fy < n / 8) continue;
+                    const float w{sw[si * 1024 + fx * n + fy]};
+                    pairs[4 * (at + p * n + fx) + h] = 1.0f / w;
+                    pairs[4 * (at + p * n + fx) + 2 + h] = w;
+                }
+            }
+        }
+    }
     // log2f(1 + i) with the host libm: the rate proxy of the selection host twin.
     std::vector<float> l2(kLog2TableSize);
     for (int i{0}; i < kLog2TableSize; ++i) {
@@ -1767,22 +2207,34 @@ bool frontend_tables_init(FrontendTables* tables) {
     }
     float* d_deq{nullptr};
     float* d_sw{nullptr};
+    float* d_pairs{nullptr};
+    float* d_centre{nullptr};
+    float* d_folds{nullptr};
     float* d_l2{nullptr};
     double* d_ob{nullptr};
     if (cudaMalloc(&d_deq, deq.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_sw, sw.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_pairs, pairs.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_centre, centre.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_folds, folds.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_l2, l2.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_ob, ob.size() * 8) != cudaSuccess) {
         return false;
     }
     if (cudaMemcpy(d_deq, deq.data(), deq.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_sw, sw.data(), sw.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_pairs, pairs.data(), pairs.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_folds, folds.data(), folds.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_centre, centre.data(), centre.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_l2, l2.data(), l2.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_ob, ob.data(), ob.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
         return false;
     }
     tables->dequant = d_deq;
     tables->sel_weight = d_sw;
+    tables->sel_pairs = reinterpret_cast<const float4*>(d_pairs);
+    tables->sel_centre = d_centre;
+    tables->fold = reinterpret_cast<const float2*>(d_folds);
     tables->log2_1p = d_l2;
     tables->llf_basis = d_ob;
     return cudaFuncSetAttribute(frontend_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -6,6 +6,8 @@
 // written back.
 #pragma once
 
+#include <vector_types.h>
+
 #include <cstddef>
 #include <cstdint>
 
@@ -70,6 +72,9 @@ constexpr int kDequantInv = 3 * 3 * 1024;
 struct FrontendTables {
     const float* dequant;     // [3 sizes][3 ch][1024] stride 1024 (size 8, 16, 32), then their reciprocals
     const float* sel_weight;  // [3 sizes][1024] DCT8 Y weight sampled at round(f*8/N)
+    const float4* sel_pairs;  // weight pairs of the bounded selection: DCT8 at 0, DCT16 at 32, DCT32 at 160
+    const float2* fold;       // its folded bases: DCT16 (64 entries), DCT32 (256)
+    const float* sel_centre;  // its error per unit of centre and row frequency: DCT8 at 0, DCT16 at 8, DCT32 at 24
     const float* log2_1p;     // [kLog2TableSize] log2f(1 + i)
     const double* llf_basis;  // [2][4][4] orthonormal m-point basis for m = 2, 4
 };
