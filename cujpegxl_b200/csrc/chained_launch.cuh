@@ -1,0 +1,36 @@
+// Launches of kernels that follow each other on a stream with programmatic
+// stream serialisation: the next grid's launch proceeds as the blocks of the
+// previous one leave, instead of after its last block has and its memory is
+// flushed, which saves about a microsecond per launch of a frame's chain of
+// short kernels. Every kernel launched so waits for the previous grid (all of
+// it, its writes visible) before it reads or writes anything; and nothing
+// here triggers the next grid early, so no block sits on an SM, waiting, that
+// another stream's blocks could use.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace jxb {
+
+// (No effect in a kernel launched the ordinary way.)
+__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+bool launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, std::size_t smem, cudaStream_t stream,
+                    const A&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+
+}  // namespace jxb

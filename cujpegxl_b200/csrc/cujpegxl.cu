@@ -16,6 +16,7 @@
 
 #include "cujpegxl/cujpegxl.h"
 #include "cujpegxl_b200/cujpegxl_b200.h"
+#include "chained_launch.cuh"
 #include "encoder_internal.h"
 #include "acsnet.cuh"
 #include "entropy.cuh"
@@ -506,6 +507,7 @@ __global__ void nz_kernel(const std::int16_t* ac, const std::int8_t* acs, int bw
 __global__ void __launch_bounds__(256) readback_kernel(const unsigned long long* result, const std::uint8_t* src,
                                                        std::uint8_t* dst, unsigned long long capacity,
                                                        unsigned long long* words_out) {
+    jxb::wait_for_previous_grid();
     const unsigned long long total{result[0]};
     const unsigned long long status{result[2] != 0 ? 2ull : (total > capacity ? 1ull : 0ull)};
     const unsigned long long tid{static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x};
@@ -548,8 +550,9 @@ bool device_reachable_host(const void* p) {
 
 bool enqueue_readback(cujpegxl_encoder* e, std::uint8_t* dst, std::size_t capacity, unsigned long long* words,
                       cudaStream_t st) {
-    readback_kernel<<<kReadbackBlocks, 256, 0, st>>>(e->ed.result, e->ed.out, dst, capacity, words);
-    return cudaGetLastError() == cudaSuccess;
+    return jxb::launch_chained(readback_kernel, kReadbackBlocks, 256, 0, st, static_cast<const unsigned long long*>(e->ed.result),
+                               static_cast<const std::uint8_t*>(e->ed.out), dst,
+                               static_cast<unsigned long long>(capacity), words);
 }
 
 // A pageable output buffer: the file is copied on the device side into the

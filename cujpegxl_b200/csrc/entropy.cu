@@ -22,6 +22,7 @@
 #include <cstddef>
 #include <cstring>
 
+#include "chained_launch.cuh"
 #include "entropy.cuh"
 #include "jxl_constants.cuh"
 #include "prefix_code.cuh"
@@ -2167,6 +2168,7 @@ __host__ __device__ constexpr unsigned clear_blocks(int ndc) { return 1u + stati
 
 #define JXB_ENTROPY_KERNELS(NAME, BOUNDS, PHASE)                                                           \
     __global__ void BOUNDS NAME##_kernel(const __grid_constant__ EntropyDev e) {                              \
+        wait_for_previous_grid();                                                                             \
         NAME##_body(e, blockIdx.x);                                                                           \
     }                                                                                                         \
     __global__ void BOUNDS NAME##_batch_kernel(const __grid_constant__ EntropyBatch b) {                      \
@@ -2211,7 +2213,10 @@ __device__ __forceinline__ void emit_body(const EntropyDev& e, const unsigned bl
 JXB_ENTROPY_KERNELS(tokens, __launch_bounds__(kAcThreads, 3), kPhaseItems)
 JXB_ENTROPY_KERNELS(codes, __launch_bounds__(32), kPhaseCodes)
 JXB_ENTROPY_KERNELS(lengths, __launch_bounds__(kAcThreads, 8), kPhaseItems)
-__global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const __grid_constant__ EntropyDev e) { layout_body(e); }
+__global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const __grid_constant__ EntropyDev e) {
+    wait_for_previous_grid();
+    layout_body(e);
+}
 __global__ void __launch_bounds__(kLayoutThreads) layout_batch_kernel(const __grid_constant__ EntropyBatch b) {
     layout_body(b.frames[blockIdx.x]);
 }
@@ -2280,17 +2285,21 @@ bool entropy_launch(const EntropyDev& e, void* stream) {
     cudaStream_t st{static_cast<cudaStream_t>(stream)};
     const unsigned units{e.misc_units + static_cast<unsigned>(e.nstripes)};
     if (e.clear_first) clear_kernel<<<clear_blocks(e.ndc), 256, 0, st>>>(e);
+    const auto codes{static_cast<unsigned>(kNumClusters + 2 * e.ndc)};
     if (e.direct) {
-        tokens_kernel<<<units, kAcThreads, kDirectSmem, st>>>(e);
-    } else {
-        tokens_staged_kernel<<<units, kAcThreads, kHistSmem, st>>>(e);
+        return launch_chained(tokens_kernel, units, kAcThreads, kDirectSmem, st, e) &&
+               launch_chained(codes_kernel, codes, 32, sizeof(WarpCodeSmem), st, e) &&
+               launch_chained(lengths_kernel, units, kAcThreads, 0, st, e) &&
+               launch_chained(layout_kernel, 1, kLayoutThreads, 0, st, e) &&
+               launch_chained(emit_kernel, units, kAcThreads, kEmitStoredSmem, st, e);
     }
-    codes_kernel<<<kNumClusters + 2 * e.ndc, 32, sizeof(WarpCodeSmem), st>>>(e);
-    if (!e.direct) lengths_unstored_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(e);
+    tokens_staged_kernel<<<units, kAcThreads, kHistSmem, st>>>(e);
+    codes_kernel<<<codes, 32, sizeof(WarpCodeSmem), st>>>(e);
+    lengths_unstored_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(e);
     lengths_kernel<<<units, kAcThreads, 0, st>>>(e);
     layout_kernel<<<1, kLayoutThreads, 0, st>>>(e);
     emit_kernel<<<units, kAcThreads, kEmitStoredSmem, st>>>(e);
-    if (!e.direct) emit_unstored_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(e);
+    emit_unstored_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(e);
     return cudaGetLastError() == cudaSuccess;
 }
 
