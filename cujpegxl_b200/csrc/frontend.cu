@@ -1907,6 +1907,15 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     frontend_tile(in, sc, tb, out, tx, ty, smem + half * (kTileSmemStride / sizeof(float)), 1 + half);
 }
 
+// One tile per CTA, for frames of at most as many tiles as the device has SMs:
+// a pair would share one SM's issue slots and shared memory while another SM
+// idles.
+__global__ void __launch_bounds__(kThreads, 1)
+    frontend_single_kernel(FrontendInputs in, FrontendScalars sc, FrontendTables tb, FrontendOutputs out) {
+    extern __shared__ __align__(16) float smem[];
+    frontend_tile(in, sc, tb, out, static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), smem, 1);
+}
+
 // One tile of a batched launch, kept out of line: inlined into the work loop,
 // the tile's code held about 30 more registers live (its frame's fields and
 // coordinates are run-time values here, where the single-frame kernel reads
@@ -2237,7 +2246,14 @@ bool frontend_tables_init(FrontendTables* tables) {
     tables->fold = reinterpret_cast<const float2*>(d_folds);
     tables->log2_1p = d_l2;
     tables->llf_basis = d_ob;
-    return cudaFuncSetAttribute(frontend_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    int device{0};
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&tables->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        return false;
+    }
+    return cudaFuncSetAttribute(frontend_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(kTileSmemStride)) == cudaSuccess &&
+           cudaFuncSetAttribute(frontend_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(2 * kTileSmemStride)) == cudaSuccess &&
            cudaFuncSetAttribute(frontend_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(2 * kTileSmemStride)) == cudaSuccess &&
@@ -2250,8 +2266,12 @@ bool frontend_tables_init(FrontendTables* tables) {
 bool frontend_launch(const FrontendInputs& in, const FrontendScalars& s, const FrontendTables& t,
                      const FrontendOutputs& out, void* stream) {
     const int tiles_x{(in.width + kTile - 1) / kTile};
-    const dim3 grid{static_cast<unsigned>((tiles_x + 1) / 2), static_cast<unsigned>((in.height + kTile - 1) / kTile)};
-    if (in.tile_order != nullptr) {
+    const int tiles_y{(in.height + kTile - 1) / kTile};
+    const dim3 grid{static_cast<unsigned>((tiles_x + 1) / 2), static_cast<unsigned>(tiles_y)};
+    if (static_cast<long long>(tiles_x) * tiles_y <= t.sms) {
+        const dim3 tiles{static_cast<unsigned>(tiles_x), static_cast<unsigned>(tiles_y)};
+        frontend_single_kernel<<<tiles, kThreads, kTileSmemStride, static_cast<cudaStream_t>(stream)>>>(in, s, t, out);
+    } else if (in.tile_order != nullptr) {
         frontend_kernel<true><<<grid, kPairThreads, 2 * kTileSmemStride, static_cast<cudaStream_t>(stream)>>>(in, s, t,
                                                                                                            out);
     } else {

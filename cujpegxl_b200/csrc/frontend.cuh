@@ -77,6 +77,7 @@ struct FrontendTables {
     const float* sel_centre;  // its error per unit of centre and row frequency: DCT8 at 0, DCT16 at 8, DCT32 at 24
     const float* log2_1p;     // [kLog2TableSize] log2f(1 + i)
     const double* llf_basis;  // [2][4][4] orthonormal m-point basis for m = 2, 4
+    int sms;                  // SMs of the device
 };
 
 constexpr int kLog2TableSize = 1 << 19;
