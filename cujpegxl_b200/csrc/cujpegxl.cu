@@ -159,11 +159,9 @@ bool device_tables(int device, jxb::FrontendTables* out) {
 bool device_exists(std::int32_t ordinal, int* major, int* minor) {
     int count{0};
     if (cudaGetDeviceCount(&count) != cudaSuccess || ordinal < 0 || ordinal >= count) return false;
-    cudaDeviceProp prop{};
-    if (cudaGetDeviceProperties(&prop, ordinal) != cudaSuccess) return false;
-    *major = prop.major;
-    *minor = prop.minor;
-    return true;
+    // (Two attributes; cudaGetDeviceProperties takes milliseconds.)
+    return cudaDeviceGetAttribute(major, cudaDevAttrComputeCapabilityMajor, ordinal) == cudaSuccess &&
+           cudaDeviceGetAttribute(minor, cudaDevAttrComputeCapabilityMinor, ordinal) == cudaSuccess;
 }
 
 // src/cujpegxl.cc:36-48: distance must be positive and finite; width and

@@ -164,22 +164,40 @@ constexpr int kChromaWin = kTile / 2 + 2 * kChromaMargin;  // 36
 // tests/cpu_checks/quant_div_check.c; both sides scale exactly with a's
 // exponent and are odd in a, so it holds for every a whose quotient and
 // residual stay normal, which includes every |a| > w / 2 the quantiser
-// divides. (The selection's quantiser keeps the IEEE division: its quotients
-// are formed in an out-of-line function, where loading the reciprocal cost
-// more than the division.)
-__device__ __forceinline__ float div_weight(float a, float w, float w_inv) {
-    const float q0{a * w_inv};
-    return jx_fma(jx_fma(-q0, w, a), w_inv, q0);
+// divides. (The selection's exact quantiser keeps the IEEE division: its
+// quotients are formed in an out-of-line function, where loading the
+// reciprocal cost more than the division.) Two values at once.
+__device__ __forceinline__ float2 div_weight(float2 a, float2 w, float2 w_inv) {
+    const float2 q0{__fmul2_rn(a, w_inv)};
+    return __ffma2_rn(__ffma2_rn(f2neg(q0), w, a), w_inv, q0);
 }
 
-// lrintf((v * qgsf) / w) for a positive weight w (src/frontend_quantize.cu:
-// 165-178), with no branch: the quotient is exact wherever it can round away
-// from zero (|v * qgsf| >= w / 2 keeps div_weight's intermediates normal), and
-// where the dividend is so small that they are not, the quotient is far below
-// 1/2 and rounds to zero either way. (Without the zero fast path the lanes of
-// a warp no longer diverge: 3% fewer cycles in the phase.)
-__device__ __forceinline__ int quantize(float v, float qgsf, float w, float w_inv) {
-    return static_cast<int>(lrintf(div_weight(v * qgsf, w, w_inv)));
+// rintf((v * qgsf) / w) of two values for positive weights w
+// (src/frontend_quantize.cu:165-178), with no branch: the quotient is exact
+// wherever it can round away from zero (|v * qgsf| >= w / 2 keeps div_weight's
+// intermediates normal), and where the dividend is so small that they are not,
+// the quotient is far below 1/2 and rounds to zero either way.
+__device__ __forceinline__ float2 quantize2(float2 v, float qgsf, float2 w, float2 w_inv) {
+    const float2 q{div_weight(__fmul2_rn(v, f2dup(qgsf)), w, w_inv)};
+    return make_float2(rintf(q.x), rintf(q.y));
+}
+
+// a / b of two dividends for any divisor b, from b_inv = RN(1 / b). One
+// correction of q0 = RN(a * b_inv), which is within 1.5 ulp, gives a faithful
+// quotient (the correction's own error is that of b_inv times a few ulp); a
+// second, from a faithful quotient whose residual is exact and a correctly
+// rounded reciprocal, gives RN(a / b) (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
+// 1990). Zero dividends give zero; the others here, quanta times weights over
+// qgsf, stay far from the ends of the exponent range. The packed corrections
+// replace one IEEE division with its range check, behind a branch on zero, per
+// coefficient.
+__device__ __forceinline__ float2 div2_any(float2 a, float b, float b_inv) {
+    const float2 nb{f2dup(-b)};
+    const float2 y{f2dup(b_inv)};
+    float2 q{__fmul2_rn(a, y)};
+    q = __ffma2_rn(__ffma2_rn(q, nb, a), y, q);
+    return __ffma2_rn(__ffma2_rn(q, nb, a), y, q);
 }
 
 // RatioOfDerivativesOfCubicRootToSimpleGamma (src/adaptive_quant_impl.cuh:44-55).
@@ -1799,23 +1817,32 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 const float4 ix4{*reinterpret_cast<const float4*>(wt + kDequantInv + raw)};
                 const float4 iy4{*reinterpret_cast<const float4*>(wt + kDequantInv + 1024 + raw)};
                 const float4 ib4{*reinterpret_cast<const float4*>(wt + kDequantInv + 2048 + raw)};
-                const float wx[4]{wx4.x, wx4.y, wx4.z, wx4.w};
-                const float wy[4]{wy4.x, wy4.y, wy4.z, wy4.w};
-                const float wb[4]{wb4.x, wb4.y, wb4.z, wb4.w};
-                const float ix[4]{ix4.x, ix4.y, ix4.z, ix4.w};
-                const float iy[4]{iy4.x, iy4.y, iy4.z, iy4.w};
-                const float ib[4]{ib4.x, ib4.y, ib4.z, ib4.w};
+                const float inv_qgsf{1.0f / qgsf};
+                const float2 wx[2]{make_float2(wx4.x, wx4.y), make_float2(wx4.z, wx4.w)};
+                const float2 wy[2]{make_float2(wy4.x, wy4.y), make_float2(wy4.z, wy4.w)};
+                const float2 wb[2]{make_float2(wb4.x, wb4.y), make_float2(wb4.z, wb4.w)};
+                const float2 ix[2]{make_float2(ix4.x, ix4.y), make_float2(ix4.z, ix4.w)};
+                const float2 iy[2]{make_float2(iy4.x, iy4.y), make_float2(iy4.z, iy4.w)};
+                const float2 ib[2]{make_float2(ib4.x, ib4.y), make_float2(ib4.z, ib4.w)};
 #pragma unroll
-                for (int h{0}; h < 4; ++h) {
-                    if (llf_row && col + h < side) continue;  // an LLF slot
-                    const int qy{quantize(yr[h], qgsf, wy[h], iy[h])};
+                for (int p{0}; p < 2; ++p) {
+                    const float2 qy{quantize2(make_float2(yr[2 * p], yr[2 * p + 1]), qgsf, wy[p], iy[p])};
                     // A zero Y quantum reconstructs to a signed zero, and
                     // fma(-m, +-0, v) equals v up to the sign of a zero
                     // result, which quantises to 0 either way.
-                    const float yq{qy == 0 ? 0.0f : (static_cast<float>(qy) * wy[h]) / qgsf};
-                    ax[h] = static_cast<std::int16_t>(quantize(jx_fma(-ytox, yq, xr[h]), qgsf, wx[h], ix[h]));
-                    ay[h] = static_cast<std::int16_t>(qy);
-                    ab[h] = static_cast<std::int16_t>(quantize(jx_fma(-ytob, yq, br[h]), qgsf, wb[h], ib[h]));
+                    const float2 yq{div2_any(__fmul2_rn(qy, wy[p]), qgsf, inv_qgsf)};
+                    const float2 qx{quantize2(__ffma2_rn(f2dup(-ytox), yq, make_float2(xr[2 * p], xr[2 * p + 1])), qgsf,
+                                              wx[p], ix[p])};
+                    const float2 qb{quantize2(__ffma2_rn(f2dup(-ytob), yq, make_float2(br[2 * p], br[2 * p + 1])), qgsf,
+                                              wb[p], ib[p])};
+#pragma unroll
+                    for (int k{0}; k < 2; ++k) {
+                        const int h{2 * p + k};
+                        if (llf_row && col + h < side) continue;  // an LLF slot
+                        ax[h] = static_cast<std::int16_t>(static_cast<int>(k == 0 ? qx.x : qx.y));
+                        ay[h] = static_cast<std::int16_t>(static_cast<int>(k == 0 ? qy.x : qy.y));
+                        ab[h] = static_cast<std::int16_t>(static_cast<int>(k == 0 ? qb.x : qb.y));
+                    }
                 }
             }
             const std::size_t g{(static_cast<std::size_t>(by0 + lby) * bw + bx0 + lbx) * 64 + slot};
