@@ -144,11 +144,12 @@ constexpr std::size_t kTileSmemStride = (kSmemBytes + 15) / 16 * 16;
 constexpr int kPairThreads = 2 * kThreads;
 static_assert(2 * kTileSmemStride <= 227 * 1024, "two tiles no longer fit in one CTA");
 
-// Synchronises the kThreads threads of one tile on named barrier `bar` (1 or
+// Synchronises the kT threads of one tile on named barrier `bar` (1 or
 // 2; barrier 0 is __syncthreads), with the ordering of shared memory that
 // __syncthreads gives.
+template <int kT = kThreads>
 __device__ __forceinline__ void tile_sync(int bar) {
-    asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kThreads) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kT) : "memory");
 }
 
 // Chroma window of a tile in shared memory: kChromaWin x kChromaWin (cb, cr)
@@ -724,9 +725,10 @@ __device__ __forceinline__ void llf_to_dc(const __half* coef, int f, int ox, int
     }
 }
 
-// The whole frontend of the 64x64 tile (tx, ty) of one frame; `smem` is the
+// The whole frontend of the 64x64 tile (tx, ty) of one frame by kT threads; `smem` is the
 // CTA's dynamic shared memory (kSmemBytes). The caller synchronises before
 // the CTA starts another tile.
+template <int kT>
 __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const FrontendScalars& sc,
                                               const FrontendTables& tb, const FrontendOutputs& out, int tx,
                                               int ty, float* smem, int bar) {
@@ -737,7 +739,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     float* shp{smem + kRegionAFloats};               // [3][64*kSs]
     Small& sm{*reinterpret_cast<Small*>(smem + kRegionAFloats + 3 * kSplane)};
 
-    const int tid{static_cast<int>(threadIdx.x) & (kThreads - 1)};
+    const int tid{static_cast<int>(threadIdx.x) & (kT - 1)};
     const int lane{tid & 31};
     const int warp{tid >> 5};
     const int W{in.width};
@@ -764,9 +766,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
         const int ch{H >> 1};
         // The folded bases and the learned class are loaded here and stored
         // after the window, so that their latency overlaps the window's.
-        static_assert(64 + 256 <= 2 * kThreads, "two basis entries per thread");
-        const float2 fold_a{tb.fold[tid]};
-        const float2 fold_b{tid < 64 ? tb.fold[kThreads + tid] : make_float2(0.0f, 0.0f)};
+        constexpr int kFold{64 + 256};
+        static_assert(kFold <= 2 * kT, "two basis entries per thread");
+        const float2 fold_a{tid < kFold ? tb.fold[tid] : make_float2(0.0f, 0.0f)};
+        const float2 fold_b{tid + kT < kFold ? tb.fold[kT + tid] : make_float2(0.0f, 0.0f)};
         signed char net_entry{-1};
         if (tid < 4) {
             const int rw{(bw + 3) >> 2};
@@ -788,12 +791,12 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             constexpr int kChromaWords{kChromaWin / 2};  // 18 words per chroma row
             constexpr int kLumaItems{kXs * kLumaWords};
             constexpr int kChromaItems{kChromaWin * kChromaWords};
-            constexpr int kLumaPer{(kLumaItems + kThreads - 1) / kThreads};
-            constexpr int kChromaPer{(kChromaItems + kThreads - 1) / kThreads};
+            constexpr int kLumaPer{(kLumaItems + kT - 1) / kT};
+            constexpr int kChromaPer{(kChromaItems + kT - 1) / kT};
             std::uint32_t lo[kLumaPer], hi[kLumaPer], cv[kChromaPer];
 #pragma unroll
             for (int j{0}; j < kLumaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kLumaItems) {
                     const int row{i / kLumaWords};
                     const int w{i - row * kLumaWords};
@@ -805,7 +808,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
 #pragma unroll
             for (int j{0}; j < kChromaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kChromaItems) {
                     const int row{i / kChromaWords};
                     const int w{i - row * kChromaWords};
@@ -817,22 +820,22 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             auto* lw{reinterpret_cast<std::uint32_t*>(win_luma)};  // word i = row * kLumaWords + w
 #pragma unroll
             for (int j{0}; j < kLumaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kLumaItems) lw[i] = __funnelshift_r(lo[j], hi[j], 16);
             }
             auto* cwd{reinterpret_cast<std::uint32_t*>(win_chroma)};
 #pragma unroll
             for (int j{0}; j < kChromaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kChromaItems) cwd[i] = cv[j];
             }
         } else {
-            constexpr int kLumaPer{(kXplane + kThreads - 1) / kThreads};
-            constexpr int kChromaPer{(kChromaWin * kChromaWin + kThreads - 1) / kThreads};
+            constexpr int kLumaPer{(kXplane + kT - 1) / kT};
+            constexpr int kChromaPer{(kChromaWin * kChromaWin + kT - 1) / kT};
             std::uint8_t lv[kLumaPer], cb[kChromaPer], cr[kChromaPer];
 #pragma unroll
             for (int j{0}; j < kLumaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kXplane) {
                     const int gx{min(max(px0 - kHalo + i % kXs, 0), W - 1)};
                     const int gy{min(max(py0 - kHalo + i / kXs, 0), H - 1)};
@@ -841,7 +844,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
 #pragma unroll
             for (int j{0}; j < kChromaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kChromaWin * kChromaWin) {
                     const int jx{min(max(cx0 + i % kChromaWin, 0), cw - 1)};
                     const int jy{min(max(cy0 + i / kChromaWin, 0), ch - 1)};
@@ -852,27 +855,27 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
 #pragma unroll
             for (int j{0}; j < kLumaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kXplane) win_luma[i] = lv[j];
             }
 #pragma unroll
             for (int j{0}; j < kChromaPer; ++j) {
-                const int i{tid + j * kThreads};
+                const int i{tid + j * kT};
                 if (i < kChromaWin * kChromaWin) {
                     win_chroma[2 * i] = cb[j];
                     win_chroma[2 * i + 1] = cr[j];
                 }
             }
         }
-        sm.fold[tid] = fold_a;
-        if (tid < 64) sm.fold[kThreads + tid] = fold_b;
+        if (tid < kFold) sm.fold[tid] = fold_a;
+        if (tid + kT < kFold) sm.fold[kT + tid] = fold_b;
         if (tid < 4) sm.net[tid] = net_entry;
 #pragma unroll
         for (int k{0}; k < 6; ++k) {
             if (tid == k) sm.pow_lut[k] = make_float2(pow24_factor_c(k), pow24_factor_scale(k));
         }
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
     // Regions whose transform split (and, with net_qf, quant field) the
     // network decided; zero without a network.
     unsigned dmask{0};
@@ -883,7 +886,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     // pixels per thread (the row length kXs is even, so a pair never spans
     // two rows, and its float2 stores are 8-byte aligned).
     static_assert(kXs % 2 == 0 && kXplane % 2 == 0, "XYB pairs");
-    for (int i2{tid}; i2 < kXplane / 2; i2 += kThreads) {
+    for (int i2{tid}; i2 < kXplane / 2; i2 += kT) {
         const int i{2 * i2};
         const int row{i / kXs};
         const int col{i - row * kXs};
@@ -897,10 +900,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
         *reinterpret_cast<float2*>(xyb + kXplane + i) = y;
         *reinterpret_cast<float2*>(xyb + 2 * kXplane + i) = b;
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
 
     if (out.dbg_xyb != nullptr) {
-        for (int i{tid}; i < 3 * kTile * kTile; i += kThreads) {
+        for (int i{tid}; i < 3 * kTile * kTile; i += kT) {
             const int c{i / (kTile * kTile)};
             const int p{i % (kTile * kTile)};
             const int gx{px0 + p % kTile};
@@ -917,7 +920,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     // the phase (the branch is uniform over the CTA).
     const float* Y{xyb + kXplane};
     if (qmask != 0xFu) {
-        {
+        if (kT == 256 || tid < 256) {
             // Pixels (dx, dx + 1) of each cell row in pairs on packed f32x2
             // arithmetic (the division and square root stay scalar); the sum
             // still accumulates in raster order.
@@ -964,14 +967,15 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
             sm.pre[tid] = 0.25f * sum;
         }
-        tile_sync(bar);
-        // The four eroded cells of each of this warp's 8 blocks (block warp + 8j),
+        tile_sync<kT>(bar);
+        // The four eroded cells of each of this warp's blocks (block warp + kWarps * j),
         // one per lane: lane 4j + k holds cell k = (k & 1, k >> 1) of block j's
         // 2x2 cells. Their sum (e0 + e2) + (e1 + e3) is the order in which a
         // 32-lane tree with the cells in lanes 0-3 and zeros elsewhere adds them.
+        constexpr int kWarps{kT / 32};
         float ero_sum;
         {
-            const int lb{warp + 8 * (lane >> 2)};
+            const int lb{min(warp + kWarps * (lane >> 2), 63)};
             const int k{lane & 3};
             const int lbx{lb & 7};
             const int lby{lb >> 3};
@@ -980,12 +984,12 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const float s{e + __shfl_down_sync(0xffffffffu, e, 2)};
             ero_sum = s + __shfl_down_sync(0xffffffffu, s, 1);
         }
-        for (int lb{warp}; lb < 64; lb += kThreads / 32) {
+        for (int lb{warp}; lb < 64; lb += kT / 32) {
             const int lbx{lb & 7};
             const int lby{lb >> 3};
             const int gbx{bx0 + lbx};
             const int gby{by0 + lby};
-            const float eroded{__shfl_sync(0xffffffffu, ero_sum, 4 * (lb >> 3))};
+            const float eroded{__shfl_sync(0xffffffffu, ero_sum, 4 * (lb / kWarps))};
             if (gbx >= bw || gby >= bh || ((qmask >> region_of_block(lb)) & 1u) != 0) {
                 continue;  // warp-uniform
             }
@@ -1043,7 +1047,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     // them, and operand pair (dx, dy) is {row[x+dx], row[x+1+dx]}. (Four rows
     // instead of two: 14.1K -> 12.8K cycles per tile for the phase.)
     static_assert(kXs % 2 == 0 && kHalo % 2 == 0, "gaborish pairs");
-    for (int i8{tid}; i8 < 3 * kTile * kTile / 8; i8 += kThreads) {
+    for (int i8{tid}; i8 < 3 * kTile * kTile / 8; i8 += kT) {
         const int c{i8 >> 9};
         const int p8{i8 & 511};
         const int x{2 * (p8 & 31)};
@@ -1080,10 +1084,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             *reinterpret_cast<float2*>(shp + c * kSplane + (y0 + h) * kSs + x) = sv;
         }
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
 
     if (out.dbg_sharp != nullptr) {
-        for (int i{tid}; i < 3 * kTile * kTile; i += kThreads) {
+        for (int i{tid}; i < 3 * kTile * kTile; i += kT) {
             const int c{i >> 12};
             const int p{i & 4095};
             const int gx{px0 + (p & 63)};
@@ -1111,7 +1115,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     // Warps 4-7 clear the non-zero counters and CfL sums and finish
     // each block's quant field from its AQ sums.
     if (tid >= 128) {
-        for (int i{tid - 128}; i < 192; i += 128) {
+        for (int i{tid - 128}; i < 192; i += kT - 128) {
             sm.nz[i >> 6][i & 63] = 0;
             sm.cfl[i >> 6][i & 63] = 0.0f;  // blocks that are not first blocks add zero
         }
@@ -1158,8 +1162,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
         static_assert(kRows32 % 4 == 0 && kRows32 + 4 * 32 * kNearStride<32> <= kRegionAFloats, "row scratch of the bounded selection");
         auto centre_of = [&](int ri) { return SY[((ri >> 1) * 32 + 16) * kSs + (ri & 1) * 32 + 16] * qg; };
 #pragma unroll
-        for (int h{0}; h < 2; ++h) {
-            const int k{tid + h * kThreads};
+        for (int h{0}; h < 512 / kT; ++h) {
+            const int k{tid + h * kT};
             const int lb{k >> 3};
             const int r{k & 7};
             if (((exact >> region_of_block(lb)) & 1u) != 0) {
@@ -1167,8 +1171,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                                   rows + lb * 72 + r);
             }
         }
-        {
-            const int qd{tid >> 4};
+        // (With 512 threads the DCT16 rows and columns go to the upper half, the
+        // DCT32 ones to the lower.)
+        if (kT == 256 || tid >= 256) {
+            const int qd{(tid & 255) >> 4};
             const int r{tid & 15};
             const int ri{((qd >> 3) << 1) | ((qd & 3) >> 1)};
             if (((exact >> ri) & 1u) != 0) {
@@ -1176,7 +1182,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                                    rows + kRows16 + qd * 272 + r);
             }
         }
-        {
+        if (kT == 256 || tid < 256) {
             // A warp per region and parity.
             const int ri{tid >> 6};
             const int r{tid & 31};
@@ -1192,9 +1198,9 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 }
             }
         }
-        tile_sync(bar);
+        tile_sync<kT>(bar);
         const float inv_scale2{1.0f / (qg * qg)};
-        {
+        if (kT == 256 || tid < 256) {
             const int ri{tid >> 6};
             const int fx{tid & 31};
             if (((exact >> ri) & 1u) != 0) {
@@ -1208,8 +1214,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 if (lane == 0) sm.near32[ri][(tid >> 5) & 1] = v;
             }
         }
-        {
-            const int qd{tid >> 4};
+        if (kT == 256 || tid >= 256) {
+            const int qd{(tid & 255) >> 4};
             const int fx{tid & 15};
             const int ri{((qd >> 3) << 1) | ((qd & 3) >> 1)};
             const bool on{((exact >> ri) & 1u) != 0};
@@ -1222,8 +1228,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             if (on && fx == 0) sm.near16[qd] = v;
         }
 #pragma unroll
-        for (int h{0}; h < 2; ++h) {
-            const int k{tid + h * kThreads};
+        for (int h{0}; h < 512 / kT; ++h) {
+            const int k{tid + h * kT};
             const int lb{k >> 3};
             const int fx{k & 7};
             const int ri{region_of_block(lb)};
@@ -1236,7 +1242,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             v = group_sum2<8>(v);
             if (on && fx == 0) sm.near8[lb] = v;
         }
-        tile_sync(bar);
+        tile_sync<kT>(bar);
         // Decisions, a warp per region and a lane per block, four lanes to a
         // quad: the comparisons of 4d on [cost - bound, cost + bound].
         if (warp < 4) {
@@ -1283,7 +1289,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 if (lane == 0) sm.undecided[ri] = take32 || split ? 0 : 1;
             }
         }
-        tile_sync(bar);
+        tile_sync<kT>(bar);
         unsigned left{0};
 #pragma unroll
         for (int ri{0}; ri < 4; ++ri) left |= (((exact >> ri) & 1u) != 0 && sm.undecided[ri] != 0 ? 1u : 0u) << ri;
@@ -1291,7 +1297,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     }
     if (exact != 0u) {
         // 4a. DCT8 candidates: one per block inside the image.
-        for (int k{tid}; k < 512; k += kThreads) {
+        for (int k{tid}; k < 512; k += kT) {
             const int lb{k >> 3};
             const int r{k & 7};
             const int lbx{lb & 7};
@@ -1300,8 +1306,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 row_pass<8, 0, 8, true>(SY + (lby * 8 + r) * kSs + lbx * 8, rows + lb * 72 + r);
             }
         }
-        tile_sync(bar);
-        for (int k{tid}; k < 512; k += kThreads) {
+        tile_sync<kT>(bar);
+        for (int k{tid}; k < 512; k += kT) {
             const int lb{k >> 3};
             const int fx{k & 7};
             if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh &&
@@ -1310,10 +1316,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                                  crate + lb * 72 + fx * 9, fx, qg, tb.sel_weight, tb.log2_1p);
             }
         }
-        tile_sync(bar);
+        tile_sync<kT>(bar);
         // Distortion and rate ride one packed pair through each step.
 #pragma unroll 2
-        for (int lb{warp}; lb < 64; lb += kThreads / 32) {
+        for (int lb{warp}; lb < 64; lb += kT / 32) {
             if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh &&
                 ((exact >> region_of_block(lb)) & 1u) != 0) {
                 const int i0{lb * 72 + (lane >> 3) * 9 + (lane & 7)};
@@ -1328,7 +1334,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
         // 4b. DCT16 candidates: the 16 quads of the tile that fit in the image.
         // Their row pass writes only the row scratch, which the DCT8
         // reduction above does not read, so it shares that phase.
-        for (int k{tid}; k < 256; k += kThreads) {
+        for (int k{tid}; k < 256; k += kT) {
             const int qd{k >> 4};
             const int r{k & 15};
             const int qx{qd & 3};
@@ -1338,8 +1344,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 row_pass<16, 0, 16, true>(SY + (qy * 16 + r) * kSs + qx * 16, rows + qd * 272 + r);
             }
         }
-        tile_sync(bar);
-        for (int k{tid}; k < 256; k += kThreads) {
+        tile_sync<kT>(bar);
+        for (int k{tid}; k < 256; k += kT) {
             const int qd{k >> 4};
             const int fx{k & 15};
             if (bx0 + 2 * (qd & 3) + 2 <= bw && by0 + 2 * (qd >> 2) + 2 <= bh &&
@@ -1349,8 +1355,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                                    tb.log2_1p);
             }
         }
-        tile_sync(bar);
-        for (int qd{warp}; qd < 16; qd += kThreads / 32) {
+        tile_sync<kT>(bar);
+        for (int qd{warp}; qd < 16; qd += kT / 32) {
             if (bx0 + 2 * (qd & 3) + 2 <= bw && by0 + 2 * (qd >> 2) + 2 <= bh &&
                 ((exact >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) != 0) {
                 // Distortion (x) and rate (y) as packed pairs, each in the
@@ -1375,7 +1381,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
         // 4c. DCT32 candidates: the 4 regions of the tile that fit in the image.
         // Their row pass shares the DCT16 reduction's phase (disjoint
         // scratch).
-        for (int k{tid}; k < 256; k += kThreads) {
+        for (int k{tid}; k < 256; k += kT) {
             const int ri{k >> 6};
             const int r{k & 31};
             const bool hi{(k & 32) != 0};
@@ -1391,8 +1397,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 }
             }
         }
-        tile_sync(bar);
-        for (int k{tid}; k < 256; k += kThreads) {
+        tile_sync<kT>(bar);
+        for (int k{tid}; k < 256; k += kT) {
             const int ri{k >> 6};
             const int fx{k & 31};
             const bool hi{(k & 32) != 0};
@@ -1408,7 +1414,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                 }
             }
         }
-        tile_sync(bar);
+        tile_sync<kT>(bar);
         if (warp < 4) {
             const int ri{warp};
             if (bx0 + 4 * (ri & 1) + 4 <= bw && by0 + 4 * (ri >> 1) + 4 <= bh &&
@@ -1531,10 +1537,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
         }
     }
-        tile_sync(bar);
+        tile_sync<kT>(bar);
     }
     if (out.dbg_cost != nullptr) {
-        for (int lb{tid}; lb < 64; lb += kThreads) {
+        for (int lb{tid}; lb < 64; lb += kT) {
             const int lbx{lb & 7};
             const int lby{lb >> 3};
             if (bx0 + lbx < bw && by0 + lby < bh) {
@@ -1602,7 +1608,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             off += cnt * step;
         }
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
 
     // ---- 5. variable DCT of X, Y, B -> FP16 coefficients (src/frontend_transform.cu:190-266).
     // The three channels' row passes run in one phase (each channel has its
@@ -1616,7 +1622,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     const int t32{64 * n32};
     const int t16{t32 + 16 * n16};
     const int tall{t16 + 8 * n8};
-    for (int k3{tid}; k3 < 3 * tall; k3 += kThreads) {
+    for (int k3{tid}; k3 < 3 * tall; k3 += kT) {
         const int c{k3 >= 2 * tall ? 2 : (k3 >= tall ? 1 : 0)};
         const int k{k3 - c * tall};
         const float* P{shp + c * kSplane};
@@ -1644,8 +1650,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             row_pass<8, 0, 8, false>(P + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, drows + sm.fb_off[f] + r);
         }
     }
-    tile_sync(bar);
-    for (int k3{tid}; k3 < 3 * tall; k3 += kThreads) {
+    tile_sync<kT>(bar);
+    for (int k3{tid}; k3 < 3 * tall; k3 += kT) {
         const int c{k3 >= 2 * tall ? 2 : (k3 >= tall ? 1 : 0)};
         const int k{k3 - c * tall};
         const float* drows{smem + c * kDrowsChannel};
@@ -1672,10 +1678,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             dct_col<8, 0, 8>(drows + sm.fb_off[f] + fx * 9, cc, fx, lb & 7, lb >> 3);
         }
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
 
     if (out.dbg_coeff != nullptr) {
-        for (int i{tid}; i < 3 * 4096; i += kThreads) {
+        for (int i{tid}; i < 3 * 4096; i += kT) {
             const int c{i >> 12};
             const int lb{(i >> 6) & 63};
             const int gbx{bx0 + (lb & 7)};
@@ -1690,13 +1696,14 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
 
     // ---- 6. chroma from luma over the tile (src/frontend_quantize.cu:49-117),
     // and DC from the low-frequency corners (src/frontend_quantize.cu:180-200,
-    // src/vardct_layout.h:88-111), which needs no CfL result. Warps 0-5 take
-    // the (first block, sum kind) pairs round-robin, the largest transforms
-    // first, each sum across the warp (cfl_sum_warp). Warps 6-7: one 8x8 DC
-    // position per thread.
-    if (tid < 192) {
+    // src/vardct_layout.h:88-111), which needs no CfL result. All warps but
+    // the last two take the (first block, sum kind) pairs round-robin, the largest transforms
+    // first, each sum across the warp (cfl_sum_warp). The last two: one
+    // 8x8 DC position per thread.
+    constexpr int kCflThreads{kT - 64};
+    if (tid < kCflThreads) {
         const int nfb{sm.n32 + sm.n16 + sm.n8};
-        for (int t{warp}; t < 3 * nfb; t += 6) {
+        for (int t{warp}; t < 3 * nfb; t += kCflThreads / 32) {
             const int i{t / 3};
             const int which{t - 3 * i};
             const int lb{sm.fb_list[i]};
@@ -1705,8 +1712,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
                                                             : cfl_sum_kind<8>(coef, lb, which, lane))};
             if (lane == 0) sm.cfl[which][lb] = v;
         }
-    } else if (tid >= 192) {
-        const int p{tid - 192};
+    } else {
+        const int p{tid - kCflThreads};
         const int f{sm.owner[p]};
         if (bx0 + (p & 7) < bw && by0 + (p >> 3) < bh) {
             const int n{sm.acs[f]};
@@ -1734,7 +1741,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             out.dc[2 * static_cast<std::size_t>(nblocks) + blk] = static_cast<int>(lrintf((dcv[2] - ydr) * dcq_b));
         }
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
     // The tile's maps: every warp reduces the 64 partials itself (the same
     // tree, so the same maps on every warp) instead of waiting at one more
     // barrier for warp 0 to do it. The trees leave the sums in lane 0, which
@@ -1774,8 +1781,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     // warp's iteration take the 64 slots of one tile block, lanes 16-31 those
     // of the next, so the block's setup serves four slots per lane, weights
     // move as 16-byte loads and outputs as 8-byte stores.
-    static_assert(kThreads % 32 == 0 && 1024 % kThreads == 0, "two tile blocks per warp iteration");
-    for (int k4{tid}; k4 < 1024; k4 += kThreads) {  // 4 uniform iterations per warp
+    static_assert(kT % 32 == 0 && 1024 % kT == 0, "two tile blocks per warp iteration");
+    for (int k4{tid}; k4 < 1024; k4 += kT) {  // uniform iterations per warp
         const int k{4 * k4};
         const int lb{k >> 6};
         const int slot{k & 63};
@@ -1874,10 +1881,10 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             if (cb) atomicAdd(&sm.nz[2][f], static_cast<int>(cb));
         }
     }
-    tile_sync(bar);
+    tile_sync<kT>(bar);
 
     // ---- 8. side information.
-    for (int k{tid}; k < 64; k += kThreads) {
+    for (int k{tid}; k < 64; k += kT) {
         const int lb{k};
         const int gbx{bx0 + (lb & 7)};
         const int gby{by0 + (lb >> 3)};
@@ -1931,16 +1938,18 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     } else {
         if (tx * kTile >= in.width) return;  // the right half of an odd tile row: no barrier waits on it
     }
-    frontend_tile(in, sc, tb, out, tx, ty, smem + half * (kTileSmemStride / sizeof(float)), 1 + half);
+    frontend_tile<kThreads>(in, sc, tb, out, tx, ty, smem + half * (kTileSmemStride / sizeof(float)), 1 + half);
 }
 
-// One tile per CTA, for frames of at most as many tiles as the device has SMs:
-// a pair would share one SM's issue slots and shared memory while another SM
-// idles.
-__global__ void __launch_bounds__(kThreads, 1)
+// One tile per CTA of twice the threads, for frames of at most as many tiles
+// as the device has SMs: paired, two tiles would share one SM's issue slots
+// while another SM idles, and one tile of kThreads threads would leave half of
+// its SM's warp slots empty (a tile is latency-bound). A 256x256 call took 131
+// us paired, 112 with one tile of 256 threads per CTA, 107 with 512.
+__global__ void __launch_bounds__(kPairThreads, 1)
     frontend_single_kernel(FrontendInputs in, FrontendScalars sc, FrontendTables tb, FrontendOutputs out) {
     extern __shared__ __align__(16) float smem[];
-    frontend_tile(in, sc, tb, out, static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), smem, 1);
+    frontend_tile<kPairThreads>(in, sc, tb, out, static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), smem, 1);
 }
 
 // One tile of a batched launch, kept out of line: inlined into the work loop,
@@ -1953,7 +1962,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // block): 1.8% fewer cycles per tile.
 __device__ __noinline__ void batch_tile(const FrontendJob j, const FrontendTables tb, int local, float* smem,
                                        int bar) {
-    frontend_tile(j.in, j.sc, tb, j.out, local % j.tiles_x, local / j.tiles_x, smem, bar);
+    frontend_tile<kThreads>(j.in, j.sc, tb, j.out, local % j.tiles_x, local / j.tiles_x, smem, bar);
 }
 
 // The frame of work-list item `item` and the item's tile within it.
@@ -2297,7 +2306,7 @@ bool frontend_launch(const FrontendInputs& in, const FrontendScalars& s, const F
     const dim3 grid{static_cast<unsigned>((tiles_x + 1) / 2), static_cast<unsigned>(tiles_y)};
     if (static_cast<long long>(tiles_x) * tiles_y <= t.sms) {
         const dim3 tiles{static_cast<unsigned>(tiles_x), static_cast<unsigned>(tiles_y)};
-        frontend_single_kernel<<<tiles, kThreads, kTileSmemStride, static_cast<cudaStream_t>(stream)>>>(in, s, t, out);
+        frontend_single_kernel<<<tiles, kPairThreads, kTileSmemStride, static_cast<cudaStream_t>(stream)>>>(in, s, t, out);
     } else if (in.tile_order != nullptr) {
         frontend_kernel<true><<<grid, kPairThreads, 2 * kTileSmemStride, static_cast<cudaStream_t>(stream)>>>(in, s, t,
                                                                                                            out);
