@@ -389,7 +389,9 @@ bool allocate(cujpegxl_encoder* e) {
                 cudaSuccess};
     ok = ok && cudaMemcpy(b + o_msec, plan.unit_section.data(), units * 4, cudaMemcpyHostToDevice) ==
                    cudaSuccess &&
-         cudaMemset(b + o_zero, 0, zero_bytes) == cudaSuccess;
+         // Waited for: a batch's kernels run on a stream of their own.
+         cudaMemsetAsync(b + o_zero, 0, zero_bytes, e->stream) == cudaSuccess &&
+         cudaStreamSynchronize(e->stream) == cudaSuccess;
     ok = ok && acquire_pinned(reinterpret_cast<void**>(&e->nv12_pinned), static_cast<std::size_t>(W) * H * 3 / 2 + 64);
     if (!ok) {
         release(e);
