@@ -1223,8 +1223,8 @@ __device__ void warp_canonical_codes(WarpCodeSmem& s, const std::uint8_t* depth,
         const int d{sym < len ? depth[sym] : 0};
         const unsigned peers{__match_any_sync(kFull, d)};
         if (d != 0 && (__ffs(peers) - 1) == lane) s.len_count[d] += static_cast<std::uint32_t>(__popc(peers));
+        __syncwarp();
     }
-    __syncwarp();
     // First code of each length, next[l] = (next[l - 1] + count[l - 1]) << 1,
     // as a sum of the shorter lengths' counts in units of 2^-15.
     {
@@ -1277,8 +1277,8 @@ __device__ void warp_store_complex(WarpCodeSmem& s, int num, BitSink& w, int lan
         const int d{i < new_len ? s.depth[i] : -1};
         const unsigned peers{__match_any_sync(kFull, d)};
         if (d >= 0 && (__ffs(peers) - 1) == lane) scr.hist[d] += static_cast<std::uint32_t>(__popc(peers));
+        __syncwarp();
     }
-    __syncwarp();
     // The code-length code: the same construction (limit 5) and canonical
     // codes, across the warp.
     if (lane < 18) {
