@@ -1138,6 +1138,8 @@ __device__ void warp_create_tree(WarpCodeSmem& s, const std::uint32_t* hist, int
             rank += (q.z < c || (q.z == c && t + 2 > i)) ? 1 : 0;
             rank += (q.w < c || (q.w == c && t + 3 > i)) ? 1 : 0;
         }
+        // The padding counts as equal to a symbol of the largest count.
+        if (c == kInf) rank -= -n & 3;
         s.cnt[rank] = c;
         s.leaf_sym[rank] = s.used[i];
     }

@@ -15,10 +15,44 @@ import numpy as np
 import pytest
 
 from cujpegxl_b200 import _capi
+from oracle import api
 
 pytestmark = pytest.mark.gpu
 
 GOLD = Path(__file__).resolve().parent / "golden" / "huffman.npz"
+
+
+def _device_code(h: np.ndarray):
+    depth = np.zeros(h.size, np.uint8)
+    bits = np.zeros(h.size, np.uint16)
+    head = np.zeros(256, np.uint8)
+    nbits = ctypes.c_uint32(0)
+    assert _capi.lib().cujpegxl_b200_debug_prefix_code(0, h.ctypes.data, h.size, depth.ctypes.data, bits.ctypes.data,
+                                                       head.ctypes.data, head.size, ctypes.byref(nbits)) == _capi.OK
+    return depth, bits, head[: (nbits.value + 7) // 8], nbits.value
+
+
+@pytest.mark.parametrize("length", [2, 3, 4, 5, 33, 254, 255, 256])
+@pytest.mark.parametrize("kind", ["largest", "even", "steep"])
+def test_device_prefix_codes_equal_serial_builder(length, kind):
+    """Alphabets around whole vectors of four counts, one of them the largest
+    32-bit count ("largest"; the others' sum stays below it), and lengths whose
+    symbols lie in every round of 32 ("even", "steep")."""
+    rng = np.random.Generator(np.random.PCG64(length))
+    h = np.ones(length, np.uint32) if kind == "even" else rng.integers(1, 50, length).astype(np.uint32)
+    if kind == "largest":
+        h[length // 2] = 0xFFFFFFFF
+    elif kind == "steep":
+        h[rng.integers(0, length, min(length, 20))] = 1 << np.arange(min(length, 20))
+    depth = np.zeros(length, np.uint8)
+    bits = np.zeros(length, np.uint16)
+    head = np.zeros(512, np.uint8)
+    nbits = api.oracle().oracle_huffman(h.ctypes.data, length, depth.ctypes.data, bits.ctypes.data, head.ctypes.data, 512)
+    got = _device_code(h)
+    assert got[3] == nbits
+    np.testing.assert_array_equal(got[0], depth)
+    np.testing.assert_array_equal(got[1], bits)
+    np.testing.assert_array_equal(got[2], head[: (nbits + 7) // 8])
 
 
 def test_device_prefix_codes_equal_reference_golden():
