@@ -44,7 +44,7 @@ EXPORTS = (
     "cujpegxl_b200_encoder_create_ex", "cujpegxl_b200_max_output_size_ex",
     "cujpegxl_b200_debug_fail_allocation", "cujpegxl_b200_debug_live_allocations",
     "cujpegxl_b200_encoder_enqueue_readback", "cujpegxl_b200_batch_schedule",
-    "cujpegxl_b200_debug_prefix_code",
+    "cujpegxl_b200_debug_prefix_code", "cujpegxl_b200_debug_fail_launch",
 )
 
 
@@ -124,6 +124,8 @@ def lib() -> ctypes.CDLL:
                                                   P(ctypes.c_uint32)]
     L.cujpegxl_b200_debug_fail_allocation.argtypes = [ctypes.c_uint32]
     L.cujpegxl_b200_debug_fail_allocation.restype = None
+    L.cujpegxl_b200_debug_fail_launch.argtypes = [ctypes.c_uint32]
+    L.cujpegxl_b200_debug_fail_launch.restype = None
     L.cujpegxl_b200_debug_live_allocations.restype = ctypes.c_uint64
     L.cujpegxl_b200_encoder_memory.argtypes = [E, P(ctypes.c_size_t), P(ctypes.c_size_t)]
     L.cujpegxl_b200_encode_planes_noalloc.argtypes = [P(DevicePlanes), ctypes.c_uint32, ctypes.c_uint32,

@@ -17,9 +17,15 @@ namespace jxb {
 // (No effect in a kernel launched the ordinary way.)
 __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// False when a test asked for this launch to fail
+// (cujpegxl_b200_debug_fail_launch).
+bool launch_allowed();
+
+// One launch, chained to the previous grid or an ordinary one. A failed launch
+// leaves no error behind for a later check on this thread to find.
 template <class... P, class... A>
-bool launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, std::size_t smem, cudaStream_t stream,
-                    const A&... args) {
+bool launch_one(bool chained, void (*kernel)(P...), unsigned blocks, unsigned threads, std::size_t smem,
+                cudaStream_t stream, const A&... args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -29,8 +35,23 @@ bool launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, std
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+    cfg.numAttrs = chained ? 1 : 0;
+    if (!launch_allowed()) return false;
+    if (cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+template <class... P, class... A>
+bool launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, std::size_t smem, cudaStream_t stream,
+                    const A&... args) {
+    return launch_one(true, kernel, blocks, threads, smem, stream, args...);
+}
+
+template <class... P, class... A>
+bool launch_plain(void (*kernel)(P...), unsigned blocks, unsigned threads, std::size_t smem, cudaStream_t stream,
+                  const A&... args) {
+    return launch_one(false, kernel, blocks, threads, smem, stream, args...);
 }
 
 }  // namespace jxb

@@ -81,13 +81,19 @@ DeviceTables g_tables[64];
 std::atomic<std::uint32_t> g_fail_countdown{0};
 std::atomic<std::uint64_t> g_live{0};
 
-bool injected_failure() {
-    std::uint32_t n{g_fail_countdown.load()};
+// Likewise for launches of the entropy stage and the read-back
+// (cujpegxl_b200_debug_fail_launch).
+std::atomic<std::uint32_t> g_fail_launch_countdown{0};
+
+bool counted_down(std::atomic<std::uint32_t>& countdown) {
+    std::uint32_t n{countdown.load()};
     while (n != 0) {
-        if (g_fail_countdown.compare_exchange_weak(n, n - 1)) return n == 1;
+        if (countdown.compare_exchange_weak(n, n - 1)) return n == 1;
     }
     return false;
 }
+
+bool injected_failure() { return counted_down(g_fail_countdown); }
 
 bool acquire_device(void** p, std::size_t bytes) {
     if (injected_failure() || cudaMalloc(p, bytes) != cudaSuccess) {
@@ -602,6 +608,8 @@ cujpegxl_status finish(cujpegxl_encoder* e, cujpegxl_output* output) {
 
 namespace jxb {
 
+bool launch_allowed() { return !counted_down(g_fail_launch_countdown); }
+
 bool encoder_prepare(cujpegxl_encoder* e) {
     DeviceScope scope{e->device};
     return scope.ok() && prepare(e);
@@ -992,6 +1000,8 @@ cujpegxl_status cujpegxl_b200_encoder_memory(cujpegxl_encoder* encoder, size_t* 
 uint32_t cujpegxl_b200_kernels_per_encode(void) { return 6u; }
 
 void cujpegxl_b200_debug_fail_allocation(uint32_t nth) { g_fail_countdown.store(nth); }
+
+void cujpegxl_b200_debug_fail_launch(uint32_t nth) { g_fail_launch_countdown.store(nth); }
 
 uint64_t cujpegxl_b200_debug_live_allocations(void) { return g_live.load(); }
 

@@ -2287,7 +2287,7 @@ bool entropy_launch(const EntropyDev& e, void* stream) {
     if (e.nsec > kMaxSections) return false;
     cudaStream_t st{static_cast<cudaStream_t>(stream)};
     const unsigned units{e.misc_units + static_cast<unsigned>(e.nstripes)};
-    if (e.clear_first) clear_kernel<<<clear_blocks(e.ndc), 256, 0, st>>>(e);
+    if (e.clear_first && !launch_plain(clear_kernel, clear_blocks(e.ndc), 256, 0, st, e)) return false;
     const auto codes{static_cast<unsigned>(kNumClusters + 2 * e.ndc)};
     if (e.direct) {
         return launch_chained(tokens_kernel, units, kAcThreads, kDirectSmem, st, e) &&
@@ -2296,14 +2296,13 @@ bool entropy_launch(const EntropyDev& e, void* stream) {
                launch_chained(layout_kernel, 1, kLayoutThreads, 0, st, e) &&
                launch_chained(emit_kernel, units, kAcThreads, kEmitStoredSmem, st, e);
     }
-    tokens_staged_kernel<<<units, kAcThreads, kHistSmem, st>>>(e);
-    codes_kernel<<<codes, 32, sizeof(WarpCodeSmem), st>>>(e);
-    lengths_unstored_kernel<<<kUnstoredCtas, kAcThreads, kBitsSmem, st>>>(e);
-    lengths_kernel<<<units, kAcThreads, 0, st>>>(e);
-    layout_kernel<<<1, kLayoutThreads, 0, st>>>(e);
-    emit_kernel<<<units, kAcThreads, kEmitStoredSmem, st>>>(e);
-    emit_unstored_kernel<<<kUnstoredCtas, kAcThreads, kEmitSmem, st>>>(e);
-    return cudaGetLastError() == cudaSuccess;
+    return launch_plain(tokens_staged_kernel, units, kAcThreads, kHistSmem, st, e) &&
+           launch_plain(codes_kernel, codes, 32, sizeof(WarpCodeSmem), st, e) &&
+           launch_plain(lengths_unstored_kernel, kUnstoredCtas, kAcThreads, kBitsSmem, st, e) &&
+           launch_plain(lengths_kernel, units, kAcThreads, 0, st, e) &&
+           launch_plain(layout_kernel, 1, kLayoutThreads, 0, st, e) &&
+           launch_plain(emit_kernel, units, kAcThreads, kEmitStoredSmem, st, e) &&
+           launch_plain(emit_unstored_kernel, kUnstoredCtas, kAcThreads, kEmitSmem, st, e);
 }
 
 void entropy_batch_plan(EntropyBatch& b) {

@@ -167,6 +167,12 @@ uint32_t cujpegxl_b200_kernels_per_encode(void);
 void cujpegxl_b200_debug_fail_allocation(uint32_t nth);
 uint64_t cujpegxl_b200_debug_live_allocations(void);
 
+/* Test hook: with n > 0, the n-th launch of an encode's entropy stage or
+ * read-back from then on (in the process) is not made and reported as failed;
+ * n = 0 turns the injection off. The encode returns CUJPEGXL_INTERNAL_ERROR,
+ * and the encoder's next encode must be unaffected. */
+void cujpegxl_b200_debug_fail_launch(uint32_t nth);
+
 /* Test hook: the device's prefix-code builder (the one every encode runs) on
  * one histogram of `length` symbols (1..256, host memory), for comparison with
  * the reference's build_and_store_huffman_tree (src/bitstream/prefix_code.cc):

@@ -18,6 +18,7 @@ import pytest
 
 from cujpegxl_b200 import Encoder, _capi
 from cujpegxl_b200.synth import make_nv12
+from oracle import api
 
 from .gpu_util import device_nv12
 
@@ -128,3 +129,42 @@ def test_enqueue_readback_rejects_pageable_memory():
         words = np.zeros(2, np.uint64)
         code = L.cujpegxl_b200_encoder_enqueue_readback(enc.handle, buf.ctypes.data, buf.size, words.ctypes.data)
         assert code == _capi.INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("planes", [False, True])
+def test_failed_launch_leaves_the_next_encode_unaffected(planes):
+    """The histograms and counters of the entropy stage are cleared by its own
+    passes, so a sequence that ends half-way leaves them filled: the next
+    encode has to clear them, and a clear that fails must not pass for one.
+    Every launch of the frontend's route (five passes and the read-back) and
+    of the caller's-planes route (seven) fails once, alone and followed by a
+    failure of the first launch after it, the clear."""
+    w, h, d = 520, 264, 1.0
+    keep, luma, chroma, lp, cp = device_nv12(make_nv12(w, h, 9), w, h)
+    L = _capi.lib()
+    with Encoder(w, h, d) as enc:
+        full = enc.encode_device(luma, chroma, lp, cp)
+        given = enc.read_planes()
+        sc = api.scalars(d)
+
+        def run():
+            if planes:
+                return enc.encode_planes(given, sc["global_scale"], sc["quant_dc"])
+            return enc.encode_device(luma, chroma, lp, cp)
+
+        assert run() == full
+        try:
+            for nth in range(1, 9 if planes else 7):
+                for again in (False, True):
+                    L.cujpegxl_b200_debug_fail_launch(nth)
+                    with pytest.raises(RuntimeError):
+                        run()
+                    if again:
+                        L.cujpegxl_b200_debug_fail_launch(1)
+                        with pytest.raises(RuntimeError):
+                            run()
+                    L.cujpegxl_b200_debug_fail_launch(0)
+                    assert run() == full, (nth, again)
+                    assert run() == full, (nth, again)
+        finally:
+            L.cujpegxl_b200_debug_fail_launch(0)
