@@ -5,7 +5,11 @@
 // short kernels. Every kernel launched so waits for the previous grid (all of
 // it, its writes visible) before it reads or writes anything; and nothing
 // here triggers the next grid early, so no block sits on an SM, waiting, that
-// another stream's blocks could use.
+// another stream's blocks could use. Because such a kernel can be resident
+// while the grid before it still writes, it reads what that grid writes by
+// ordinary loads: read-only-cache loads (__ldg) are for data that no one
+// writes while the kernel lives, and a compiler may move them ahead of the
+// wait.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -683,7 +683,7 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
                              e.ac + (static_cast<std::size_t>(c) * e.nblocks + blk0) * kCoeffsPerBlock) + tid};
 #pragma unroll
         for (int r{0}; r < kStripeRows; ++r) {
-            v[c][r] = loads && r < st.rows ? __ldg(src + static_cast<std::size_t>(r) * e.bw * (kCoeffsPerBlock / 8))
+            v[c][r] = loads && r < st.rows ? src[static_cast<std::size_t>(r) * e.bw * (kCoeffsPerBlock / 8)]
                                            : make_uint4(0, 0, 0, 0);
         }
     }
@@ -913,7 +913,7 @@ __device__ __forceinline__ void ac_tok_direct_body(const EntropyDev& e, const un
                 const int q{raw >> 6};
                 const std::size_t b{blk0 + static_cast<std::size_t>(r + (q >> lside)) * e.bw + x +
                                     (q & ((1 << lside) - 1))};
-                val[g] = __ldg(e.ac + (static_cast<std::size_t>(c) * e.nblocks + b) * kCoeffsPerBlock + (raw & 63));
+                val[g] = e.ac[(static_cast<std::size_t>(c) * e.nblocks + b) * kCoeffsPerBlock + (raw & 63)];
             }
         }
 #pragma unroll
@@ -984,7 +984,7 @@ __device__ __forceinline__ int misc_code_base(const EntropyDev& e, bool am, int 
 }
 // Its depth << 16 | code bits, in DC group g.
 __device__ __forceinline__ std::uint32_t misc_code(const EntropyDev& e, int g, std::uint32_t t) {
-    return __ldg(&e.code[misc_code_base(e, (t & 0x40000000u) != 0, g) + (t & 127u)]);
+    return e.code[misc_code_base(e, (t & 0x40000000u) != 0, g) + (t & 127u)];
 }
 __device__ __forceinline__ std::uint32_t misc_extra_count(std::uint32_t t) { return (t >> 7) & 31u; }
 __device__ __forceinline__ std::uint32_t misc_extra_bits(std::uint32_t t) { return (t >> 12) & 0x3ffffu; }
@@ -1499,7 +1499,7 @@ __device__ __forceinline__ void ac_bits_stored_body(const EntropyDev& e, const u
 #pragma unroll 4
     for (std::uint32_t t{static_cast<std::uint32_t>(tid)}; t < ntok; t += kAcThreads) {
         const std::uint32_t tk{*pool.at(t)};
-        sum += (__ldg(&e.code[token_code_index(tk)]) >> 16) + token_extra_count(tk);
+        sum += (e.code[token_code_index(tk)] >> 16) + token_extra_count(tk);
     }
     sum = warp_sum(sum);
     if ((tid & 31) == 0) sh_sum[tid >> 5] = sum;
@@ -1530,7 +1530,7 @@ __device__ __forceinline__ void ac_bits_unstored_body(const EntropyDev& e, const
             int cl;
             std::uint32_t tok, nb, bits;
             count_token(s, st, it, cl, tok, nb, bits);
-            b = __ldg(&e.ac_depth[cl * 256 + tok]) + nb;
+            b = e.ac_depth[cl * 256 + tok] + nb;
             if (it.nz != 0) s.active[atomicAdd(&s.nactive, 1)] = static_cast<std::uint16_t>(j);
         }
         s.aux[j] = b;
@@ -1541,7 +1541,7 @@ __device__ __forceinline__ void ac_bits_unstored_body(const EntropyDev& e, const
         const StripeItem it{stripe_item(s, gg.gw, j)};
         std::uint32_t total{0};
         coeff_tokens(s, it, lane, [&](bool has, int cl, std::uint32_t sym, std::uint32_t nb, std::uint32_t) {
-            if (has) total += __ldg(&e.ac_depth[cl * 256 + sym]) + nb;
+            if (has) total += e.ac_depth[cl * 256 + sym] + nb;
         });
         total = warp_sum(total);
         if (lane == 0) s.aux[j] += total;
@@ -1913,7 +1913,7 @@ __device__ __forceinline__ void ac_emit_stored_body(const EntropyDev& e, const u
     const unsigned long long pos{e.unit_pos[e.misc_units + blk]};
     const std::uint32_t bits{e.unit_sum[e.misc_units + blk]};
     for (int i{static_cast<int>(tid)}; i < kNumClusters * kAcSymbols / 4; i += kAcThreads) {
-        reinterpret_cast<uint4*>(code)[i] = __ldg(reinterpret_cast<const uint4*>(e.code) + i);
+        reinterpret_cast<uint4*>(code)[i] = reinterpret_cast<const uint4*>(e.code)[i];
     }
     const EmitTarget to{emit_target(e, pos, bits, win, kWindowWords)};
     __syncthreads();
@@ -1987,9 +1987,9 @@ __device__ __forceinline__ void ac_emit_unstored_body(const EntropyDev& e, const
         int cl;
         std::uint32_t tok, nb, bits;
         count_token(s, st, it, cl, tok, nb, bits);
-        const std::uint32_t d{__ldg(&e.ac_depth[cl * 256 + tok])};
+        const std::uint32_t d{e.ac_depth[cl * 256 + tok]};
         const unsigned long long at{to.base + s.aux[j]};
-        put_bits_at(to.words, at, d, __ldg(&e.ac_bits[cl * 256 + tok]));
+        put_bits_at(to.words, at, d, e.ac_bits[cl * 256 + tok]);
         if (nb) put_bits_at(to.words, at + d, nb, bits);
         if (it.nz != 0) {
             s.active[atomicAdd(&s.nactive, 1)] = static_cast<std::uint16_t>(j);
@@ -2002,12 +2002,12 @@ __device__ __forceinline__ void ac_emit_unstored_body(const EntropyDev& e, const
         const StripeItem it{stripe_item(s, gg.gw, j)};
         unsigned long long pos{to.base + s.aux[j]};
         coeff_tokens(s, it, lane, [&](bool has, int cl, std::uint32_t sym, std::uint32_t nb, std::uint32_t bits) {
-            const std::uint32_t d{has ? __ldg(&e.ac_depth[cl * 256 + sym]) : 0u};
+            const std::uint32_t d{has ? e.ac_depth[cl * 256 + sym] : 0u};
             const std::uint32_t tb{has ? d + nb : 0u};
             const std::uint32_t incl{warp_incl_scan(tb, lane)};
             if (has) {
                 const unsigned long long at{pos + incl - tb};
-                put_bits_at(to.words, at, d, __ldg(&e.ac_bits[cl * 256 + sym]));
+                put_bits_at(to.words, at, d, e.ac_bits[cl * 256 + sym]);
                 if (nb) put_bits_at(to.words, at + d, nb, bits);
             }
             pos += __shfl_sync(kFull, incl, 31);

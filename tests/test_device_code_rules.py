@@ -32,3 +32,13 @@ def test_rounds_of_shared_counters_are_ordered():
     assert len(turns) >= 3
     for body in turns:
         assert body.rstrip().rstrip("}").rstrip().endswith("__syncwarp();"), body
+
+
+def test_chained_passes_read_by_ordinary_loads():
+    """A kernel launched on programmatic stream serialisation can be resident
+    while the grid before it still writes, so what that grid writes is not
+    read-only for the kernel's lifetime: no read-only-cache loads."""
+    for name in ("entropy.cu", "cujpegxl.cu"):
+        text = (CSRC / name).read_text()
+        assert "launch_chained(" in text
+        assert "__ldg(" not in text and "ld.global.nc" not in text and "__restrict__" not in text, name
