@@ -45,6 +45,7 @@ EXPORTS = (
     "cujpegxl_b200_debug_fail_allocation", "cujpegxl_b200_debug_live_allocations",
     "cujpegxl_b200_encoder_enqueue_readback", "cujpegxl_b200_batch_schedule",
     "cujpegxl_b200_debug_prefix_code", "cujpegxl_b200_debug_fail_launch",
+    "cujpegxl_b200_debug_selection_routes",
 )
 
 
@@ -124,6 +125,7 @@ def lib() -> ctypes.CDLL:
                                                   P(ctypes.c_uint32)]
     L.cujpegxl_b200_debug_fail_allocation.argtypes = [ctypes.c_uint32]
     L.cujpegxl_b200_debug_fail_allocation.restype = None
+    L.cujpegxl_b200_debug_selection_routes.argtypes = [E, P(Nv12Input), P(ctypes.c_uint32)]
     L.cujpegxl_b200_debug_fail_launch.argtypes = [ctypes.c_uint32]
     L.cujpegxl_b200_debug_fail_launch.restype = None
     L.cujpegxl_b200_debug_live_allocations.restype = ctypes.c_uint64

@@ -1005,6 +1005,27 @@ void cujpegxl_b200_debug_fail_launch(uint32_t nth) { g_fail_launch_countdown.sto
 
 uint64_t cujpegxl_b200_debug_live_allocations(void) { return g_live.load(); }
 
+cujpegxl_status cujpegxl_b200_debug_selection_routes(cujpegxl_encoder* encoder, const cujpegxl_nv12_input* input,
+                                                     uint32_t counts[3]) {
+    if (encoder == nullptr || input == nullptr || counts == nullptr || input->luma == 0 || input->chroma == 0 ||
+        input->luma_pitch < encoder->config.width || input->chroma_pitch < encoder->config.width) {
+        return CUJPEGXL_INVALID_ARGUMENT;
+    }
+    DeviceScope scope{encoder->device};
+    if (!scope.ok() || !prepare(encoder)) return CUJPEGXL_INTERNAL_ERROR;
+    unsigned* dev{nullptr};
+    if (cudaMalloc(&dev, 3 * sizeof(unsigned)) != cudaSuccess) return CUJPEGXL_INTERNAL_ERROR;
+    encoder->fo.dbg_routes = dev;
+    const bool ok{cudaMemsetAsync(dev, 0, 3 * sizeof(unsigned), encoder->stream) == cudaSuccess &&
+                  enqueue_frame(encoder, reinterpret_cast<const std::uint8_t*>(input->luma), input->luma_pitch,
+                                reinterpret_cast<const std::uint8_t*>(input->chroma), input->chroma_pitch, 1u) &&
+                  cudaMemcpyAsync(counts, dev, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, encoder->stream) == cudaSuccess};
+    encoder->fo.dbg_routes = nullptr;
+    const bool done{cudaStreamSynchronize(encoder->stream) == cudaSuccess};
+    cudaFree(dev);
+    return ok && done ? CUJPEGXL_OK : CUJPEGXL_INTERNAL_ERROR;
+}
+
 cujpegxl_status cujpegxl_b200_debug_prefix_code(int32_t device_ordinal, const uint32_t* hist, uint32_t length,
                                                 uint8_t* depth, uint16_t* bits, uint8_t* header,
                                                 size_t header_cap, uint32_t* header_bits) {

@@ -60,42 +60,42 @@ static_assert(3 * kDrowsChannel <= kRegionAFloats, "final-DCT scratch exceeds re
 template <int N>
 constexpr int kDrowsStride = N == 32 ? 36 : N + 1;
 
-// Selection bases: double-precision DCT-II basis narrowed to float
-// (basis[k*n + t], src/transform_select.cu:29-37). Final-DCT bases: the float
-// basis of src/frontend_transform.cu:104-106 (cosf of a float argument).
-// Stored as pairs of consecutive frequencies, {basis[k][t], basis[k+1][t]} at
-// (k/2)*n + t for even k, so that the DCT passes compute two coefficients per
-// packed f32x2 instruction (per component the same rounding as the scalar
-// instruction, so the results are those of the scalar chains).
-__constant__ float2 c_sel8[32];
-__constant__ float2 c_sel16[128];
-__constant__ float2 c_sel32[512];
+// Final-DCT bases: the float basis of src/frontend_transform.cu:104-106 (cosf
+// of a float argument). Stored as pairs of consecutive frequencies,
+// {basis[k][t], basis[k+1][t]} at (k/2)*n + t for even k, so that the DCT
+// passes compute two coefficients per packed f32x2 instruction (per component
+// the same rounding as the scalar instruction, so the results are those of the
+// scalar chains).
 __constant__ float2 c_dct8[32];
 __constant__ float2 c_dct16[128];
 __constant__ float2 c_dct32[512];
 
+// Entries of FrontendTables::sel_basis: the selection bases of DCT8, DCT16 and
+// DCT32, double-precision DCT-II bases narrowed to float (basis[k*n + t],
+// src/transform_select.cu:29-37), in pairs as above.
+constexpr int kSelBasis = 32 + 128 + 512;
+
 // The selection bases folded for the bounded selection: element
 // (parity * N/4 + j) * N/2 + t holds {basis[k][t], basis[k + 2][t]} with
 // k = parity + 4j, for t < N/2 (basis[k][N-1-t] is +-basis[k][t] by parity, up
-// to the rounding that kFold of c_bound covers).
+// to a rounding that the bounds cover).
 // DCT8's are constants of its unrolled passes; DCT16's and DCT32's are read
 // from shared memory by passes rolled over the coefficient pairs (a third of
 // the code, which every launch fetches anew).
 __constant__ float2 c_fold8[16];
 // Error-bound coefficients of the bounded selection per size (bound_init).
 struct SelectBound {
-    float pixel;   // per unit of the largest centred pixel or row output
-    float column;  // per unit of the centre, for row frequency 0 in the column pass
-    float weight;  // largest reciprocal weight
-    float span;    // largest weight
+    float centre_max;   // column pass of row frequency 0, per unit of the centre: a coefficient's error at most
+    float centre_norm;  // ... and the norm of the column's
+    float col_max;      // column pass, per unit of the column's norm: a coefficient's error at most
+    float col_norm;     // ... and the norm of the column's
+    float weight;       // largest reciprocal weight
+    float span;         // largest weight
 };
 __constant__ SelectBound c_bound[3];
 
-template <int N, bool kSel>
+template <int N>
 __device__ __forceinline__ float2 basis2(int i) {
-    if (kSel) {
-        return N == 8 ? c_sel8[i] : (N == 16 ? c_sel16[i] : c_sel32[i]);
-    }
     return N == 8 ? c_dct8[i] : (N == 16 ? c_dct16[i] : c_dct32[i]);
 }
 
@@ -103,7 +103,7 @@ __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
 struct Small {
     float pre[256];       // AQ pre-erosion cells, 16x16 over the tile
-    float2 fold[64 + 256];  // folded bases of the bounded selection: DCT16, DCT32 (fold_entry)
+    float2 fold[64 + 256];  // folded bases of the bounded selection: DCT16, DCT32
     float cost8[64];
     float cost16[16];
     float cost32[4];
@@ -118,12 +118,13 @@ struct Small {
     int n32, n16, n8;
     signed char net[4];   // learned split class of each 32x32 region, -1 = RD heuristic
     // The bounded selection's costs and how far each can be from the exact
-    // one, the two halves of each DCT32 apart; the largest centred pixel of
-    // each region; and whether the bounds left the region undecided.
+    // one, the two halves of each DCT32 apart; the sum of squares of each
+    // region's centred pixels, in two halves; and whether the bounds left the
+    // region undecided.
     float2 near8[64];
     float2 near16[16];
     float2 near32[4][2];
-    float spread[4];
+    float energy[4][2];
     unsigned char undecided[4];
     float2 pow_lut[6];    // factor table of jx_pow24_2, for the packed sRGB transfer
 };
@@ -306,17 +307,14 @@ __device__ __forceinline__ float warp_tree(float v) {
     return v;
 }
 
-// Row pass of an N-point separable DCT: dst[fx*(N+1)] for fx in [F0, F1) from
-// one pixel row. Selection bases accumulate without FMA (the host twin's
-// arithmetic); final-DCT bases accumulate with FMA. Coefficients fx and fx+1
+// Row pass of the N-point final DCT: dst[fx * kDrowsStride<N>] for fx in
+// [F0, F1) from one pixel row, accumulated with FMA. Coefficients fx and fx+1
 // share each packed instruction; each is its own chain in c order.
-// src is 16-byte aligned (block rows of the sharpened planes are). The
-// outputs of frequency fx go to dst[fx * stride]: stride N + 1 for the
-// selection scratch, kDrowsStride<N> for the final DCT.
-template <int N, int F0, int F1, bool kSel>
+// src is 16-byte aligned (block rows of the sharpened planes are).
+template <int N, int F0, int F1>
 __device__ __forceinline__ void row_pass(const float* src, float* dst) {
     static_assert(F0 % 2 == 0 && F1 % 2 == 0, "pairs of frequencies");
-    constexpr int kStride{kSel ? N + 1 : kDrowsStride<N>};
+    constexpr int kStride{kDrowsStride<N>};
     float2 p[N];
 #pragma unroll
     for (int c{0}; c < N; c += 4) {
@@ -331,22 +329,67 @@ __device__ __forceinline__ void row_pass(const float* src, float* dst) {
         float2 s{0.0f, 0.0f};
 #pragma unroll
         for (int c{0}; c < N; ++c) {
-            if (kSel) {
-                s = __fadd2_rn(s, __fmul2_rn(basis2<N, true>((fx >> 1) * N + c), p[c]));
-            } else {
-                s = __ffma2_rn(basis2<N, false>((fx >> 1) * N + c), p[c], s);
-            }
+            s = __ffma2_rn(basis2<N>((fx >> 1) * N + c), p[c], s);
         }
         dst[fx * kStride] = s.x;
         dst[(fx + 1) * kStride] = s.y;
     }
 }
 
-// Column pass of the selection proxy fused with its quantiser: for fy in
-// [Y0, Y1) computes coefficient (fx, fy), quantises it with the DCT8 Y weight
-// sampled at the coefficient's frequency and stores its distortion and rate
-// contributions (zero for the low-frequency corner), as in block_ac_cost
-// (src/transform_select_impl.cuh:80-106).
+// Frequencies 2j .. 2j + 3 of N samples (each given twice) on the selection
+// basis, without FMA (the host twin's arithmetic), each its own chain in
+// sample order. `basis` is the block size's part of FrontendTables::sel_basis
+// in shared memory: in constant memory the warps of the exact selection, each
+// at its own place of 5 KB of bases, waited for its cache (17K cycles a region).
+template <int N>
+__device__ __forceinline__ void sel_dot(const float2* basis, int j, const float2 (&p)[N], float2& s0, float2& s1) {
+    const float4* b0{reinterpret_cast<const float4*>(basis + j * N)};
+    const float4* b1{b0 + N / 2};
+    s0 = make_float2(0.0f, 0.0f);
+    s1 = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int c{0}; c < N; c += 2) {
+        const float4 u{b0[c / 2]};
+        const float4 v{b1[c / 2]};
+        s0 = __fadd2_rn(s0, __fmul2_rn(make_float2(u.x, u.y), p[c]));
+        s1 = __fadd2_rn(s1, __fmul2_rn(make_float2(v.x, v.y), p[c]));
+        s0 = __fadd2_rn(s0, __fmul2_rn(make_float2(u.z, u.w), p[c + 1]));
+        s1 = __fadd2_rn(s1, __fmul2_rn(make_float2(v.z, v.w), p[c + 1]));
+    }
+}
+
+// Stride of a frequency's outputs in the exact selection's scratch: 16-byte
+// aligned for the column pass's loads, and lanes on distinct banks.
+template <int N>
+constexpr int kSelStride = N == 32 ? 36 : (N == 16 ? 20 : 12);
+template <int N>
+constexpr int kSelBlock = N == 32 ? 32 * 36 : (N == 16 ? 16 * 20 + 16 : 8 * 12 + 8);  // a block's outputs
+
+// Exact row pass of the selection: frequencies 2j and 2j + 1, j in [J0, J1), of
+// one pixel row to dst[k * kSelStride]. Rolled, as the column pass: unrolled
+// its code took longer to fetch than to run.
+template <int N>
+__device__ __forceinline__ void sel_row(const float* src, float* dst, const float2* basis, int J0, int J1) {
+    float2 p[N];
+#pragma unroll
+    for (int c{0}; c < N; c += 4) {
+        const float4 v{*reinterpret_cast<const float4*>(src + c)};
+        p[c] = dup2(v.x);
+        p[c + 1] = dup2(v.y);
+        p[c + 2] = dup2(v.z);
+        p[c + 3] = dup2(v.w);
+    }
+#pragma unroll 1
+    for (int j{J0}; j < J1; j += 2) {
+        float2 s0, s1;
+        sel_dot<N>(basis, j, p, s0, s1);
+        dst[2 * j * kSelStride<N>] = s0.x;
+        dst[(2 * j + 1) * kSelStride<N>] = s0.y;
+        dst[(2 * j + 2) * kSelStride<N>] = s1.x;
+        dst[(2 * j + 3) * kSelStride<N>] = s1.y;
+    }
+}
+
 // Distortion and rate of a selection coefficient whose quantum may be non-zero
 // (block_ac_cost, src/transform_select_impl.cuh:80-106). Kept out of line:
 // the unrolled column passes call it from hundreds of sites, and one shared
@@ -363,51 +406,137 @@ __device__ __noinline__ float2 sel_cost_nonzero(float coeff, float scaled, float
     return make_float2(err * err, rt);
 }
 
-template <int N, int Y0, int Y1>
-__device__ __forceinline__ void sel_col(const float* rows_fx, float* cd_fx, float* cr_fx, int fx,
-                                        float qgsf, const float* wsel, const float* l2t) {
-    static_assert(Y0 % 2 == 0 && Y1 % 2 == 0, "pairs of frequencies");
-    float2 rr[N];
+// Distortion and rate contributions {d, r} of coefficients (fx, fy0) and (fx,
+// fy0 + 1), quantised with the DCT8 Y weights sampled at their frequencies
+// (zero for the low-frequency corner), as in block_ac_cost
+// (src/transform_select_impl.cuh:80-106).
+template <int N>
+__device__ __forceinline__ void sel_terms(float2 coeffs, float2 w2, int fx, int fy0, float qgsf, const float* l2t,
+                                          float2& t0, float2& t1) {
+    // Scaled values, half-weights and squares of the pair at once.
+    const float2 sc2{__fmul2_rn(coeffs, f2dup(qgsf))};
+    const float2 hw2{__fmul2_rn(f2dup(0.5f), w2)};
+    const float2 sq2{__fmul2_rn(coeffs, coeffs)};
 #pragma unroll
-    for (int r{0}; r < N; ++r) {
-        rr[r] = dup2(rows_fx[r]);
-    }
-#pragma unroll
-    for (int fy0{Y0}; fy0 < Y1; fy0 += 2) {
-        float2 c2{0.0f, 0.0f};
-#pragma unroll
-        for (int r{0}; r < N; ++r) {
-            c2 = __fadd2_rn(c2, __fmul2_rn(basis2<N, true>((fy0 >> 1) * N + r), rr[r]));
-        }
-        // Weights, scaled values, half-weights and squares of the pair at once
-        // (fx * N + fy0 is even: one 8-byte weight load).
-        const float2 w2{*reinterpret_cast<const float2*>(wsel + fx * N + fy0)};
-        const float2 sc2{__fmul2_rn(c2, f2dup(qgsf))};
-        const float2 hw2{__fmul2_rn(f2dup(0.5f), w2)};
-        const float2 sq2{__fmul2_rn(c2, c2)};
-#pragma unroll
-        for (int h{0}; h < 2; ++h) {
-            const int fy{fy0 + h};
-            const float coeff{h == 0 ? c2.x : c2.y};
-            float d{0.0f};
-            float rt{0.0f};
-            if (!(fx < N / 8 && fy < N / 8)) {
-                const float w{h == 0 ? w2.x : w2.y};
-                const float scaled{h == 0 ? sc2.x : sc2.y};
-                if (fabsf(scaled) <= (h == 0 ? hw2.x : hw2.y)) {
-                    // |scaled / w| <= 1/2 rounds to a quotient of at most 1/2,
-                    // so q is zero and err is -coeff exactly: the same d, no
-                    // rate.
-                    d = h == 0 ? sq2.x : sq2.y;
-                } else {
-                    const float2 dr{sel_cost_nonzero(coeff, scaled, w, qgsf, l2t)};
-                    d = dr.x;
-                    rt = dr.y;
-                }
+    for (int h{0}; h < 2; ++h) {
+        float2 t{0.0f, 0.0f};
+        if (!(fx < N / 8 && fy0 + h < N / 8)) {
+            const float scaled{h == 0 ? sc2.x : sc2.y};
+            if (fabsf(scaled) <= (h == 0 ? hw2.x : hw2.y)) {
+                // |scaled / w| <= 1/2 rounds to a quotient of at most 1/2,
+                // so q is zero and err is -coeff exactly: the same d, no
+                // rate.
+                t.x = h == 0 ? sq2.x : sq2.y;
+            } else {
+                t = sel_cost_nonzero(h == 0 ? coeffs.x : coeffs.y, scaled, h == 0 ? w2.x : w2.y, qgsf, l2t);
             }
-            cd_fx[fy] = d;
-            cr_fx[fy] = rt;
         }
+        (h == 0 ? t0 : t1) = t;
+    }
+}
+
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int off) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.y, off));
+}
+__device__ __forceinline__ float2 pick2(bool second, float2 a, float2 b) { return second ? b : a; }
+
+// The N samples of a column of the exact selection's scratch, each twice.
+template <int N>
+__device__ __forceinline__ void sel_load(const float* rows_fx, float2 (&x)[N]) {
+#pragma unroll
+    for (int r{0}; r < N; r += 4) {
+        const float4 v{*reinterpret_cast<const float4*>(rows_fx + r)};
+        x[r] = dup2(v.x);
+        x[r + 1] = dup2(v.y);
+        x[r + 2] = dup2(v.z);
+        x[r + 3] = dup2(v.w);
+    }
+}
+
+// Exact column pass of a DCT8 or DCT16 and the sums of its distortions and
+// rates, {D, R} in all N lanes of the block; lane l has row frequency l % N.
+// The sums are the host twin's trees: over e = fx * N + fy, halves added from
+// the farthest apart down, so first over fx, then over fy. Of each four
+// frequencies fy the lanes a tree step apart swap two, then one, so that a
+// lane adds only what it goes on with; sums of two commute.
+template <int N>
+__device__ __forceinline__ float2 sel_col(const float* rows_fx, float qgsf, const float2* wsel, const float* l2t,
+                                          const float2* basis) {
+    static_assert(N == 8 || N == 16, "a block's columns in adjacent lanes");
+    const int lane{static_cast<int>(threadIdx.x) & 31};
+    const int fx{lane & (N - 1)};
+    constexpr int kFar{N / 2};
+    constexpr int kNear{N / 4};
+    const bool far{(lane & kFar) != 0};
+    const bool near{(lane & kNear) != 0};
+    float2 x[N];
+    sel_load<N>(rows_fx, x);
+    float2 before{0.0f, 0.0f};
+    float2 last{0.0f, 0.0f};
+#pragma unroll 1
+    for (int j{0}; j < N / 2; j += 2) {
+        float2 c0, c1;
+        sel_dot<N>(basis, j, x, c0, c1);
+        float2 t[4];
+        sel_terms<N>(c0, wsel[j * N + fx], fx, 2 * j, qgsf, l2t, t[0], t[1]);
+        sel_terms<N>(c1, wsel[(j + 1) * N + fx], fx, 2 * j + 2, qgsf, l2t, t[2], t[3]);
+        const float2 a{__fadd2_rn(pick2(far, t[0], t[2]), shfl_xor2(pick2(far, t[2], t[0]), kFar))};
+        const float2 b{__fadd2_rn(pick2(far, t[1], t[3]), shfl_xor2(pick2(far, t[3], t[1]), kFar))};
+        float2 sum{__fadd2_rn(pick2(near, a, b), shfl_xor2(pick2(near, b, a), kNear))};
+#pragma unroll
+        for (int off{N / 8}; off > 0; off >>= 1) sum = __fadd2_rn(sum, shfl_xor2(sum, off));
+        // Now fy = 2j + 2 far + near. Halves of fy: DCT8 adds the second four
+        // to the first; DCT16 the third to the first, the fourth to the second.
+        if constexpr (N == 8) {
+            last = __fadd2_rn(last, sum);
+        } else {
+            sum = __fadd2_rn(before, sum);
+            before = last;
+            last = sum;
+        }
+    }
+    if constexpr (N == 16) last = __fadd2_rn(before, last);
+    last = __fadd2_rn(last, shfl_xor2(last, kFar));
+    return __fadd2_rn(last, shfl_xor2(last, kNear));
+}
+
+// Exact column pass of DCT32 for fy = 8w .. 8w + 7, lane fx, and the sums of
+// the distortions and rates over fx to sums[fy]. The host twin's partials run
+// over e = fx * 32 + fy in steps of 256 (fx in steps of 8, one after the
+// other), then its tree over fx; the tree over fy is the caller's.
+__device__ __forceinline__ void sel_col32(const float* rows_fx, int w, float qgsf, const float2* wsel, const float* l2t,
+                                          const float2* basis, float2* sums) {
+    const int fx{static_cast<int>(threadIdx.x) & 31};
+    const bool b8{(fx & 8) != 0};
+    const bool b16{(fx & 16) != 0};
+    float2 x[32];
+    sel_load<32>(rows_fx, x);
+#pragma unroll 1
+    for (int j{4 * w}; j < 4 * w + 4; j += 2) {
+        float2 c0, c1;
+        sel_dot<32>(basis, j, x, c0, c1);
+        float2 t[4];
+        sel_terms<32>(c0, wsel[j * 32 + fx], fx, 2 * j, qgsf, l2t, t[0], t[1]);
+        sel_terms<32>(c1, wsel[(j + 1) * 32 + fx], fx, 2 * j + 2, qgsf, l2t, t[2], t[3]);
+        // Lane fx = 8g + i gathers fy = 2j + g of the lanes 8m + i, m = 0..3.
+        const float2 k0{pick2(b16, t[0], t[2])};
+        const float2 k1{pick2(b16, t[1], t[3])};
+        const float2 o0{shfl_xor2(pick2(b16, t[2], t[0]), 16)};
+        const float2 o1{shfl_xor2(pick2(b16, t[3], t[1]), 16)};
+        const float2 own{pick2(b8, k0, k1)};                                  // m = g
+        const float2 across{pick2(b8, o0, o1)};                               // m = g ^ 2
+        const float2 next{shfl_xor2(pick2(b8, k1, k0), 8)};             // m = g ^ 1
+        const float2 opposite{shfl_xor2(pick2(b8, o1, o0), 8)};         // m = g ^ 3
+        const float2 e0{pick2(b8, own, next)};                                // m = 2 b16
+        const float2 e1{pick2(b8, next, own)};                                // m = 2 b16 + 1
+        const float2 f0{pick2(b8, across, opposite)};                         // m = 2 - 2 b16
+        const float2 f1{pick2(b8, opposite, across)};
+        float2 sum{__fadd2_rn(pick2(b16, e0, f0), pick2(b16, e1, f1))};
+        sum = __fadd2_rn(sum, pick2(b16, f0, e0));
+        sum = __fadd2_rn(sum, pick2(b16, f1, e1));
+#pragma unroll
+        for (int off{4}; off > 0; off >>= 1) sum = __fadd2_rn(sum, shfl_xor2(sum, off));
+        if ((fx & 7) == 0) sums[2 * j + (fx >> 3)] = sum;
     }
 }
 
@@ -441,7 +570,7 @@ __device__ __forceinline__ void dct_col(const float* rows_fx, __half* coef, int 
         float2 c2{0.0f, 0.0f};
 #pragma unroll
         for (int r{0}; r < N; ++r) {
-            c2 = __ffma2_rn(basis2<N, false>((fy >> 1) * N + r), rr[r], c2);
+            c2 = __ffma2_rn(basis2<N>((fy >> 1) * N + r), rr[r], c2);
         }
         // raw and raw + 1 share their 64-slot group (raw is even), and the
         // pair's slot is 4-byte aligned (kCoefBlock is even).
@@ -462,31 +591,41 @@ __device__ __forceinline__ void dct_col(const float* rows_fx, __half* coef, int 
 // its distance from the host twin's float cost; a region whose decisions the
 // bounds settle is done, and the others go through the exact passes.
 //
-// The bound. All in units scaled by qgsf; u = 2^-24; m the centre, D the
-// largest |pixel - m| of the region. A chain of products and sums without FMA
+// The bound. All in units scaled by qgsf; u = 2^-24; |.| of a vector its
+// 2-norm; m the centre, d = pixel - m, S = |d| of the region; b_k the basis row
+// of frequency k, |b_k| = 1/sqrt(N). A chain of products and sums without FMA
 // is off by at most u times the sum of its products' and partial sums'
-// magnitudes. With pixel = m + d the partial sums of row frequency k are at
-// most |m| P_k(c) + D B_k(c), P_k(c) = |sum_{t<=c} b_k[t]|, B_k(c) =
-// sum_{t<=c} |b_k[t]|: hence FrontendTables::sel_centre (B_k + sum_c P_k(c)
-// per frequency) and SelectBound::pixel (the largest B_k + sum_c B_k(c) for
-// the host twin's chain, N/4 + 4 for the folded one in two accumulators, and
-// the basis's asymmetry). Row frequency 0 keeps the centre in its outputs,
-// which its column pass sees again (::column, the largest sel_centre of
-// k >= 1). With R the largest row output of a column (less the centre), every
-// coefficient is within
-//   delta = sel_centre m + pixel (D + R) [+ column m for row frequency 0]
-// and, quantised, within theta = delta + 10 u R of the host twin's (its
-// scaling, division and product round once each). |t| closer than theta / w to
-// a half-integer may then round the other way, which moves the rate by at most
-// 2 (0 <-> 1; less above) and the error term, near half a weight w, by at most
-// 2 theta; every other error term is off by at most theta, so the distortion
-// sum by at most 2 theta sqrt(n D2) + n theta^2 (Cauchy-Schwarz; D2 the sum of
-// n squares) and, per close call, theta w + 3 theta^2. Sums of non-negative
-// terms and the logarithms are covered by a relative 2e-5.
+// magnitudes, so the host twin's output of row frequency k by at most
+//   A_k m + G_k |d of the row|,  A_k = u (sum |b_k| + sum_c |sum_{t<=c} b_k[t]|)
+// (and what the rounded entries sum to), G_k = u (|b_k| + sum_c |b_k[0..c]|) by
+// Cauchy-Schwarz, to which G_k adds as much for the folded chains, their
+// fold, and the basis's asymmetry (bound_init). The column pass is an
+// orthogonal matrix over sqrt(N): the errors r of a column's N inputs, |r| <= sqrt(N) A_k m + G_k S,
+// come out as a vector of norm |r| / sqrt(N) =: eps, and as at most eps in
+// any one coefficient. (Taking every coefficient's error at its largest
+// overstates the sum below by up to sqrt(N): so 91% of the regions of a level
+// area with noise of one grey level stayed open, and 27% do.) Its own
+// roundings add G times the norm of the column's centred inputs (col_max,
+// col_norm; 10 u / sqrt(N) of it for scaling, division and product, each in
+// proportion to the coefficient), and for row frequency 0, whose inputs hold
+// the centre, A m once more (centre_max, centre_norm). So every coefficient
+// is within theta, and the column's vector of them within E, of the host
+// twin's. |t| closer than theta / w to a half-integer may round the other way,
+// which moves the rate by at most 2 (0 <-> 1; less above) and the square of
+// the error term, near half a weight w, by at most 2 theta (w + theta); the
+// other error terms, D2 the sum of their squares, move the sum by at most
+// 2 E sqrt(D2) + E^2. Sums of non-negative terms are off by at most 54 u
+// together, their logarithms by less than a relative 2e-5.
 
 __device__ __forceinline__ float log2_hw(float v) {
     float r;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));  // every v here is at least 1
+    return r;
+}
+
+__device__ __forceinline__ float sqrt_hw(float v) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
 
@@ -515,60 +654,78 @@ __device__ __forceinline__ float2 fold_dot8(int at, const float2 (&h)[4]) {
 template <int N>
 constexpr int kNearStride = N == 32 ? 36 : N + 1;
 
-// Folded row pass of parities [P0, P1): frequencies k of those parities of the
-// scaled centred row to dst[k * kNearStride]; the largest centred pixel.
-template <int N, int P0, int P1>
-__device__ __forceinline__ float near_row(const float* src, const float2* fold, float scale, float centre, float* dst) {
+// Folded row pass of the scaled centred row: frequency k to dst[k * kNearStride].
+// DCT16 and DCT8 take both parities; of DCT32 a lane takes parity `par` (0 or
+// 1) and returns the row's sum of squares.
+template <int N>
+__device__ __forceinline__ float near_row(const float* src, const float2* fold, float scale, float centre, int par,
+                                          float* dst) {
     float2 x[N / 2];
-    float big{0.0f};
 #pragma unroll
     for (int c{0}; c < N; c += 4) {
         const float4 v{*reinterpret_cast<const float4*>(src + c)};
         x[c / 2] = __ffma2_rn(make_float2(v.x, v.y), f2dup(scale), f2dup(-centre));
         x[c / 2 + 1] = __ffma2_rn(make_float2(v.z, v.w), f2dup(scale), f2dup(-centre));
     }
-    if (N == 32 && P0 == 0) {
+    float2 sq{0.0f, 0.0f};
+    if constexpr (N == 32) {
 #pragma unroll
-        for (int c{0}; c < N / 2; ++c) big = fmaxf(big, fmaxf(fabsf(x[c].x), fabsf(x[c].y)));
+        for (int c{0}; c < N / 2; ++c) sq = __ffma2_rn(x[c], x[c], sq);
     }
-#pragma unroll
-    for (int par{P0}; par < P1; ++par) {
+    // One parity: even frequencies from x[t] + x[N - 1 - t], odd ones from
+    // the differences.
+    auto half = [&](int p, float sign) {
         float2 h[N / 2];
 #pragma unroll
         for (int t{0}; t < N / 2; t += 2) {
-            const float2 lo{x[t / 2]};
             const float2 hi{make_float2(x[N / 2 - 1 - t / 2].y, x[N / 2 - 1 - t / 2].x)};
-            const float2 f{par == 0 ? __fadd2_rn(lo, hi) : __fadd2_rn(lo, f2neg(hi))};
+            const float2 f{__ffma2_rn(hi, f2dup(sign), x[t / 2])};
             h[t] = dup2(f.x);
             h[t + 1] = dup2(f.y);
         }
 #pragma unroll (N == 8 ? 2 : 1)
         for (int j{0}; j < N / 4; ++j) {
-            const int at{(par * (N / 4) + j) * (N / 2)};
+            const int at{(p * (N / 4) + j) * (N / 2)};
             float2 a;
             if constexpr (N == 8) {
                 a = fold_dot8(at, h);
             } else {
                 a = fold_dot<N>(fold + at, h);
             }
-            dst[(par + 4 * j) * kNearStride<N>] = a.x;
-            dst[(par + 4 * j + 2) * kNearStride<N>] = a.y;
+            dst[(p + 4 * j) * kNearStride<N>] = a.x;
+            dst[(p + 4 * j + 2) * kNearStride<N>] = a.y;
         }
+    };
+    if constexpr (N == 32) {
+        half(par, par == 0 ? 1.0f : -1.0f);
+    } else {
+#pragma unroll
+        for (int p{0}; p < 2; ++p) half(p, p == 0 ? 1.0f : -1.0f);
     }
-    return big;
+    return sq.x + sq.y;
 }
 
-// Folded column pass of parities [P0, P1) of row frequency fx, quantised and
-// costed; returns {cost, bound} of these coefficients. Weights of frequencies
-// (k, k + 2) as {1/w, 1/w', w, w'}, zero for the low-frequency corner.
-template <int N, int P0, int P1>
-__device__ __forceinline__ float2 near_col(const float* rows_fx, const float2* fold, int fx, const float4* weights,
-                                           const float* centre_bound, float centre, float spread, float inv_scale2) {
+// Sum over groups of kLanes adjacent lanes; the whole warp is here.
+template <int kLanes>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+    for (int off{1}; off < kLanes; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+// Folded column pass of row frequency fx, quantised and costed; returns
+// {cost, bound} of the column's coefficients (of DCT32: of those of parity
+// `par`; lanes l and l ^ 16 hold the two of a column). `energy`: the sum of
+// squares of centred pixels of the block, or of a region around it.
+// Weights of frequencies (k, k + 2) as {1/w, 1/w', w, w'}, zero for the
+// low-frequency corner.
+template <int N>
+__device__ __forceinline__ float2 near_col(const float* rows_fx, const float2* fold, int fx, int par, const float4* weights,
+                                           const float2* row_bound, float centre, float energy, float inv_scale2) {
     constexpr int kSize{N == 8 ? 0 : (N == 16 ? 1 : 2)};
-    constexpr float kU{5.9604645e-8f};
+    constexpr float kRootN{N == 8 ? 2.8284271f : (N == 16 ? 4.0f : 5.6568542f)};
     constexpr float kMagic{12582912.0f};  // 1.5 * 2^23: adding it rounds to integers
     float x[N];
-    float big{0.0f};
     if constexpr (N == 32) {
 #pragma unroll
         for (int r{0}; r < N; r += 4) {  // 16-byte aligned (kNearStride)
@@ -582,31 +739,34 @@ __device__ __forceinline__ float2 near_col(const float* rows_fx, const float2* f
 #pragma unroll
         for (int r{0}; r < N; ++r) x[r] = rows_fx[r];
     }
+    float2 sq{0.0f, 0.0f};
 #pragma unroll
-    for (int r{0}; r < N; ++r) big = fmaxf(big, fabsf(x[r]));
+    for (int r{0}; r < N; r += 2) sq = __ffma2_rn(make_float2(x[r], x[r + 1]), make_float2(x[r], x[r + 1]), sq);
+    const float norm_col{sqrt_hw(sq.x + sq.y)};
     const SelectBound sb{c_bound[kSize]};
-    const float delta{(centre_bound[fx] + (fx == 0 ? sb.column : 0.0f)) * centre + sb.pixel * (spread + big)};
-    const float theta{delta + 10.0f * kU * big};
+    const float2 rb{row_bound[fx]};
+    const float eps_row{rb.x * centre + rb.y * sqrt_hw(energy)};
+    const float theta{eps_row + (fx == 0 ? sb.centre_max * centre : 0.0f) + sb.col_max * norm_col};
+    const float err2{eps_row + (fx == 0 ? sb.centre_norm * centre : 0.0f) + sb.col_norm * norm_col};
     float2 dist{0.0f, 0.0f};
     float rate{0.0f};
     // A quantum beyond the rate table or the rounding trick: undecidable here.
     // Neither is one whose error may reach a whole quantum.
-    float flips{big * sb.weight > 4.0e5f || theta * sb.weight > 0.25f ? 1.0e9f : 0.0f};
-#pragma unroll
-    for (int par{P0}; par < P1; ++par) {
+    float flips{norm_col * sb.weight > 4.0e5f * kRootN || theta * sb.weight > 0.25f ? 1.0e9f : 0.0f};
+    auto half = [&](int p, float sign) {
         float2 h[N / 2];
 #pragma unroll
-        for (int t{0}; t < N / 2; ++t) h[t] = dup2(par == 0 ? x[t] + x[N - 1 - t] : x[t] - x[N - 1 - t]);
+        for (int t{0}; t < N / 2; ++t) h[t] = dup2(fmaf(x[N - 1 - t], sign, x[t]));
 #pragma unroll (N == 8 ? 2 : 1)
         for (int j{0}; j < N / 4; ++j) {
-            const int at{(par * (N / 4) + j) * (N / 2)};
+            const int at{(p * (N / 4) + j) * (N / 2)};
             float2 a;
             if constexpr (N == 8) {
                 a = fold_dot8(at, h);
             } else {
                 a = fold_dot<N>(fold + at, h);
             }
-            const float4 w{weights[(par * (N / 4) + j) * N + fx]};
+            const float4 w{weights[(p * (N / 4) + j) * N + fx]};
             const float2 inv{w.x, w.y};
             const float2 q{__fmul2_rn(a, inv)};
             const float2 qi{__fadd2_rn(__fadd2_rn(q, f2dup(kMagic)), f2dup(-kMagic))};
@@ -620,13 +780,25 @@ __device__ __forceinline__ float2 near_col(const float* rows_fx, const float2* f
                 rate += (fminf(mag.x, 1.0f) + log2_hw(1.0f + mag.x)) + (fminf(mag.y, 1.0f) + log2_hw(1.0f + mag.y));
             }
         }
+    };
+    if constexpr (N == 32) {
+        half(par, par == 0 ? 1.0f : -1.0f);
+    } else {
+#pragma unroll
+        for (int p{0}; p < 2; ++p) half(p, p == 0 ? 1.0f : -1.0f);
     }
     constexpr float kN2{static_cast<float>(N * N)};
-    constexpr float kCount{static_cast<float>(N / 2 * (P1 - P0))};
     const float d2{dist.x + dist.y};
-    const float off{theta * (2.0f * sqrtf(kCount * d2) + kCount * theta + flips * (theta + sb.span))};
-    const float cost{kN2 * inv_scale2 * d2 + kSelectLambda * rate};
-    return make_float2(cost, 1.01f * kN2 * inv_scale2 * off + kSelectLambda * flips + 2.0e-5f * cost);
+    float d2_col{d2};
+    float share{1.0f};
+    if constexpr (N == 32) {
+        d2_col += __shfl_xor_sync(0xffffffffu, d2, 16);
+        share = 0.5f;  // each of the two lanes adds half of the column's bound
+    }
+    const float off{share * err2 * (2.0f * sqrt_hw(d2_col) + err2) + flips * theta * (theta + sb.span)};
+    const float dc{kN2 * inv_scale2 * d2};
+    const float rc{kSelectLambda * rate};
+    return make_float2(dc + rc, 1.02f * kN2 * inv_scale2 * off + kSelectLambda * flips + 5.0e-6f * dc + 2.0e-5f * rc);
 }
 
 // Sum of both components over groups of kLanes adjacent lanes.
@@ -723,6 +895,229 @@ __device__ __forceinline__ void llf_to_dc(const __half* coef, int f, int ox, int
         }
         dcv[c] = static_cast<float>(static_cast<double>(M) * sum);
     }
+}
+
+// The exact selection of the regions in `exact`, with the host twin's
+// arithmetic: every candidate's cost, then the RD decisions, written to
+// Small::acs without a barrier behind them.
+//
+// A region at a time, all sizes side by side: warps 0-3 take eight frequencies
+// of DCT32 each, 4 and 5 two DCT16 each, the rest the sixteen DCT8; a phase is
+// one region's columns and the next one's rows. Mostly one region of a tile
+// comes here, and a phase costs its longest chain and its cold code whatever
+// the number of regions: size after size over the whole tile, unrolled, in
+// nine phases, a pair of tiles took 25K cycles with one region and 28K with
+// eight; here about 10K and 34K. Out of line, which is as fast and keeps the
+// tile's own code together.
+template <int kT>
+__device__ __noinline__ void exact_selection(unsigned exact, int bx0, int by0, int bw, int bh, float qg,
+                                             const float2* sel_basis, const float2* sel_weight, const float* log2_1p,
+                                             float* smem, int bar) {
+    const int tid{static_cast<int>(threadIdx.x) & (kT - 1)};
+    const int lane{tid & 31};
+    const int warp{tid >> 5};
+    const float* SY{smem + kRegionAFloats + kSplane};
+    Small& sm{*reinterpret_cast<Small*>(smem + kRegionAFloats + 3 * kSplane)};
+    // Region A: the row outputs of two regions, each DCT32, then four DCT16,
+    // then sixteen DCT8; DCT32's sums of two; the bases.
+    constexpr int kAt16{kSelBlock<32>};
+    constexpr int kAt8{kAt16 + 4 * kSelBlock<16>};
+    constexpr int kRows{kAt8 + 16 * kSelBlock<8>};
+    constexpr int kBases{2 * kRows + 2 * 64};
+    static_assert(kRows % 4 == 0 && kBases + 2 * kSelBasis <= kRegionAFloats, "scratch of the exact selection");
+    float2* basis8{reinterpret_cast<float2*>(smem + kBases)};
+    float2* basis16{basis8 + 32};
+    float2* basis32{basis16 + 128};
+    for (int i{tid}; i < kSelBasis / 2; i += kT) {
+        reinterpret_cast<float4*>(basis8)[i] = reinterpret_cast<const float4*>(sel_basis)[i];
+    }
+    tile_sync<kT>(bar);
+    constexpr int kWarps{kT / 32};
+    constexpr int kWarps8{kWarps - 6 < 4 ? kWarps - 6 : 4};  // with 128 row or column items of DCT8
+    // The other tile of a CTA swaps DCT16 and DCT8, so that no scheduler has
+    // both tiles' DCT16.
+    const int role{kT == 256 && bar == 2 && warp >= 4 ? warp ^ 2 : warp};
+    const int quad{(2 * (role - 4) + (lane >> 4)) & 3};  // DCT16 of roles 4 and 5
+    // (Blocks outside the image are costed as well, from the replicated border;
+    // the decision leaves them out.)
+    auto rows_of = [&](int ri, float* rows) {
+        const float* src{SY + (ri >> 1) * 32 * kSs + (ri & 1) * 32};
+        if (role < 4) {
+            sel_row<32>(src + lane * kSs, rows + lane, basis32, 4 * role, 4 * role + 4);
+        } else if (role < 6) {
+            sel_row<16>(src + ((quad >> 1) * 16 + (lane & 15)) * kSs + (quad & 1) * 16,
+                        rows + kAt16 + quad * kSelBlock<16> + (lane & 15), basis16, 0, 8);
+        } else if (role < 6 + kWarps8) {
+#pragma unroll 1
+            for (int k{(role - 6) * 32 + lane}; k < 128; k += 32 * kWarps8) {
+                const int b{k >> 3};
+                sel_row<8>(src + ((b >> 2) * 8 + (k & 7)) * kSs + (b & 3) * 8, rows + kAt8 + b * kSelBlock<8> + (k & 7),
+                           basis8, 0, 4);
+            }
+        }
+    };
+    auto cols_of = [&](int ri, const float* rows, float2* sums) {
+        if (role < 4) {
+            sel_col32(rows + lane * kSelStride<32>, role, qg, sel_weight + 160, log2_1p, basis32, sums);
+        } else if (role < 6) {
+            const float2 DR{sel_col<16>(rows + kAt16 + quad * kSelBlock<16> + (lane & 15) * kSelStride<16>, qg,
+                                        sel_weight + 32, log2_1p, basis16)};
+            if ((lane & 15) == 0) {
+                sm.cost16[(2 * (ri >> 1) + (quad >> 1)) * 4 + 2 * (ri & 1) + (quad & 1)] =
+                    256.0f * DR.x + kSelectLambda * DR.y;
+            }
+        } else if (role < 6 + kWarps8) {
+#pragma unroll 1
+            for (int k{(role - 6) * 32 + lane}; k < 128; k += 32 * kWarps8) {
+                const int b{k >> 3};
+                const float2 DR{sel_col<8>(rows + kAt8 + b * kSelBlock<8> + (k & 7) * kSelStride<8>, qg, sel_weight,
+                                           log2_1p, basis8)};
+                if ((k & 7) == 0) {
+                    sm.cost8[(ri >> 1) * 32 + (ri & 1) * 4 + 8 * (b >> 2) + (b & 3)] = 64.0f * DR.x + kSelectLambda * DR.y;
+                }
+            }
+        }
+    };
+    // 4d. RD decision of a region (src/transform_select_impl.cuh:130-201), by
+    // one warp.
+    auto decide = [&](int ri, const float2* sums) {
+        const float2 DR{warp_tree2(sums[lane])};
+        if (lane == 0) sm.cost32[ri] = 1024.0f * DR.x + kSelectLambda * DR.y;
+        if (lane == 0) {
+            const int rlx{(ri & 1) * 4};
+            const int rly{(ri >> 1) * 4};
+            const int rbx{bx0 + rlx};
+            const int rby{by0 + rly};
+            constexpr float kInf{1.0e30f};
+            const bool fit32{rbx + 4 <= bw && rby + 4 <= bh};
+            const float c32{fit32 ? sm.cost32[ri] : kInf};
+            float split{0.0f};
+            int choice[2][2];
+            for (int qy{0}; qy < 2; ++qy) {
+                for (int qx{0}; qx < 2; ++qx) {
+                    const int bx{rbx + 2 * qx};
+                    const int by{rby + 2 * qy};
+                    float sum8{0.0f};
+                    bool any{false};
+                    for (int dy{0}; dy < 2; ++dy) {
+                        for (int dx{0}; dx < 2; ++dx) {
+                            if (bx + dx < bw && by + dy < bh) {
+                                sum8 = sum8 + sm.cost8[(rly + 2 * qy + dy) * 8 + rlx + 2 * qx + dx];
+                                any = true;
+                            }
+                        }
+                    }
+                    if (!any) {
+                        choice[qy][qx] = -1;
+                        continue;
+                    }
+                    const bool fit16{bx + 2 <= bw && by + 2 <= bh};
+                    const float c16{fit16 ? sm.cost16[((rly >> 1) + qy) * 4 + (rlx >> 1) + qx] : kInf};
+                    if (fit16 && c16 <= sum8 + kSelectSplitEps) {
+                        choice[qy][qx] = 16;
+                        split = split + c16;
+                    } else {
+                        choice[qy][qx] = 8;
+                        split = split + sum8;
+                    }
+                }
+            }
+            if (fit32 && c32 <= split + kSelectSplitEps) {
+                for (int dy{0}; dy < 4; ++dy) {
+                    for (int dx{0}; dx < 4; ++dx) {
+                        sm.acs[(rly + dy) * 8 + rlx + dx] = (dx == 0 && dy == 0) ? 32 : 0;
+                    }
+                }
+            } else {
+                for (int qy{0}; qy < 2; ++qy) {
+                    for (int qx{0}; qx < 2; ++qx) {
+                        const int ch{choice[qy][qx]};
+                        if (ch < 0) {
+                            continue;
+                        }
+                        for (int dy{0}; dy < 2; ++dy) {
+                            for (int dx{0}; dx < 2; ++dx) {
+                                const int l{(rly + 2 * qy + dy) * 8 + rlx + 2 * qx + dx};
+                                if (ch == 16) {
+                                    sm.acs[l] = (dx == 0 && dy == 0) ? 16 : 0;
+                                } else if (rbx + 2 * qx + dx < bw && rby + 2 * qy + dy < bh) {
+                                    sm.acs[l] = 8;
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    };
+    float* rows[2]{smem, smem + kRows};
+    float2* sums[2]{reinterpret_cast<float2*>(smem + 2 * kRows), reinterpret_cast<float2*>(smem + 2 * kRows) + 32};
+    int ri{__ffs(static_cast<int>(exact)) - 1};
+    rows_of(ri, rows[0]);
+    tile_sync<kT>(bar);
+#pragma unroll 1
+    for (int b{0};; b ^= 1) {
+        exact &= exact - 1u;
+        cols_of(ri, b == 0 ? rows[0] : rows[1], b == 0 ? sums[0] : sums[1]);
+        const int next{__ffs(static_cast<int>(exact)) - 1};
+        if (next >= 0) rows_of(next, b == 0 ? rows[1] : rows[0]);
+        tile_sync<kT>(bar);
+        if (role == 7) decide(ri, b == 0 ? sums[0] : sums[1]);
+        if (next < 0) break;
+        ri = next;
+    }
+}
+
+// Whether most of the tile's regions in `open` show little else than weak
+// noise on a level ground; every warp finds the same.
+// Such regions go to the exact passes at once: all their quanta are zero, the
+// transforms then code the same energy to within a few times the rounding
+// errors, and the bounds leave a third to two thirds of them open (level 180,
+// distance 1: 27% with normal noise of one grey level, 66% with 0.4; on the
+// synthetic frame and on textures under 1%, on slopes with noise up to 20%).
+// Bounds for all and the exact passes for a third of the regions cost a pair
+// of tiles more (20K + 15K cycles) than the exact passes for all (34K).
+// The lines: the AQ stage's mean step between neighbours under 0.8% of the
+// level (over it, fewer than a quarter stay open), over 2.5e-4 (under it the
+// margin of the decisions settles them) and under 0.004 quanta (over it the
+// noise leaves non-zero quanta); the blocks' levels within 1.3 steps of each
+// other (noise alone gives 0.5 to 1; on slopes and textures the transforms'
+// energies differ).
+__device__ __forceinline__ bool noisy_tile(const Small& sm, const float* SY, unsigned open, int lane, int bx0, int by0,
+                                           int bw, int bh, float qg) {
+    // Eight lanes a region, two blocks each.
+    const int ri{lane >> 3};
+    const int x{4 * (ri & 1) + (lane & 3)};
+    const int y{4 * (ri >> 1) + ((lane >> 2) & 1)};
+    const float blocks{static_cast<float>(min(4, max(0, bw - bx0 - 4 * (ri & 1))) * min(4, max(0, bh - by0 - 4 * (ri >> 1))))};
+    float step{bx0 + x < bw && by0 + y < bh ? sm.aq_sums[0][8 * y + x] : 0.0f};
+    step += bx0 + x < bw && by0 + y + 2 < bh ? sm.aq_sums[0][8 * (y + 2) + x] : 0.0f;
+#pragma unroll
+    for (int off{1}; off < 8; off <<= 1) step += __shfl_xor_sync(0xffffffffu, step, off);
+    step *= 1.0f / 112.0f;  // differences a block; in multiples of the block count
+    const float level{SY[((ri >> 1) * 32 + 16) * kSs + (ri & 1) * 32 + 16]};
+    const bool weak{step > 2.5e-4f * blocks && step < 0.008f * blocks * level && step * qg < 0.004f * blocks};
+    unsigned v{__ballot_sync(0xffffffffu, weak)};
+    auto mask = [](unsigned b) { return (b & 1u) | ((b >> 7) & 2u) | ((b >> 14) & 4u) | ((b >> 21) & 8u); };
+    if (2 * __popc(mask(v) & open) < __popc(open)) return false;
+    // The variance of the blocks' levels (a row of eight pixels each), all
+    // sixteen: those outside the image repeat the last ones inside.
+    float2 sums{0.0f, 0.0f};
+#pragma unroll
+    for (int h{0}; h < 4; h += 2) {
+        const float4* row{reinterpret_cast<const float4*>(SY + (8 * (y + h) + 3) * kSs + 8 * x)};
+        const float4 a{row[0]};
+        const float4 b{row[1]};
+        const float mean{(((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) * 0.125f - level};
+        sums = __fadd2_rn(sums, make_float2(mean, mean * mean));
+    }
+#pragma unroll
+    for (int off{1}; off < 8; off <<= 1) {
+        sums = __fadd2_rn(sums, make_float2(__shfl_xor_sync(0xffffffffu, sums.x, off), __shfl_xor_sync(0xffffffffu, sums.y, off)));
+    }
+    const float variance{(sums.y - sums.x * sums.x * (1.0f / 16.0f)) * (1.0f / 16.0f)};
+    v = __ballot_sync(0xffffffffu, weak && variance * blocks * blocks < 1.7f * step * step);
+    return 2 * __popc(mask(v) & open) >= __popc(open);
 }
 
 // The whole frontend of the 64x64 tile (tx, ty) of one frame by kT threads; `smem` is the
@@ -1101,9 +1496,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
 
     // ---- 4. transform selection on the sharpened Y (src/transform_select.cu:134-262).
     const float* SY{shp + kSplane};
-    float* rows{smem};             // region A reused: row-pass scratch
-    float* cdist{smem + 4608};     // per-coefficient distortion contributions
-    float* crate{smem + 9216};     // per-coefficient rate contributions
+    float* rows{smem};  // region A reused: row-pass scratch
     const float qg{sc.qgsf_select};
     // Regions inside the image that the network did not decide need the RD
     // costs: first the bounded ones (not when the exact costs are dumped).
@@ -1112,8 +1505,8 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
     for (int ri{0}; ri < 4; ++ri) {
         inimg |= (bx0 + 4 * (ri & 1) < bw && by0 + 4 * (ri >> 1) < bh ? 1u : 0u) << ri;
     }
-    // Warps 4-7 clear the non-zero counters and CfL sums and finish
-    // each block's quant field from its AQ sums.
+    // The warps from 4 on clear the non-zero counters and CfL sums, and warps 4
+    // and 5 finish each block's quant field from its AQ sums.
     if (tid >= 128) {
         for (int i{tid - 128}; i < 192; i += kT - 128) {
             sm.nz[i >> 6][i & 63] = 0;
@@ -1146,17 +1539,21 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             sm.qf[lb] = qi;
         }
     }
-    unsigned exact{inimg & ~dmask};  // regions for the exact passes
-    if (exact != 0u && out.dbg_cost == nullptr) {
+    // Regions for the exact passes: all of a tile whose decisions the bounds are
+    // likely to leave open, otherwise those that they do.
+    unsigned exact{inimg & ~dmask};
+    const unsigned bounded{
+        out.dbg_cost != nullptr || exact == 0u || noisy_tile(sm, SY, exact, lane, bx0, by0, bw, bh, qg) ? 0u : exact};
+    if (bounded != 0u) {
         // Row passes of all three sizes, then their column passes, two phases
         // in all: every item is independent, and costs are summed in registers
-        // and across lanes. (The exact passes take nine phases, with every
-        // coefficient's two cost terms through shared memory.) Bound by issue
-        // and latency as the rest of the tile; at 4K the selection of a pair
-        // of tiles went from 37.7K cycles to 19K (rows 5.5K, columns 13K,
-        // decisions 0.7K), and about 1% of the regions, at distance 1 on the
-        // synthetic frame, go on to the exact passes (25K for a pair of tiles
-        // that has one); the launch went from 0.40 to 0.34 ms.
+        // and across lanes. Bound by latency and instruction fetch as the rest
+        // of the tile: 20K cycles for a pair of tiles (rows 6K, columns 11K,
+        // decisions 3K) against 28K to 33K of the exact passes on all regions.
+        // Launch of a 1280x720 frame, with bounds that left more regions open
+        // and exact passes inline behind them, then now: synthetic 65 -> 60 us;
+        // of a 3840x2160 one: synthetic 340 -> 342, level with noise of 0.4
+        // grey levels 435 -> 396, of one 453 -> 424, of 8 354 -> 329.
         constexpr int kRows16{4608};
         constexpr int kRows32{kRows16 + 16 * 272};
         static_assert(kRows32 % 4 == 0 && kRows32 + 4 * 32 * kNearStride<32> <= kRegionAFloats, "row scratch of the bounded selection");
@@ -1166,9 +1563,9 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int k{tid + h * kT};
             const int lb{k >> 3};
             const int r{k & 7};
-            if (((exact >> region_of_block(lb)) & 1u) != 0) {
-                near_row<8, 0, 2>(SY + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, nullptr, qg, centre_of(region_of_block(lb)),
-                                  rows + lb * 72 + r);
+            if (((bounded >> region_of_block(lb)) & 1u) != 0) {
+                near_row<8>(SY + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, nullptr, qg, centre_of(region_of_block(lb)), 0,
+                            rows + lb * 72 + r);
             }
         }
         // (With 512 threads the DCT16 rows and columns go to the upper half, the
@@ -1177,52 +1574,45 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int qd{(tid & 255) >> 4};
             const int r{tid & 15};
             const int ri{((qd >> 3) << 1) | ((qd & 3) >> 1)};
-            if (((exact >> ri) & 1u) != 0) {
-                near_row<16, 0, 2>(SY + ((qd >> 2) * 16 + r) * kSs + (qd & 3) * 16, sm.fold, qg, centre_of(ri),
-                                   rows + kRows16 + qd * 272 + r);
+            if (((bounded >> ri) & 1u) != 0) {
+                near_row<16>(SY + ((qd >> 2) * 16 + r) * kSs + (qd & 3) * 16, sm.fold, qg, centre_of(ri), 0,
+                             rows + kRows16 + qd * 272 + r);
             }
         }
+        // DCT32: two warps per region, each with 16 rows (then columns), the
+        // two parities of one in lanes l and l + 16.
+        const int part32{(tid >> 5) & 1};
+        const int line32{16 * part32 + (lane & 15)};
+        const int par32{lane >> 4};
         if (kT == 256 || tid < 256) {
-            // A warp per region and parity.
             const int ri{tid >> 6};
-            const int r{tid & 31};
-            if (((exact >> ri) & 1u) != 0) {
-                const float* src{SY + ((ri >> 1) * 32 + r) * kSs + (ri & 1) * 32};
-                float* dst{rows + kRows32 + ri * 32 * kNearStride<32> + r};
-                if ((tid & 32) == 0) {
-                    const float big{near_row<32, 0, 1>(src, sm.fold + 64, qg, centre_of(ri), dst)};
-                    const unsigned most{__reduce_max_sync(0xffffffffu, __float_as_uint(big))};
-                    if (lane == 0) sm.spread[ri] = __uint_as_float(most);
-                } else {
-                    near_row<32, 1, 2>(src, sm.fold + 64, qg, centre_of(ri), dst);
-                }
+            if (((bounded >> ri) & 1u) != 0) {
+                const float sq{near_row<32>(SY + ((ri >> 1) * 32 + line32) * kSs + (ri & 1) * 32, sm.fold + 64, qg,
+                                            centre_of(ri), par32, rows + kRows32 + ri * 32 * kNearStride<32> + line32)};
+                const float sum{group_sum<16>(sq)};
+                if (lane == 0) sm.energy[ri][part32] = sum;
             }
         }
         tile_sync<kT>(bar);
         const float inv_scale2{1.0f / (qg * qg)};
         if (kT == 256 || tid < 256) {
             const int ri{tid >> 6};
-            const int fx{tid & 31};
-            if (((exact >> ri) & 1u) != 0) {
-                const float* src{rows + kRows32 + (ri * 32 + fx) * kNearStride<32>};
-                const float c{fabsf(centre_of(ri))};
-                const float2 v{group_sum2<32>(
-                    (tid & 32) == 0 ? near_col<32, 0, 1>(src, sm.fold + 64, fx, tb.sel_pairs + 160, tb.sel_centre + 24, c,
-                                                         sm.spread[ri], inv_scale2)
-                                    : near_col<32, 1, 2>(src, sm.fold + 64, fx, tb.sel_pairs + 160, tb.sel_centre + 24, c,
-                                                         sm.spread[ri], inv_scale2))};
-                if (lane == 0) sm.near32[ri][(tid >> 5) & 1] = v;
+            if (((bounded >> ri) & 1u) != 0) {
+                const float2 v{group_sum2<32>(near_col<32>(
+                    rows + kRows32 + (ri * 32 + line32) * kNearStride<32>, sm.fold + 64, line32, par32, tb.sel_pairs + 160,
+                    tb.sel_row + 24, fabsf(centre_of(ri)), sm.energy[ri][0] + sm.energy[ri][1], inv_scale2))};
+                if (lane == 0) sm.near32[ri][part32] = v;
             }
         }
         if (kT == 256 || tid >= 256) {
             const int qd{(tid & 255) >> 4};
             const int fx{tid & 15};
             const int ri{((qd >> 3) << 1) | ((qd & 3) >> 1)};
-            const bool on{((exact >> ri) & 1u) != 0};
+            const bool on{((bounded >> ri) & 1u) != 0};
             float2 v{0.0f, 0.0f};
             if (on) {
-                v = near_col<16, 0, 2>(rows + kRows16 + qd * 272 + fx * 17, sm.fold, fx, tb.sel_pairs + 32, tb.sel_centre + 8,
-                                       fabsf(centre_of(ri)), sm.spread[ri], inv_scale2);
+                v = near_col<16>(rows + kRows16 + qd * 272 + fx * 17, sm.fold, fx, 0, tb.sel_pairs + 32, tb.sel_row + 8,
+                                 fabsf(centre_of(ri)), sm.energy[ri][0] + sm.energy[ri][1], inv_scale2);
             }
             v = group_sum2<16>(v);
             if (on && fx == 0) sm.near16[qd] = v;
@@ -1233,11 +1623,11 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const int lb{k >> 3};
             const int fx{k & 7};
             const int ri{region_of_block(lb)};
-            const bool on{((exact >> ri) & 1u) != 0};
+            const bool on{((bounded >> ri) & 1u) != 0};
             float2 v{0.0f, 0.0f};
             if (on) {
-                v = near_col<8, 0, 2>(rows + lb * 72 + fx * 9, nullptr, fx, tb.sel_pairs, tb.sel_centre, fabsf(centre_of(ri)), sm.spread[ri],
-                                      inv_scale2);
+                v = near_col<8>(rows + lb * 72 + fx * 9, nullptr, fx, 0, tb.sel_pairs, tb.sel_row, fabsf(centre_of(ri)),
+                                sm.energy[ri][0] + sm.energy[ri][1], inv_scale2);
             }
             v = group_sum2<8>(v);
             if (on && fx == 0) sm.near8[lb] = v;
@@ -1281,7 +1671,7 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const bool any_unsure{__any_sync(0xffffffffu, unsure) != 0};
             const bool take32{fit32 && c32.x + c32.y + 1.0e-9f <= lohi.x + kSelectSplitEps};
             const bool split{!any_unsure && (!fit32 || c32.x - c32.y > lohi.y + kSelectSplitEps + 1.0e-9f)};
-            if (((exact >> ri) & 1u) != 0) {
+            if (((bounded >> ri) & 1u) != 0) {
                 if (lane < 16 && inside && (take32 || split)) {
                     sm.acs[lby * 8 + lbx] = static_cast<signed char>(
                         take32 ? (lane == 0 ? 32 : 0) : (take16 ? ((lane & 3) == 0 ? 16 : 0) : 8));
@@ -1290,255 +1680,42 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             }
         }
         tile_sync<kT>(bar);
-        unsigned left{0};
 #pragma unroll
-        for (int ri{0}; ri < 4; ++ri) left |= (((exact >> ri) & 1u) != 0 && sm.undecided[ri] != 0 ? 1u : 0u) << ri;
-        exact = left;
+        for (int ri{0}; ri < 4; ++ri) {
+            if (((bounded >> ri) & 1u) != 0 && sm.undecided[ri] == 0) exact &= ~(1u << ri);
+        }
+    }
+    if (out.dbg_routes != nullptr && tid == 0) {
+        const int left{__popc(exact)};
+        atomicAdd(&out.dbg_routes[0], static_cast<unsigned>(__popc(bounded) - (bounded != 0u ? left : 0)));
+        atomicAdd(&out.dbg_routes[bounded != 0u ? 1 : 2], static_cast<unsigned>(left));
     }
     if (exact != 0u) {
-        // 4a. DCT8 candidates: one per block inside the image.
-        for (int k{tid}; k < 512; k += kT) {
-            const int lb{k >> 3};
-            const int r{k & 7};
-            const int lbx{lb & 7};
-            const int lby{lb >> 3};
-            if (bx0 + lbx < bw && by0 + lby < bh && ((exact >> region_of_block(lb)) & 1u) != 0) {
-                row_pass<8, 0, 8, true>(SY + (lby * 8 + r) * kSs + lbx * 8, rows + lb * 72 + r);
-            }
-        }
-        tile_sync<kT>(bar);
-        for (int k{tid}; k < 512; k += kT) {
-            const int lb{k >> 3};
-            const int fx{k & 7};
-            if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh &&
-                ((exact >> region_of_block(lb)) & 1u) != 0) {
-                sel_col<8, 0, 8>(rows + lb * 72 + fx * 9, cdist + lb * 72 + fx * 9,
-                                 crate + lb * 72 + fx * 9, fx, qg, tb.sel_weight, tb.log2_1p);
-            }
-        }
-        tile_sync<kT>(bar);
-        // Distortion and rate ride one packed pair through each step.
-#pragma unroll 2
-        for (int lb{warp}; lb < 64; lb += kT / 32) {
-            if (bx0 + (lb & 7) < bw && by0 + (lb >> 3) < bh &&
-                ((exact >> region_of_block(lb)) & 1u) != 0) {
-                const int i0{lb * 72 + (lane >> 3) * 9 + (lane & 7)};
-                const int i1{lb * 72 + ((lane + 32) >> 3) * 9 + (lane & 7)};
-                const float2 DR{warp_tree2(
-                    __fadd2_rn(make_float2(cdist[i0], crate[i0]), make_float2(cdist[i1], crate[i1])))};
-                if (lane == 0) {
-                    sm.cost8[lb] = 64.0f * DR.x + kSelectLambda * DR.y;
-                }
-            }
-        }
-        // 4b. DCT16 candidates: the 16 quads of the tile that fit in the image.
-        // Their row pass writes only the row scratch, which the DCT8
-        // reduction above does not read, so it shares that phase.
-        for (int k{tid}; k < 256; k += kT) {
-            const int qd{k >> 4};
-            const int r{k & 15};
-            const int qx{qd & 3};
-            const int qy{qd >> 2};
-            if (bx0 + 2 * qx + 2 <= bw && by0 + 2 * qy + 2 <= bh &&
-                ((exact >> (((qy >> 1) << 1) | (qx >> 1))) & 1u) != 0) {
-                row_pass<16, 0, 16, true>(SY + (qy * 16 + r) * kSs + qx * 16, rows + qd * 272 + r);
-            }
-        }
-        tile_sync<kT>(bar);
-        for (int k{tid}; k < 256; k += kT) {
-            const int qd{k >> 4};
-            const int fx{k & 15};
-            if (bx0 + 2 * (qd & 3) + 2 <= bw && by0 + 2 * (qd >> 2) + 2 <= bh &&
-                ((exact >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) != 0) {
-                sel_col<16, 0, 16>(rows + qd * 272 + fx * 17, cdist + qd * 272 + fx * 17,
-                                   crate + qd * 272 + fx * 17, fx, qg, tb.sel_weight + 1024,
-                                   tb.log2_1p);
-            }
-        }
-        tile_sync<kT>(bar);
-        for (int qd{warp}; qd < 16; qd += kT / 32) {
-            if (bx0 + 2 * (qd & 3) + 2 <= bw && by0 + 2 * (qd >> 2) + 2 <= bh &&
-                ((exact >> (((qd >> 3) << 1) | ((qd & 3) >> 1))) & 1u) != 0) {
-                // Distortion (x) and rate (y) as packed pairs, each in the
-                // host twin's order.
-                float2 p[8];
-#pragma unroll
-                for (int j{0}; j < 8; ++j) {
-                    const int t{lane + 32 * j};
-                    const int at{qd * 272 + (t >> 4) * 17 + (t & 15)};
-                    p[j] = make_float2(cdist[at], crate[at]);
-                }
-#pragma unroll
-                for (int j{0}; j < 4; ++j) p[j] = __fadd2_rn(p[j], p[j + 4]);
-                p[0] = __fadd2_rn(p[0], p[2]);
-                p[1] = __fadd2_rn(p[1], p[3]);
-                const float2 DR{warp_tree2(__fadd2_rn(p[0], p[1]))};
-                if (lane == 0) {
-                    sm.cost16[qd] = 256.0f * DR.x + kSelectLambda * DR.y;
-                }
-            }
-        }
-        // 4c. DCT32 candidates: the 4 regions of the tile that fit in the image.
-        // Their row pass shares the DCT16 reduction's phase (disjoint
-        // scratch).
-        for (int k{tid}; k < 256; k += kT) {
-            const int ri{k >> 6};
-            const int r{k & 31};
-            const bool hi{(k & 32) != 0};
-            const int rx{ri & 1};
-            const int ry{ri >> 1};
-            if (bx0 + 4 * rx + 4 <= bw && by0 + 4 * ry + 4 <= bh && ((exact >> ri) & 1u) != 0) {
-                const float* src{SY + (ry * 32 + r) * kSs + rx * 32};
-                float* dst{rows + ri * 1056 + r};
-                if (hi) {
-                    row_pass<32, 16, 32, true>(src, dst);
+        exact_selection<kT>(exact, bx0, by0, bw, bh, qg, tb.sel_basis, tb.sel_weight, tb.log2_1p, smem, bar);
+    }
+    if (dmask != 0u && warp < 4 && lane == 0 && ((dmask >> warp) & 1u) != 0) {
+        const int rlx{(warp & 1) * 4};
+        const int rly{(warp >> 1) * 4};
+        // Network split of a full region: class 0 is one DCT32, class
+        // 1 + m has quadrant q as four DCT8 when bit q of m is set, else
+        // as one DCT16.
+        const int cls{sm.net[warp]};
+        for (int dy{0}; dy < 4; ++dy) {
+            for (int dx{0}; dx < 4; ++dx) {
+                const int q{(dy >> 1) * 2 + (dx >> 1)};
+                signed char a;
+                if (cls == 0) {
+                    a = (dx == 0 && dy == 0) ? 32 : 0;
+                } else if ((((cls - 1) >> q) & 1) != 0) {
+                    a = 8;
                 } else {
-                    row_pass<32, 0, 16, true>(src, dst);
+                    a = ((dx & 1) == 0 && (dy & 1) == 0) ? 16 : 0;
                 }
-            }
-        }
-        tile_sync<kT>(bar);
-        for (int k{tid}; k < 256; k += kT) {
-            const int ri{k >> 6};
-            const int fx{k & 31};
-            const bool hi{(k & 32) != 0};
-            if (bx0 + 4 * (ri & 1) + 4 <= bw && by0 + 4 * (ri >> 1) + 4 <= bh &&
-                ((exact >> ri) & 1u) != 0) {
-                const float* src{rows + ri * 1056 + fx * 33};
-                float* cd{cdist + ri * 1056 + fx * 33};
-                float* cr{crate + ri * 1056 + fx * 33};
-                if (hi) {
-                    sel_col<32, 16, 32>(src, cd, cr, fx, qg, tb.sel_weight + 2048, tb.log2_1p);
-                } else {
-                    sel_col<32, 0, 16>(src, cd, cr, fx, qg, tb.sel_weight + 2048, tb.log2_1p);
-                }
-            }
-        }
-        tile_sync<kT>(bar);
-        if (warp < 4) {
-            const int ri{warp};
-            if (bx0 + 4 * (ri & 1) + 4 <= bw && by0 + 4 * (ri >> 1) + 4 <= bh &&
-                ((exact >> ri) & 1u) != 0) {
-                // Distortion (x) and rate (y) as packed pairs, each in the
-                // host twin's order.
-                float2 p[8];
-#pragma unroll
-                for (int j{0}; j < 8; ++j) {
-                    float2 dr{0.0f, 0.0f};
-#pragma unroll
-                    for (int m{0}; m < 4; ++m) {
-                        const int e{lane + 32 * j + 256 * m};
-                        const int at{ri * 1056 + (e >> 5) * 33 + (e & 31)};
-                        dr = __fadd2_rn(dr, make_float2(cdist[at], crate[at]));
-                    }
-                    p[j] = dr;
-                }
-#pragma unroll
-                for (int j{0}; j < 4; ++j) p[j] = __fadd2_rn(p[j], p[j + 4]);
-                p[0] = __fadd2_rn(p[0], p[2]);
-                p[1] = __fadd2_rn(p[1], p[3]);
-                const float2 DR{warp_tree2(__fadd2_rn(p[0], p[1]))};
-                if (lane == 0) {
-                    sm.cost32[ri] = 1024.0f * DR.x + kSelectLambda * DR.y;
-                }
+                sm.acs[(rly + dy) * 8 + rlx + dx] = a;
             }
         }
     }
-    // Decided regions of the network and of the exact passes.
-    if ((dmask | exact) != 0u) {
-    // 4d. RD decision per region (src/transform_select_impl.cuh:130-201), by
-    // lane 0 of warp ri, which wrote cost32[ri] itself (the DCT8 and DCT16
-    // costs are older than the last barrier).
-    if (warp < 4 && lane == 0) {
-        const int ri{warp};
-        const int rlx{(ri & 1) * 4};
-        const int rly{(ri >> 1) * 4};
-        const int rbx{bx0 + rlx};
-        const int rby{by0 + rly};
-        if (((dmask >> ri) & 1u) != 0) {
-            // Network split of a full region: class 0 is one DCT32, class
-            // 1 + m has quadrant q as four DCT8 when bit q of m is set, else
-            // as one DCT16.
-            const int cls{sm.net[ri]};
-            for (int dy{0}; dy < 4; ++dy) {
-                for (int dx{0}; dx < 4; ++dx) {
-                    const int q{(dy >> 1) * 2 + (dx >> 1)};
-                    signed char a;
-                    if (cls == 0) {
-                        a = (dx == 0 && dy == 0) ? 32 : 0;
-                    } else if ((((cls - 1) >> q) & 1) != 0) {
-                        a = 8;
-                    } else {
-                        a = ((dx & 1) == 0 && (dy & 1) == 0) ? 16 : 0;
-                    }
-                    sm.acs[(rly + dy) * 8 + rlx + dx] = a;
-                }
-            }
-        } else if (((exact >> ri) & 1u) != 0) {
-            constexpr float kInf{1.0e30f};
-            const bool fit32{rbx + 4 <= bw && rby + 4 <= bh};
-            const float c32{fit32 ? sm.cost32[ri] : kInf};
-            float split{0.0f};
-            int choice[2][2];
-            for (int qy{0}; qy < 2; ++qy) {
-                for (int qx{0}; qx < 2; ++qx) {
-                    const int bx{rbx + 2 * qx};
-                    const int by{rby + 2 * qy};
-                    float sum8{0.0f};
-                    bool any{false};
-                    for (int dy{0}; dy < 2; ++dy) {
-                        for (int dx{0}; dx < 2; ++dx) {
-                            if (bx + dx < bw && by + dy < bh) {
-                                sum8 = sum8 + sm.cost8[(rly + 2 * qy + dy) * 8 + rlx + 2 * qx + dx];
-                                any = true;
-                            }
-                        }
-                    }
-                    if (!any) {
-                        choice[qy][qx] = -1;
-                        continue;
-                    }
-                    const bool fit16{bx + 2 <= bw && by + 2 <= bh};
-                    const float c16{fit16 ? sm.cost16[((rly >> 1) + qy) * 4 + (rlx >> 1) + qx] : kInf};
-                    if (fit16 && c16 <= sum8 + kSelectSplitEps) {
-                        choice[qy][qx] = 16;
-                        split = split + c16;
-                    } else {
-                        choice[qy][qx] = 8;
-                        split = split + sum8;
-                    }
-                }
-            }
-            if (fit32 && c32 <= split + kSelectSplitEps) {
-                for (int dy{0}; dy < 4; ++dy) {
-                    for (int dx{0}; dx < 4; ++dx) {
-                        sm.acs[(rly + dy) * 8 + rlx + dx] = (dx == 0 && dy == 0) ? 32 : 0;
-                    }
-                }
-            } else {
-                for (int qy{0}; qy < 2; ++qy) {
-                    for (int qx{0}; qx < 2; ++qx) {
-                        const int ch{choice[qy][qx]};
-                        if (ch < 0) {
-                            continue;
-                        }
-                        for (int dy{0}; dy < 2; ++dy) {
-                            for (int dx{0}; dx < 2; ++dx) {
-                                const int l{(rly + 2 * qy + dy) * 8 + rlx + 2 * qx + dx};
-                                if (ch == 16) {
-                                    sm.acs[l] = (dx == 0 && dy == 0) ? 16 : 0;
-                                } else if (rbx + 2 * qx + dx < bw && rby + 2 * qy + dy < bh) {
-                                    sm.acs[l] = 8;
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-        }
-    }
-        tile_sync<kT>(bar);
-    }
+    if ((dmask | exact) != 0u) tile_sync<kT>(bar);
     if (out.dbg_cost != nullptr) {
         for (int lb{tid}; lb < 64; lb += kT) {
             const int lbx{lb & 7};
@@ -1634,20 +1811,20 @@ __device__ __forceinline__ void frontend_tile(const FrontendInputs& in, const Fr
             const float* src{P + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8};
             float* dst{drows + sm.fb_off[f] + r};
             if (k & 32) {
-                row_pass<32, 16, 32, false>(src, dst);
+                row_pass<32, 16, 32>(src, dst);
             } else {
-                row_pass<32, 0, 16, false>(src, dst);
+                row_pass<32, 0, 16>(src, dst);
             }
         } else if (k < t16) {
             const int f{n32 + ((k - t32) >> 4)};
             const int lb{sm.fb_list[f]};
             const int r{(k - t32) & 15};
-            row_pass<16, 0, 16, false>(P + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, drows + sm.fb_off[f] + r);
+            row_pass<16, 0, 16>(P + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, drows + sm.fb_off[f] + r);
         } else {
             const int f{n32 + n16 + ((k - t16) >> 3)};
             const int lb{sm.fb_list[f]};
             const int r{(k - t16) & 7};
-            row_pass<8, 0, 8, false>(P + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, drows + sm.fb_off[f] + r);
+            row_pass<8, 0, 8>(P + ((lb >> 3) * 8 + r) * kSs + (lb & 7) * 8, drows + sm.fb_off[f] + r);
         }
     }
     tile_sync<kT>(bar);
@@ -2105,41 +2282,53 @@ namespace {
 
 // Folded selection bases and the error-bound coefficients of the bounded
 // selection, from the bases the exact passes use. sw: the selection weights;
-// centre_bound: FrontendTables::sel_centre; folds: FrontendTables::fold.
-bool bound_init(const std::vector<float>& sw, float* centre_bound, std::vector<float>* folds) {
+// row_bound: FrontendTables::sel_row; folds: FrontendTables::fold.
+bool bound_init(const std::vector<float>& sw, std::vector<float>* row_bound, std::vector<float>* folds) {
     constexpr double kU{1.0 / 16777216.0};
     SelectBound bounds[3]{};
     for (int n : {8, 16, 32}) {
         const int si{n == 8 ? 0 : (n == 16 ? 1 : 2)};
+        const double root{std::sqrt(static_cast<double>(n))};
         std::vector<float> fold(static_cast<std::size_t>(n) * n / 2);
-        double pixel{0.0}, column{0.0}, skew{0.0};
+        double centre_max{0.0}, centre_sq{0.0}, col_max{0.0}, col_sq{0.0};
         for (int k{0}; k < n; ++k) {
-            double part{0.0}, mag{0.0}, parts{0.0}, mags{0.0}, asym{0.0};
+            double part{0.0}, mag{0.0}, parts{0.0}, sq{0.0}, chain{0.0}, asym{0.0}, folded{0.0};
+            double half_sq[2]{};  // of the folded chains: two, of the even and the odd samples (DCT8: one)
             for (int t{0}; t < n; ++t) {
                 const double b{selection_basis(n, k, t)};
                 const double mirror{selection_basis(n, k, n - 1 - t) * ((k & 1) != 0 ? -1.0 : 1.0)};
                 part += b;
                 mag += std::fabs(b);
                 parts += std::fabs(part);
-                mags += mag;
-                asym += std::fabs(b - mirror);
+                sq += b * b;
+                chain += std::sqrt(sq);
+                asym += (b - mirror) * (b - mirror);
                 if (t < n / 2) {
                     const int p{(k & 1) * (n / 4) + k / 4};
                     fold[2 * (p * (n / 2) + t) + ((k >> 1) & 1)] = static_cast<float>(b);
+                    double& h{half_sq[n == 8 ? 0 : t & 1]};
+                    h += b * b;
+                    folded += std::sqrt(2.0 * h);  // folding doubles a sample's square at most
                 }
             }
-            // Each basis row's magnitudes sum to at most 1 (so a pass hands on
-            // the errors of the one before), and a centre outside frequency
-            // 0 leaves what the row's rounded entries sum to; the margin
-            // covers second-order terms.
-            const double bound{1.02 * (kU * (mag + parts) + (k > 0 ? 2.0 * std::fabs(part) : 0.0))};
-            centre_bound[n - 8 + k] = static_cast<float>(bound);
-            if (k > 0) column = std::max(column, bound);
-            pixel = std::max(pixel, mag + mags + n / 4 + 4);
-            skew = std::max(skew, asym);
+            // Products and partial sums of the host twin's chain; the folded
+            // chains' partial sums, and the rounding of pixels, folded samples
+            // and the chains' sum. The margins cover second-order terms.
+            const double centre{1.02 * (kU * (mag + parts) + (k > 0 ? 2.0 * std::fabs(part) : 0.0))};
+            const double gain{1.02 * (kU * (std::sqrt(sq) + chain + folded + 3.0 * std::sqrt(sq)) + 2.0 * std::sqrt(asym))};
+            row_bound->push_back(static_cast<float>(centre));
+            row_bound->push_back(static_cast<float>(gain / root));
+            if (k > 0) {
+                centre_max = std::max(centre_max, centre);
+                centre_sq += centre * centre;
+            }
+            col_max = std::max(col_max, gain);
+            col_sq += gain * gain;
         }
-        bounds[si].pixel = static_cast<float>(1.02 * (kU * pixel + 2.0 * skew));
-        bounds[si].column = static_cast<float>(column);
+        bounds[si].centre_max = static_cast<float>(centre_max);
+        bounds[si].centre_norm = static_cast<float>(std::sqrt(centre_sq));
+        bounds[si].col_max = static_cast<float>(col_max + 10.0 * kU / root);
+        bounds[si].col_norm = static_cast<float>(std::sqrt(col_sq) + 10.0 * kU / root);
         for (int i{0}; i < n * n; ++i) {
             bounds[si].weight = std::max(bounds[si].weight, 1.0f / sw[si * 1024 + i]);
             bounds[si].span = std::max(bounds[si].span, sw[si * 1024 + i]);
@@ -2157,6 +2346,7 @@ bool bound_init(const std::vector<float>& sw, float* centre_bound, std::vector<f
 
 bool frontend_tables_init(FrontendTables* tables) {
     // Bases.
+    std::vector<float> bases;
     for (int n : {8, 16, 32}) {
         // Pair layout: element 2 * ((k / 2) * n + t) + (k & 1) holds basis[k][t].
         std::vector<float> sel(static_cast<std::size_t>(n) * n);
@@ -2170,16 +2360,11 @@ bool frontend_tables_init(FrontendTables* tables) {
                 dct[at] = gf * std::cos(arg);
             }
         }
-        const void* sel_sym{n == 8 ? static_cast<const void*>(&c_sel8)
-                                   : (n == 16 ? static_cast<const void*>(&c_sel16)
-                                              : static_cast<const void*>(&c_sel32))};
+        bases.insert(bases.end(), sel.begin(), sel.end());
         const void* dct_sym{n == 8 ? static_cast<const void*>(&c_dct8)
                                    : (n == 16 ? static_cast<const void*>(&c_dct16)
                                               : static_cast<const void*>(&c_dct32))};
-        if (cudaMemcpyToSymbol(sel_sym, sel.data(), sel.size() * sizeof(float)) != cudaSuccess ||
-            cudaMemcpyToSymbol(dct_sym, dct.data(), dct.size() * sizeof(float)) != cudaSuccess) {
-            return false;
-        }
+        if (cudaMemcpyToSymbol(dct_sym, dct.data(), dct.size() * sizeof(float)) != cudaSuccess) return false;
     }
     // Dequantisation weights [size][channel][1024].
     std::vector<float> deq(3 * 3 * 1024, 0.0f);
@@ -2202,9 +2387,20 @@ bool frontend_tables_init(FrontendTables* tables) {
             }
         }
     }
-    std::vector<float> centre(8 + 16 + 32);
+    std::vector<float> row_bound;
     std::vector<float> folds;
-    if (!bound_init(sw, centre.data(), &folds)) return false;
+    if (!bound_init(sw, &row_bound, &folds)) return false;
+    // The exact selection's: {w, w'} of frequencies (2j, 2j + 1) at [j][fx].
+    std::vector<float> exact_pairs(2 * (32 + 128 + 512));
+    for (int n : {8, 16, 32}) {
+        const int si{n == 8 ? 0 : (n == 16 ? 1 : 2)};
+        const int at{n == 8 ? 0 : (n == 16 ? 32 : 160)};
+        for (int fx{0}; fx < n; ++fx) {
+            for (int fy{0}; fy < n; ++fy) {
+                exact_pairs[2 * (at + (fy >> 1) * n + fx) + (fy & 1)] = sw[si * 1024 + fx * n + fy];
+            }
+        }
+    }
     // Weight pairs of the bounded selection: {1/w, 1/w', w, w'} of
     // frequencies (k, k + 2), k = parity + 4j, at [parity * N/4 + j][fx];
     // zeros in the low-frequency corner.
@@ -2253,32 +2449,36 @@ bool frontend_tables_init(FrontendTables* tables) {
     float* d_deq{nullptr};
     float* d_sw{nullptr};
     float* d_pairs{nullptr};
-    float* d_centre{nullptr};
+    float* d_row{nullptr};
     float* d_folds{nullptr};
+    float* d_bases{nullptr};
     float* d_l2{nullptr};
     double* d_ob{nullptr};
     if (cudaMalloc(&d_deq, deq.size() * 4) != cudaSuccess ||
-        cudaMalloc(&d_sw, sw.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_sw, exact_pairs.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_pairs, pairs.size() * 4) != cudaSuccess ||
-        cudaMalloc(&d_centre, centre.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_row, row_bound.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_folds, folds.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_bases, bases.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_l2, l2.size() * 4) != cudaSuccess ||
         cudaMalloc(&d_ob, ob.size() * 8) != cudaSuccess) {
         return false;
     }
     if (cudaMemcpy(d_deq, deq.data(), deq.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(d_sw, sw.data(), sw.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_sw, exact_pairs.data(), exact_pairs.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_pairs, pairs.data(), pairs.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_folds, folds.data(), folds.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(d_centre, centre.data(), centre.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_bases, bases.data(), bases.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_row, row_bound.data(), row_bound.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_l2, l2.data(), l2.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d_ob, ob.data(), ob.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
         return false;
     }
     tables->dequant = d_deq;
-    tables->sel_weight = d_sw;
+    tables->sel_weight = reinterpret_cast<const float2*>(d_sw);
     tables->sel_pairs = reinterpret_cast<const float4*>(d_pairs);
-    tables->sel_centre = d_centre;
+    tables->sel_row = reinterpret_cast<const float2*>(d_row);
+    tables->sel_basis = reinterpret_cast<const float2*>(d_bases);
     tables->fold = reinterpret_cast<const float2*>(d_folds);
     tables->log2_1p = d_l2;
     tables->llf_basis = d_ob;

@@ -42,6 +42,9 @@ struct FrontendOutputs {
     float* dbg_sharp;     // [3][H][W] XYB after inverse gaborish
     std::uint16_t* dbg_coeff;  // [3][B*64] FP16 bit patterns, covered-block layout
     float* dbg_cost;      // [3][B] selection costs: DCT8, DCT16 at quad and DCT32 at region first blocks
+    // Counters for tests: regions whose selection the bounds decided, left open
+    // to the exact passes, and that went to those at once.
+    unsigned* dbg_routes;  // [3]
 };
 
 struct FrontendInputs {
@@ -71,10 +74,11 @@ constexpr int kDequantInv = 3 * 3 * 1024;
 
 struct FrontendTables {
     const float* dequant;     // [3 sizes][3 ch][1024] stride 1024 (size 8, 16, 32), then their reciprocals
-    const float* sel_weight;  // [3 sizes][1024] DCT8 Y weight sampled at round(f*8/N)
+    const float2* sel_weight;  // DCT8 Y weights sampled at round(f*8/N), pairs (2j, 2j + 1) at [j][fx]: DCT8 at 0, DCT16 at 32, DCT32 at 160
+    const float2* sel_basis;  // selection bases in pairs of frequencies: DCT8 at 0, DCT16 at 32, DCT32 at 160
     const float4* sel_pairs;  // weight pairs of the bounded selection: DCT8 at 0, DCT16 at 32, DCT32 at 160
     const float2* fold;       // its folded bases: DCT16 (64 entries), DCT32 (256)
-    const float* sel_centre;  // its error per unit of centre and row frequency: DCT8 at 0, DCT16 at 8, DCT32 at 24
+    const float2* sel_row;    // its row errors per unit of centre and of the pixels' norm, by row frequency: DCT8 at 0, DCT16 at 8, DCT32 at 24
     const float* log2_1p;     // [kLog2TableSize] log2f(1 + i)
     const double* llf_basis;  // [2][4][4] orthonormal m-point basis for m = 2, 4
     int sms;                  // SMs of the device

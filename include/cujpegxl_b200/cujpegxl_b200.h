@@ -173,6 +173,14 @@ uint64_t cujpegxl_b200_debug_live_allocations(void);
  * and the encoder's next encode must be unaffected. */
 void cujpegxl_b200_debug_fail_launch(uint32_t nth);
 
+/* Test hook: runs the frontend on `input` (device memory) and counts the 32x32
+ * regions by the route of their transform selection: decided by costs with
+ * error bounds (counts[0]), left open by those and decided by the exact passes
+ * (counts[1]), sent to the exact passes at once (counts[2]). Regions that a
+ * network decided are in none of them. Synchronous. */
+cujpegxl_status cujpegxl_b200_debug_selection_routes(cujpegxl_encoder* encoder, const cujpegxl_nv12_input* input,
+                                                     uint32_t counts[3]);
+
 /* Test hook: the device's prefix-code builder (the one every encode runs) on
  * one histogram of `length` symbols (1..256, host memory), for comparison with
  * the reference's build_and_store_huffman_tree (src/bitstream/prefix_code.cc):

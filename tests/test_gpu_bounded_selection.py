@@ -6,10 +6,12 @@ blocks), at the smallest and largest quanta, and on partial regions."""
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 
-from cujpegxl_b200 import SINGLE_GROUP, Encoder
+from cujpegxl_b200 import SINGLE_GROUP, Encoder, _capi
 from cujpegxl_b200.synth import make_nv12
 
 from .gpu_util import device_nv12
@@ -28,6 +30,10 @@ def _content(kind: str, w: int, h: int) -> np.ndarray:
         luma = 90 + (rng.random((h, w)) < 0.5)
     elif kind == "repeated":
         luma = np.tile(rng.integers(0, 256, (8, 8)), (h // 8, w // 8))
+    elif kind.startswith("noise"):
+        luma = np.clip(np.round(180 + rng.normal(0, float(kind[5:]), (h, w))), 0, 255)
+    elif kind.startswith("slope"):
+        luma = np.clip(np.round(90 + x * 0.05 + y * 0.06 + rng.normal(0, float(kind[5:]), (h, w))), 0, 255)
     elif kind == "edges":
         luma = np.where((x // 40 + y // 24) % 2 == 0, 0, 255)
     else:
@@ -37,7 +43,7 @@ def _content(kind: str, w: int, h: int) -> np.ndarray:
 
 
 @pytest.mark.parametrize("w,h", [(256, 256), (328, 200)])
-@pytest.mark.parametrize("kind", ["flat", "gradient", "dither", "repeated", "edges", "synth"])
+@pytest.mark.parametrize("kind", ["flat", "gradient", "dither", "repeated", "edges", "synth", "noise1", "noise0.3", "slope0.4"])
 @pytest.mark.parametrize("distance", [0.01, 0.5, 1.0, 9.0])
 def test_bounded_selection_decides_as_the_exact_passes(w, h, kind, distance):
     keep, luma, chroma, lp, cp = device_nv12(_content(kind, w, h), w, h)
@@ -49,3 +55,25 @@ def test_bounded_selection_decides_as_the_exact_passes(w, h, kind, distance):
             planes.append(enc.read_planes())
     for key in planes[0]:
         assert np.array_equal(planes[0][key], planes[1][key]), key
+
+
+@pytest.mark.parametrize("w,h", [(640, 512), (1280, 720)])  # one tile per CTA, and pairs
+@pytest.mark.parametrize("kind,most", [("flat", 0.0), ("gradient", 0.0), ("synth", 0.03), ("noise4", 0.15), ("noise2", 0.15),
+                                       ("noise1", 0.1), ("noise0.4", 0.1), ("slope1", 0.25), ("slope0.4", 0.3)])
+def test_few_regions_pay_for_bounds_and_exact_passes(w, h, kind, most):
+    """Weak noise leaves the transforms' costs closer together than on any
+    other content. Bounds that add up every coefficient's error at its largest
+    left 50% to 100% of these regions open (the noisy kinds), and each of those
+    paid for both passes. `most`: twice to three times the shares that a
+    restatement of the bounds on the CPU gives, where the region does not go to
+    the exact passes at once."""
+    keep, luma, chroma, lp, cp = device_nv12(_content(kind, w, h), w, h)
+    counts = (ctypes.c_uint32 * 3)()
+    with Encoder(w, h, 1.0) as enc:
+        inp = _capi.Nv12Input(luma, chroma, lp, cp)
+        _capi.check("routes", _capi.lib().cujpegxl_b200_debug_selection_routes(enc.handle, ctypes.byref(inp), counts))
+    decided, left, at_once = counts
+    assert decided + left + at_once == -(-w // 32) * -(-h // 32)
+    assert left <= most * (decided + left + at_once), (decided, left, at_once)
+    if kind in ("flat", "gradient", "synth", "noise4"):
+        assert at_once <= 0.02 * (decided + left + at_once), (decided, left, at_once)
