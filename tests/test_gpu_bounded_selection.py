@@ -42,7 +42,10 @@ def _content(kind: str, w: int, h: int) -> np.ndarray:
     return np.concatenate([luma.astype(np.uint8).ravel(), chroma.astype(np.uint8).ravel()])
 
 
-@pytest.mark.parametrize("w,h", [(256, 256), (328, 200)])
+# Up to as many tiles as the GPU has SMs a CTA of 512 threads takes one tile;
+# above, one of two halves of 256 each, which map the work otherwise: 24 x 16
+# tiles, and 15 x 18 and 13 x 18 (an odd column; partial regions).
+@pytest.mark.parametrize("w,h", [(256, 256), (328, 200), (1480, 1000), (904, 1096), (808, 1128)])
 @pytest.mark.parametrize("kind", ["flat", "gradient", "dither", "repeated", "edges", "synth", "noise1", "noise0.3", "slope0.4"])
 @pytest.mark.parametrize("distance", [0.01, 0.5, 1.0, 9.0])
 def test_bounded_selection_decides_as_the_exact_passes(w, h, kind, distance):

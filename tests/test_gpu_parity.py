@@ -10,7 +10,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from cujpegxl_b200 import Encoder
+from cujpegxl_b200 import Encoder, acsnet
 from cujpegxl_b200.decode import decode_planes, psnr_y
 from cujpegxl_b200.synth import make_nv12
 from oracle import api
@@ -130,11 +130,66 @@ def test_host_input_path_matches_device_path():
     assert a == b
 
 
-def test_token_pool_overflow_falls_back_bit_exact():
-    """At distance 0.05 a 520x392 frame needs about 65 AC tokens per block,
-    twice what the token pool holds: the stripes that find the pool full are
-    tokenised again from their coefficients, and the file is still the
-    restatement's, byte for byte."""
+# Frames of more tiles than the GPU has SMs take two tiles per CTA: 15 x 18 and
+# 13 x 18 tiles (an odd column, whose right half leaves at once, and partial
+# regions on both sides). Without the stage dumps, so that the bounds decide.
+@pytest.mark.parametrize("network", [False, True])
+@pytest.mark.parametrize("w,h,d", [(904, 1096, 1.0), (808, 1128, 0.4), (1480, 1000, 3.0)])
+def test_paired_tiles_file_bit_exact(w, h, d, network):
+    """Against the restatement. With an all-zero network, which decides
+    nothing, the tiles come in the order that the inference kernel writes."""
+    nv = make_nv12(w, h, 7)
+    keep, luma, chroma, lp, cp = device_nv12(nv, w, h)
+    with Encoder(w, h, d) as enc:
+        if network:
+            norm = np.array([30.0, 4.0, 4.0, 1.0, 0.0, 0.4, 0.4, 0.5], np.float32)
+            net = acsnet.AcsNet(acsnet.pack_blob(np.zeros(acsnet.NPARAMS, np.float32), norm))
+            enc.set_acsnet(net, 0.2, acsnet.SPLIT | acsnet.QF)
+        assert enc.encode_device(luma, chroma, lp, cp) == api.encode(nv, w, h, d)
+
+
+def test_more_sections_than_layout_threads_bit_exact():
+    """1161 sections (1030 AC and 129 DC groups of a column of blocks): the
+    threads of the layout's one block take two TOC entries each."""
+    w, h, d = 8, 1030 * 256, 1.0
+    rng = np.random.Generator(np.random.PCG64(8))
+    luma8 = np.repeat(rng.integers(0, 256, (h // 4, w // 2)), 4, axis=0).repeat(2, axis=1)
+    nv = np.concatenate([luma8.ravel(), np.full(w * h // 2, 128)]).astype(np.uint8)
+    keep, luma, chroma, lp, cp = device_nv12(nv, w, h)
+    with Encoder(w, h, d) as enc:
+        assert enc.encode_device(luma, chroma, lp, cp) == api.encode(nv, w, h, d)
+
+
+TOKENS_PER_BLOCK = 32  # places of a block in the token pool
+
+
+def _tokens(g: dict) -> int:
+    """AC tokens of a frame's planes: a count per first block and channel, and
+    every scan position through the last non-zero coefficient, here at least
+    the non-zeros."""
+    first = int((g["acs"] != 0).sum())
+    return 3 * first + int((g["ac"] != 0).sum())
+
+
+def test_tokens_beyond_their_places_bit_exact():
+    """At distance 0.05 a 520x392 frame has more AC tokens than the pool has
+    places: those of the frontend's own planes go to the unused end of the
+    output buffer. Still the restatement's file."""
     w, h, d = 520, 392, 0.05
     nv, data, g = _frontend_and_file(w, h, d, 2)
+    assert _tokens(g) > TOKENS_PER_BLOCK * (w // 8) * (h // 8)
     assert data == api.encode(nv, w, h, d)
+
+
+def test_token_pool_overflow_of_given_planes_bit_exact():
+    """The same planes given by the caller: the stripes that find the pool full
+    are tokenised again from their coefficients in the length and emission
+    passes (planes from a frontend never are)."""
+    w, h, d = 520, 392, 0.05
+    nv, data, g = _frontend_and_file(w, h, d, 2)
+    assert _tokens(g) > TOKENS_PER_BLOCK * (w // 8) * (h // 8)
+    sc = api.scalars(d)
+    with Encoder(w, h, d) as enc:
+        given = enc.encode_planes({k: g[k] for k in ("ac", "dc", "acs", "qf", "ytox", "ytob")}, sc["global_scale"],
+                                  sc["quant_dc"])
+    assert given == api.encode(nv, w, h, d)
