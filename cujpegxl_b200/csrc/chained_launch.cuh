@@ -1,8 +1,8 @@
 // Launches of kernels that follow each other on a stream with programmatic
-// stream serialisation: the next grid's launch proceeds as the blocks of the
-// previous one leave, instead of after its last block has and its memory is
-// flushed, which saves about a microsecond per launch of a frame's chain of
-// short kernels. Every kernel launched so waits for the previous grid (all of
+// stream serialisation: the next grid is launched once the last block of the
+// previous one has left, while its memory is still being flushed, which saves
+// about a microsecond per launch of a frame's chain of short kernels. Every
+// kernel launched so waits for the previous grid (all of
 // it, its writes visible) before it reads or writes anything; and nothing
 // here triggers the next grid early, so no block sits on an SM, waiting, that
 // another stream's blocks could use. Because such a kernel can be resident

@@ -1364,8 +1364,8 @@ __device__ void warp_build_and_store(WarpCodeSmem& s, int length, BitSink& w, in
 }
 
 // One single-warp CTA per histogram (the 32 AC clusters, then the DC and the
-// AcMetadata histogram of every DC group): the construction is a long serial
-// chain on lane 0, so each chain gets an SM to itself.
+// AcMetadata histogram of every DC group): the merges, a tree per lane, are
+// serial chains of up to 255 steps, so each warp gets an SM to itself.
 __device__ __forceinline__ void codes_body(const EntropyDev& e, const unsigned blk) {
     extern __shared__ __align__(16) unsigned char code_smem[];
     const int lane{static_cast<int>(threadIdx.x) & 31};
@@ -1571,7 +1571,7 @@ struct BitsVisitor {
         }
     }
     __device__ void count_field(int, unsigned nbits) { total += nbits; }
-    __device__ void epf(int g) { total += e->am_depth[g * 256]; }
+    __device__ void epf(int) {}  // kept as tokens, not visited again
     __device__ void first_block(int) {}
     __device__ void token(int tab, int g, std::uint32_t sym, std::uint32_t nb, std::uint32_t) {
         total += (tab == kTabDc ? e->dc_depth : e->am_depth)[g * 256 + sym] + nb;
@@ -2070,7 +2070,7 @@ struct EmitVisitor {
         put(nb, v - (1u << nb));
     }
     __device__ void count_field(int g, unsigned nbits) { put(nbits, e->frozen[1 + g] - 1); }
-    __device__ void epf(int g) { put(e->am_depth[g * 256], e->am_bits[g * 256]); }
+    __device__ void epf(int) {}  // kept as tokens, not visited again
     __device__ void first_block(int) {}
     __device__ void token(int tab, int g, std::uint32_t sym, std::uint32_t nb, std::uint32_t bits) {
         const std::uint8_t* d{tab == kTabDc ? e->dc_depth : e->am_depth};

@@ -2133,10 +2133,10 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 // the tile's code held about 30 more registers live (its frame's fields and
 // coordinates are run-time values here, where the single-frame kernel reads
 // kernel parameters and block indices) and spilled 112 bytes per thread; out
-// of line it needs no more registers than the single-frame kernel (8 x 4K
-// batch: 1653 -> 1732 frames/s). The frame and tables are passed by value
-// (read from the call's copy, not through a pointer into the parameter
-// block): 1.8% fewer cycles per tile.
+// of line it ran faster (8 x 4K batch: 1653 -> 1732 frames/s), though the tile
+// spills 32 bytes of stores and the two kernels 72 and 56. The frame and
+// tables are passed by value (read from the call's copy, not through a pointer
+// into the parameter block): 1.8% fewer cycles per tile.
 __device__ __noinline__ void batch_tile(const FrontendJob j, const FrontendTables tb, int local, float* smem,
                                        int bar) {
     frontend_tile<kThreads>(j.in, j.sc, tb, j.out, local % j.tiles_x, local / j.tiles_x, smem, bar);

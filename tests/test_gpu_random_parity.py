@@ -1,6 +1,6 @@
 """The CUDA path against the restatement on seeded random geometries,
 distances and row pitches: narrow and tall frames, partial tiles and groups,
-distances from 0.1 (token-pool overflow) to 8. Every file must be equal byte
+distances from 0.1 (tokens beyond their places) to 8. Every file must be equal byte
 for byte."""
 
 from __future__ import annotations
